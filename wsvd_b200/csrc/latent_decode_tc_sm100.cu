@@ -364,9 +364,12 @@ __device__ __forceinline__ void run_share(const TcArgs& ta, uint8_t* sm) {
   uint32_t bars = sbase + kOffBar;
   auto bar = [&](int i) { return bars + 8u * i; };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + kOffTmemSlot);
-  // 16-byte vector loads of wk need f16 data with 16-byte aligned rows
-  const bool wk_vec = p.wk_dtype == WSVD_F16 && (p.wk_stride_r & 7) == 0 &&
-                      (reinterpret_cast<uintptr_t>(p.wk) & 15) == 0;
+  // vector loads of eight values of wk need rows aligned to them: 16 bytes for f16, 8 bytes for int8
+  // (whose scales are then read as 16-byte vectors too)
+  const bool wk_i8 = p.wk_dtype == WSVD_I8;
+  const bool wk_vec = (p.wk_stride_r & 7) == 0 &&
+                      (wk_i8 ? (reinterpret_cast<uintptr_t>(p.wk) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.wk_scale) & 15) == 0
+                             : (reinterpret_cast<uintptr_t>(p.wk) & 15) == 0);
 
   uint32_t tmem = 0;
   // ---- this CTA's work: every thread walks the same items (uniform loads, no broadcast needed)
@@ -539,7 +542,15 @@ __device__ __forceinline__ void run_share(const TcArgs& ta, uint8_t* sm) {
         const int task = (threadIdx.x & 127) + 128 * i, r = task >> 3, ic = task & 7;
         wpre[2 * i] = make_uint4(0u, 0u, 0u, 0u);
         wpre[2 * i + 1] = make_uint4(0u, 0u, 0u, 0u);
-        if (r < Rk) {
+        if (r < Rk && wk_i8) {
+          const int8_t* w = reinterpret_cast<const int8_t*>(p.wk) + (int64_t)r * p.wk_stride_r + (int64_t)hk_pre * 128;
+          const uint2 a0 = *reinterpret_cast<const uint2*>(w + (il ? ic * 16 : ic * 8));
+          const uint2 a1 = *reinterpret_cast<const uint2*>(w + (il ? ic * 16 + 8 : 64 + ic * 8));
+          wpre[2 * i].x = a0.x;
+          wpre[2 * i].y = a0.y;
+          wpre[2 * i + 1].x = a1.x;
+          wpre[2 * i + 1].y = a1.y;
+        } else if (r < Rk) {
           const __half* w = reinterpret_cast<const __half*>(p.wk) + (int64_t)r * p.wk_stride_r + (int64_t)hk_pre * 128;
           wpre[2 * i] = *reinterpret_cast<const uint4*>(w + (il ? ic * 16 : ic * 8));
           wpre[2 * i + 1] = *reinterpret_cast<const uint4*>(w + (il ? ic * 16 + 8 : 64 + ic * 8));
@@ -782,7 +793,7 @@ __device__ __forceinline__ void run_share(const TcArgs& ta, uint8_t* sm) {
         }
       }
       const int64_t col = (int64_t)hk * 128;
-      if (wk_vec && !interleaved) {
+      if (wk_vec && !wk_i8 && !interleaved) {
         // Common case (f16 wk, half-split pairing): packed f16 arithmetic.  The operands are
         // rounded to f16 for the MMA anyway; forming them with one extra f16 rounding of a
         // product keeps the error of the scores within a few 1e-5.  This thread's chunk of 8
@@ -814,6 +825,58 @@ __device__ __forceinline__ void run_share(const TcArgs& ta, uint8_t* sm) {
           const uint32_t off = nrow * 128 + ((ic ^ (nrow & 7)) << 4);
           *reinterpret_cast<uint4*>(sm + kOffB + off) = *reinterpret_cast<const uint4*>(pv);
           *reinterpret_cast<uint4*>(sm + kOffB + kBHalfBytes + off) = *reinterpret_cast<const uint4*>(qv);
+        }
+      } else if (wk_vec && wk_i8) {
+        // int8 wk in vectors of eight: the columns' scales are this thread's for all four ranks and go
+        // into q once, P = (q_d0 s_d0) w_d0 + (q_d1 s_d1) w_d1, Q = (q_d1 s_d0) w_d0 - (q_d0 s_d1) w_d1,
+        // fp32 throughout.  (Byte by byte, with the scales re-read per rank, the build of an item
+        // took as long as ten tiles: 64 dependent look-ups a thread.)
+        const int ic = tid & 7;
+        const __half* ws = reinterpret_cast<const __half*>(p.wk_scale) + col;
+        const uint4 s0v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 : ic * 8));
+        const uint4 s1v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 + 8 : 64 + ic * 8));
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {  // four frequencies at a time: fewer registers
+          float p0[4], p1[4], q0[4], q1[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int e = 4 * half + j;
+            const __half* s0h = reinterpret_cast<const __half*>(&s0v);
+            const __half* s1h = reinterpret_cast<const __half*>(&s1v);
+            const __half* pair = half == 0 ? s0h : s1h;
+            const float s0 = __half2float(interleaved ? pair[(2 * e) & 7] : s0h[e]);
+            const float s1 = __half2float(interleaved ? pair[(2 * e + 1) & 7] : s1h[e]);
+            p0[j] = qlo[e] * s0;
+            p1[j] = qhi[e] * s1;
+            q0[j] = qhi[e] * s0;
+            q1[j] = qlo[e] * s1;
+          }
+#pragma unroll
+          for (int it = 0; it < 4; ++it) {
+            const int r = (tid + 128 * it) >> 3;
+            // bytes of dimension d0 and d1 of the four frequencies (rank >= rank_k: zeros)
+            uint32_t w0, w1;
+            if (interleaved) {
+              const uint4 src = wpre[2 * it + half];
+              w0 = __byte_perm(src.x, src.y, 0x6420);
+              w1 = __byte_perm(src.x, src.y, 0x7531);
+            } else {
+              w0 = half == 0 ? wpre[2 * it].x : wpre[2 * it].y;
+              w1 = half == 0 ? wpre[2 * it + 1].x : wpre[2 * it + 1].y;
+            }
+            __align__(8) __half pv[4];
+            __align__(8) __half qv[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float u0 = (float)(int8_t)(w0 >> (8 * j)), u1 = (float)(int8_t)(w1 >> (8 * j));
+              pv[j] = __float2half_rn(fmaf(p0[j], u0, p1[j] * u1));
+              qv[j] = __float2half_rn(fmaf(q0[j], u0, -(q1[j] * u1)));
+            }
+            const int nrow = g * 64 + r;
+            const uint32_t off = nrow * 128 + ((ic ^ (nrow & 7)) << 4) + 8 * half;
+            *reinterpret_cast<uint2*>(sm + kOffB + off) = *reinterpret_cast<const uint2*>(pv);
+            *reinterpret_cast<uint2*>(sm + kOffB + kBHalfBytes + off) = *reinterpret_cast<const uint2*>(qv);
+          }
         }
       } else
 #pragma unroll
