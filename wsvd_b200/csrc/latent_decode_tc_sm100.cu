@@ -72,62 +72,71 @@
 namespace wsvd {
 namespace tc {
 
-constexpr int kG = 4;          // heads per CTA
-static_assert(kG == kBalancedGroup, "the merge kernel indexes balanced partials by groups of kG heads");
 constexpr int kTile = 128;     // positions per MMA tile (= tensor-memory lanes)
 constexpr int kRkMax = 64;
-constexpr int kEpiWarps = 4 * kG;
-constexpr int kMmaWarp = kEpiWarps;
-constexpr int kProducers = 3;  // with the MMA warp they fill one warp slot per scheduler
-constexpr int kThreads = (kEpiWarps + 1 + kProducers) * 32;
-// Registers per thread after the two groups have re-balanced them.  The pool is the CTA's own: what
-// the control warpgroup hands back, (96 - 64) * 128, is exactly what the epilogue warpgroups take,
-// (104 - 96) * 512.  (A request the pool cannot satisfy would block for ever.)
-constexpr int kLaunchRegs = 96;  // what 640 threads per CTA leave the compiler
-constexpr int kEpiRegs = 104;
-constexpr int kCtlRegs = 64;
-static_assert((kLaunchRegs - kCtlRegs) * 4 * 32 >= (kEpiRegs - kLaunchRegs) * kEpiWarps * 32, "register pool");
-static_assert(kProducers == 3, "the control warps must form one warpgroup (4 warps) for setmaxnreg");
-constexpr int kKSlots = 1;     // tiles of K: a tile's rows are copied to registers at the top of the tile
-constexpr int kVSlots = 2;     // tiles of V: the tile whose value MMAs are pending, and the next tile in flight
-constexpr int kWBufs = 3;      // W accumulators of 128 columns (one pair of heads each)
-
-constexpr uint32_t kHeadBytes = kTile * 64;         // one head's part of a unit: 128 tokens x 64 bytes (rank < 64: zero-filled)
-constexpr uint32_t kUnitBytes = kG * kHeadBytes;    // a ring slot: one tile of K or V for up to 4 KV heads
 constexpr uint32_t kAHalfBytes = kTile * 128;       // 128 rows x 64 f16
 constexpr uint32_t kABufBytes = 2 * kAHalfBytes;    // cos half + sin half
-constexpr uint32_t kBHalfBytes = kG * kRkMax * 128; // 256 rows x 64 f16
-constexpr uint32_t kPlaneBytes = 256;               // per pair of warps: 2 chunks of 16 tokens x 8 rows x 16 bytes
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kTmemD = kWBufs * 128;           // first column of the value accumulators: 8 per (head, warp)
 constexpr float kPlaneScale = 16776960.f;           // 2^24 - 256: a weight of 1 is 0xFFFF00
 
-// shared-memory map (offsets from a 1024-byte aligned base)
-constexpr uint32_t kOffB = 0;
-constexpr uint32_t kOffA = kOffB + 2 * kBHalfBytes;
-constexpr uint32_t kOffV = kOffA + 2 * kABufBytes;
-constexpr uint32_t kOffK = kOffV + kVSlots * kUnitBytes;
-constexpr uint32_t kOffPlanes = kOffK + kKSlots * kUnitBytes;
-constexpr uint32_t kOffRef = kOffPlanes + (kEpiWarps / 2) * kPlaneBytes;  // [head][tile parity][warp] reference max y of the planes
-constexpr uint32_t kOffSum = kOffRef + kG * 2 * 4 * 4;        // [head][warp] (max z, denominator) at the end
-constexpr uint32_t kOffBar = kOffSum + kG * 4 * 8;
-// barriers: V and K full/empty per ring slot, table full/empty x2, W full/empty x3, per head: D
-// full, planes ready; [P;Q] ready
-constexpr int kBarVFull = 0;
-constexpr int kBarKFull = kBarVFull + kVSlots;
-constexpr int kBarVEmpty = kBarKFull + kKSlots;
-constexpr int kBarKEmpty = kBarVEmpty + kVSlots;
-constexpr int kBarAFull = kBarKEmpty + kKSlots;
-constexpr int kBarAEmpty = kBarAFull + 2;
-constexpr int kBarWFull = kBarAEmpty + 2;
-constexpr int kBarWEmpty = kBarWFull + kWBufs;
-constexpr int kBarDFull = kBarWEmpty + kWBufs;
-constexpr int kBarPlanes = kBarDFull + kG;
-constexpr int kBarPq = kBarPlanes + kG;
-constexpr int kNumBars = kBarPq + 1;
-constexpr uint32_t kOffTmemSlot = kOffBar + 2 * kNumBars * 8;  // two sets of barriers, used by alternate items
-constexpr uint32_t kSmemBytes = kOffTmemSlot + 16;  // the dynamic shared-memory base is 1024-byte aligned
-static_assert(kOffA % 1024 == 0 && kOffV % 1024 == 0 && kOffPlanes % 256 == 0 && kOffBar % 8 == 0, "alignment");
+// Shape of the CTA.
+struct Cfg {
+  static constexpr int kG = 4;                     // heads per CTA
+  static constexpr int kEpiWarps = 4 * kG;
+  static constexpr int kMmaWarp = kEpiWarps;       // score MMAs
+  static constexpr int kLoadWarp = kEpiWarps + 1;  // copies
+  static constexpr int kValWarp = kEpiWarps + 2;   // value MMAs: one warp per pair of heads
+  static constexpr int kThreads = (kEpiWarps + 2 + kG / 2) * 32;
+  static constexpr int kRowBytes = 64;             // a latent row in shared memory (rank < 64: zero-filled)
+  static constexpr int kKSlots = 1;  // tiles of K: a tile's rows are copied to registers at the top of the tile
+  static constexpr int kVSlots = 2;  // tiles of V: the tile whose value MMAs are pending, and the next tile in flight
+  static constexpr int kWBufs = 3;   // W accumulators of 128 columns (one pair of heads each)
+  // Registers per thread after the two groups have re-balanced them.  The pool is the CTA's own: what
+  // the control warpgroup hands back, (96 - 64) * 128, is exactly what the epilogue warpgroups take,
+  // (104 - 96) * 512.  (A request the pool cannot satisfy would block for ever.)
+  static constexpr int kLaunchRegs = 96;  // what 640 threads per CTA leave the compiler
+  static constexpr int kEpiRegs = 104;
+  static constexpr int kCtlRegs = 64;
+  static_assert((kLaunchRegs - kCtlRegs) * 4 * 32 >= (kEpiRegs - kLaunchRegs) * kEpiWarps * 32, "register pool");
+  static_assert(kThreads == (kEpiWarps + 4) * 32, "the control warps must form one warpgroup (4 warps) for setmaxnreg");
+
+  static constexpr uint32_t kHeadBytes = kTile * kRowBytes;  // one head's part of a ring slot
+  static constexpr uint32_t kUnitBytes = kG * kHeadBytes;    // a ring slot: one tile of K or V for the group's KV heads
+  static constexpr uint32_t kBHalfBytes = kG * kRkMax * 128; // rows of 64 f16
+  static constexpr uint32_t kPlaneBytes = 256;               // per pair of warps: 2 chunks of 16 tokens x 8 rows x 16 bytes
+  static constexpr uint32_t kTmemD = kWBufs * 128;           // first column of the value accumulators: 8 per (head, warp)
+
+  // shared-memory map (offsets from a 1024-byte aligned base)
+  static constexpr uint32_t kOffB = 0;
+  static constexpr uint32_t kOffA = kOffB + 2 * kBHalfBytes;
+  static constexpr uint32_t kOffV = kOffA + 2 * kABufBytes;
+  static constexpr uint32_t kOffK = kOffV + kVSlots * kUnitBytes;
+  static constexpr uint32_t kOffPlanes = kOffK + kKSlots * kUnitBytes;
+  static constexpr uint32_t kOffRef = kOffPlanes + 2 * kG * kPlaneBytes;  // [head][tile parity][warp] reference max y of the planes
+  static constexpr uint32_t kOffSum = kOffRef + kG * 2 * 4 * 4;           // [head][warp] (max z, denominator) at the end
+  static constexpr uint32_t kOffMode = kOffSum + kG * 4 * 8;              // [4] how the K and V rows of a tile arrive (ring)
+  static constexpr uint32_t kOffItem = kOffMode + 16;                     // [head][item parity] ItemState
+  static constexpr uint32_t kOffBar = kOffItem + kG * 2 * 64;
+  // barriers: V and K full/empty per ring slot, table full/empty x2, W full/empty, per head: D full,
+  // planes ready; [P;Q] ready.  All are initialised once: their phases run on from one item to the next.
+  static constexpr int kBarVFull = 0;
+  static constexpr int kBarKFull = kBarVFull + kVSlots;
+  static constexpr int kBarVEmpty = kBarKFull + kKSlots;
+  static constexpr int kBarKEmpty = kBarVEmpty + kVSlots;
+  static constexpr int kBarAFull = kBarKEmpty + kKSlots;
+  static constexpr int kBarAEmpty = kBarAFull + 2;
+  static constexpr int kBarWFull = kBarAEmpty + 2;
+  static constexpr int kBarWEmpty = kBarWFull + kWBufs;
+  static constexpr int kBarDFull = kBarWEmpty + kWBufs;
+  static constexpr int kBarPlanes = kBarDFull + kG;
+  static constexpr int kBarPq = kBarPlanes + kG;
+  static constexpr int kNumBars = kBarPq + 1;
+  static constexpr uint32_t kOffTmemSlot = kOffBar + kNumBars * 8;
+  static constexpr uint32_t kSmemBytes = kOffTmemSlot + 16;  // the dynamic shared-memory base is 1024-byte aligned
+  static_assert(kOffA % 1024 == 0 && kOffV % 1024 == 0 && kOffPlanes % 256 == 0 && kOffBar % 8 == 0, "alignment");
+  static_assert(kSmemBytes <= 232448, "shared memory budget");
+};
+static_assert(Cfg::kG == kBalancedGroup, "the merge kernel indexes balanced partials by groups of kG heads");
 
 enum Status : unsigned int { kOk = 0, kTimeoutProducer = 1, kTimeoutMma = 2, kTimeoutEpilogue = 3, kBadSmemAlignment = 4 };
 
@@ -136,9 +145,6 @@ __device__ unsigned int g_status = 0;
 // ------------------------------------------------------------------ PTX helpers
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ void mbar_inval(uint32_t bar) {
-  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
@@ -189,12 +195,26 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity));
 }
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+// one lane of a converged warp (the same one every time): what it guards stays warp-uniform code
+__device__ __forceinline__ bool elect_one() {
+  uint32_t on;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(on));
+  return on != 0;
 }
-__device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+// The thread index, read anew: what is derived from it here is not kept in registers from an earlier phase.
+__device__ __forceinline__ int fresh_tid() {
+  int t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
 }
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
@@ -309,6 +329,7 @@ __device__ __forceinline__ uint64_t smem_desc_k_plain(uint32_t addr) {
   d |= (uint64_t)1 << 46;
   return d;
 }
+__device__ __forceinline__ uint64_t join64(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
 // Instruction descriptors.  f16 x f16 -> f32, both operands K-major.
 __device__ __forceinline__ uint32_t instr_desc_f16(int m, int n) {
   return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
@@ -321,16 +342,17 @@ __device__ __forceinline__ uint32_t instr_desc_i8(int m, int n) {
 struct TcArgs {
   KArgs k;
   int32_t table_rows;
-  int32_t use_tma;        // 0: latent rows are gathered with cp.async
-  int32_t slot_axis;      // 1 or 2: which coordinate of tmap_k / tmap_v is the token slot
-  int32_t box_heads;      // KV heads one tensor copy fetches: up to 4 (head-major caches), else 1
+  int32_t use_tma;         // 0: every latent row is gathered by the thread that owns its token
+  int32_t box_heads;       // KV heads one tensor copy of a whole tile fetches: up to kG
   int32_t balanced;        // 0: split mode
   int32_t* prefix_out;     // balanced mode: [batch + 2] tile prefix sums and share count for the merge kernel, or null
   unsigned int* arrivals;  // balanced mode: [batch * n_q_heads] zeroed arrival counters = merge inside this kernel, or null
   int32_t has_peers;       // with arrivals: output rows go to every rank's gathered buffer, group barrier at the end
   PeerArgs peers;
-  alignas(64) CUtensorMap tmap_k;      // latents as 3-D byte tensors: box 64 bytes x 64 slots x box_heads,
-  alignas(64) CUtensorMap tmap_v;      // 64-byte swizzle
+  alignas(64) CUtensorMap tmap_k;      // latents as 3-D tensors [KV head][slot][rank]: box rank x 128 slots x box_heads,
+  alignas(64) CUtensorMap tmap_v;      // swizzled over the row of shared memory
+  alignas(64) CUtensorMap tmap_k16;    // the same with a box of 16 slots x 1 head, for tiles made of several runs of
+  alignas(64) CUtensorMap tmap_v16;    // slots (a paged cache)
   alignas(64) CUtensorMap tmap_table;  // [2][rows][64] f16, box 64 x 128 x 2 (cos and sin tile), 128-byte swizzle
 };
 
@@ -346,51 +368,987 @@ __global__ void rope_table_kernel(__half* table, int rows, KArgs a) {
   table[((size_t)rows + pos) * 64 + i] = __float2half_rn(sn);
 }
 
-// The walk over this CTA's work items, for the epilogue warps (kEpi) or for the four control warps.
-// Two instantiations, because the two groups run with different register budgets (see the kernel):
-// everything a group executes after its setmaxnreg has to be code of its own.
-template <bool kEpi>
-__device__ __forceinline__ void run_share(const TcArgs& ta, uint8_t* sm) {
+// How the K and V rows of a tile reach shared memory, published by the copying warp with the K slot.
+enum TileMode : int { kTileCopied = 0, kTileGather = 1 };
+
+// A CTA's place in the list of work.
+struct Share {
+  int b, hg, t_first, tiles_left;  // first item: sequence, head group, tile; tiles of the whole share
+  int before_b;                    // tiles in the sequences before b
+  int shares;                      // CTAs that have a share
+  int64_t total;                   // entries of the tile list
+};
+
+// The walk over a CTA's work items.  Every role makes it for itself, so that a role can be in another
+// item than its neighbours.
+struct Walk {
+  int b, hg, t_first, tiles_left, before_b;
+  int n, req;            // length and request of sequence b
+  int tiles_b;           // balanced mode: tiles of sequence b
+  int lo, hi, ntiles;    // the item: tokens [lo, hi) of (b, head group hg)
+
+  __device__ __forceinline__ void cut() {
+    tiles_b = (n + kTile - 1) / kTile;
+    ntiles = min(tiles_left, tiles_b - t_first);
+    lo = t_first * kTile;
+    hi = min(n, (t_first + ntiles) * kTile);
+  }
+  // false: the CTA has no work
+  __device__ __forceinline__ bool start(const TcArgs& ta, const Share& sh, int n_hg) {
+    const WsvdLatentDecodeParams& p = ta.k.p;
+    if (ta.balanced) {
+      if (sh.tiles_left <= 0) return false;
+      b = sh.b, hg = sh.hg, t_first = sh.t_first, tiles_left = sh.tiles_left, before_b = sh.before_b;
+      n = p.b_seq_len[b], req = p.b_req_idx[b];
+      cut();
+      return true;
+    }
+    // one fixed-length split; an empty one writes nothing
+    const int split = blockIdx.x % ta.k.n_splits;
+    hg = (blockIdx.x / ta.k.n_splits) % n_hg, b = blockIdx.x / (ta.k.n_splits * n_hg);
+    t_first = 0, before_b = 0, tiles_b = 0;
+    n = p.b_seq_len[b], req = p.b_req_idx[b];
+    lo = split * ta.k.split_len;
+    hi = min(n, lo + ta.k.split_len);
+    ntiles = tiles_left = (hi - lo + kTile - 1) / kTile;
+    return hi > lo;
+  }
+  // the next item of the share: the next head group, or the next sequence that has tokens
+  __device__ __forceinline__ bool next(const WsvdLatentDecodeParams& p, int n_hg) {
+    tiles_left -= ntiles;
+    if (tiles_left <= 0) return false;
+    t_first = 0;
+    if (++hg == n_hg) {
+      hg = 0;
+      before_b += tiles_b;
+      do {
+        if (++b >= p.batch) return false;
+        n = p.b_seq_len[b];
+      } while (n <= 0);
+      req = p.b_req_idx[b];
+    }
+    cut();
+    return true;
+  }
+};
+
+// ------------------------------------------------------------------ score MMAs (one warp)
+__device__ __forceinline__ void score_role(const TcArgs& ta, const Share& sh, uint32_t sbase, uint32_t tmem) {
+  using C = Cfg;
+  const WsvdLatentDecodeParams& p = ta.k.p;
+  const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG;
+  auto bar = [&](int i) { return sbase + C::kOffBar + 8u * i; };
+  // descriptors: only the start-address field changes between k-steps, buffers and pairs
+  const uint64_t adesc0 = smem_desc_sw128(sbase + C::kOffA), bdesc0 = smem_desc_sw128(sbase + C::kOffB);
+  const uint32_t a_lo = (uint32_t)adesc0, b_lo = (uint32_t)bdesc0, d_hi = (uint32_t)(adesc0 >> 32);
+  const bool issuer = elect_one();
+  Walk w;
+  bool ok = true;
+  uint32_t T = 0, u = 0, item = 0;  // tiles, (tile, pair) units (unit u uses W buffer u % kWBufs) and items so far
+  for (bool more = w.start(ta, sh, n_hg); more && ok; more = w.next(p, n_hg), ++item) {
+    const int G = min(C::kG, p.n_q_heads - w.hg * C::kG), npairs = (G + 1) >> 1;
+    ok = warp_wait(bar(C::kBarPq), item & 1);
+    for (int t = 0; t < w.ntiles && ok; ++t, ++T) {
+      const uint32_t buf = T & 1;
+      ok = warp_wait(bar(C::kBarAFull + buf), (T >> 1) & 1);
+      for (int pr = 0; pr < npairs && ok; ++pr, ++u) {
+        const uint32_t wb = u % C::kWBufs, use = u / C::kWBufs;
+        if (use > 0) ok = warp_wait(bar(C::kBarWEmpty + wb), (use - 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t idesc = instr_desc_f16(kTile, kRkMax * min(2, G - 2 * pr));
+        const uint32_t d_tmem = tmem + wb * 128;
+        const uint32_t a_at = a_lo + buf * (kABufBytes >> 4), b_at = b_lo + pr * ((2 * kRkMax * 128) >> 4);
+        if (issuer) {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            umma_f16(d_tmem, join64(a_at + (((kk >> 2) * kAHalfBytes + (kk & 3) * 32) >> 4), d_hi),
+                     join64(b_at + (((kk >> 2) * C::kBHalfBytes + (kk & 3) * 32) >> 4), d_hi), idesc, kk > 0);
+          umma_commit(bar(C::kBarWFull + wb));
+          if (pr == npairs - 1) umma_commit(bar(C::kBarAEmpty + buf));
+        }
+        __syncwarp();
+      }
+    }
+  }
+  // the releases of the last two table buffers are arrivals that nobody else waits for: none may be on
+  // its way when the CTA exits
+  for (uint32_t t = T < 2 ? 0 : T - 2; t < T && ok; ++t) ok = warp_wait(bar(C::kBarAEmpty + (t & 1)), (t >> 1) & 1);
+  if (!ok) atomicMax(&g_status, (unsigned)kTimeoutMma);
+}
+
+// ------------------------------------------------------------------ copies (one warp)
+// Per tile, in this order, each as soon as its slot is free: the table tile (free when the score MMAs of the
+// tile two before it are complete), the K rows (when every warp has copied the rows of the tile before to
+// registers), the V rows (when the value MMAs of the tile two before are complete).  The warp runs on into
+// the next item while the epilogue finishes the last one.
+// A tensor copy needs token slots that are consecutive.  The warp checks that tile by tile: lane l holds the
+// page entries of tokens 4l..4l+3 (fetched one tile ahead), and the warp votes.
+//  - the tile's 128 slots are one run (a cache laid out sequence by sequence, a page of 128 or more): one copy
+//    for K and one for V fetch all heads of the group;
+//  - every aligned group of 16 tokens is a run (pages of 16, 32, 64 slots): lane l copies run l / 4 of KV
+//    head l % 4, 1 KB a copy;
+//  - else the epilogue's threads fetch their own tokens' rows (kTileGather), and this warp asks L2 for them.
+__device__ __forceinline__ void copy_role(const TcArgs& ta, const Share& sh, uint32_t sbase, uint8_t* sm) {
+  using C = Cfg;
+  const WsvdLatentDecodeParams& p = ta.k.p;
+  const int lane = threadIdx.x & 31;
+  const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG, gqa = p.n_q_heads / p.n_kv_heads;
+  auto bar = [&](int i) { return sbase + C::kOffBar + 8u * i; };
+  volatile int* mode = reinterpret_cast<volatile int*>(sm + C::kOffMode);
+  const bool issuer = elect_one();
+  const uint32_t box_bytes = ta.box_heads * C::kHeadBytes;
+  const bool use_tma = ta.use_tma != 0;
+  Walk w;
+  bool ok = true;
+  uint32_t T = 0;
+  for (bool more = w.start(ta, sh, n_hg); more && ok; more = w.next(p, n_hg)) {
+    const int h0 = w.hg * C::kG, G = min(C::kG, p.n_q_heads - h0);
+    const int hk0 = h0 / gqa, nkv = (h0 + G - 1) / gqa - hk0 + 1;  // the group's KV heads
+    const int32_t* page = p.req_to_token + (int64_t)w.req * p.rtt_stride;
+    int pos = (p.pos_offset != nullptr ? p.pos_offset[w.b] : 0) + w.lo;  // RoPE position of the tile's first token
+    int ent[4];
+    auto fetch_entries = [&](int t) {
+      const int s0 = w.lo + t * kTile + 4 * lane;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ent[j] = s0 + j < w.hi ? page[s0 + j] : -1;
+    };
+    fetch_entries(0);
+    for (int t = 0; t < w.ntiles && ok; ++t, ++T, pos += kTile) {
+      // ---- position table
+      const uint32_t buf = T & 1;
+      if (T >= 2) ok = warp_wait(bar(C::kBarAEmpty + buf), ((T >> 1) - 1) & 1);
+      if (!ok) break;
+      if (issuer) {
+        mbar_expect_tx(bar(C::kBarAFull + buf), kABufBytes);
+        tma_load_3d(sbase + C::kOffA + buf * kABufBytes, &ta.tmap_table, 0, pos, 0, bar(C::kBarAFull + buf));
+      }
+      // ---- which way the rows come (entries past the end are -1 and match anything)
+      const int first = __shfl_sync(0xffffffffu, ent[0], 0);
+      bool good = use_tma;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) good = good && (ent[j] < 0 || ent[j] == first + 4 * lane + j);
+      const bool run = __all_sync(0xffffffffu, good);
+      const int first16 = __shfl_sync(0xffffffffu, ent[0], lane & ~3);
+      bool run16 = false;
+      int groups = 0;  // groups of 16 that hold tokens
+      if (!run) {
+        good = use_tma;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) good = good && (ent[j] < 0 || ent[j] == first16 + 4 * (lane & 3) + j);
+        run16 = __all_sync(0xffffffffu, good);
+        groups = __popc(__ballot_sync(0xffffffffu, first16 >= 0)) >> 2;
+        if (!run16) {
+#pragma unroll 1
+          for (int j = 0; j < 4; ++j) {
+            if (ent[j] < 0) continue;
+            for (int hk = hk0; hk < hk0 + nkv; ++hk) {
+              prefetch_l2(reinterpret_cast<const uint8_t*>(p.latent_k) +
+                          (C::kRowBytes / 64) * ((int64_t)ent[j] * p.k_stride_t + (int64_t)hk * p.k_stride_h));
+              prefetch_l2(reinterpret_cast<const uint8_t*>(p.latent_v) +
+                          (C::kRowBytes / 64) * ((int64_t)ent[j] * p.v_stride_t + (int64_t)hk * p.v_stride_h));
+            }
+          }
+        }
+      }
+      if (t + 1 < w.ntiles) fetch_entries(t + 1);
+      auto request = [&](const CUtensorMap* whole, const CUtensorMap* part, uint32_t dst, uint32_t full, bool is_k) {
+        if (run) {
+          if (issuer) {
+            if (is_k) mode[T & 3] = kTileCopied;
+            mbar_expect_tx(full, box_bytes);
+            tma_load_3d(dst, whole, 0, first, hk0, full);
+          }
+        } else if (run16) {
+          if (issuer) {
+            if (is_k) mode[T & 3] = kTileCopied;
+            mbar_expect_tx(full, (uint32_t)(groups * nkv) * (16u * C::kRowBytes));
+          }
+          __syncwarp();
+          const int j = lane & 3;
+          if (j < nkv && first16 >= 0)
+            tma_load_3d(dst + j * C::kHeadBytes + (lane >> 2) * (16 * C::kRowBytes), part, 0, first16, hk0 + j, full);
+        } else if (issuer) {
+          if (is_k) mode[T & 3] = kTileGather;
+          mbar_arrive(full);
+        }
+      };
+      // ---- K rows, V rows
+      const uint32_t ks = T % C::kKSlots, ku = T / C::kKSlots, vs = T % C::kVSlots, vu = T / C::kVSlots;
+      if (ku > 0) ok = warp_wait(bar(C::kBarKEmpty + ks), (ku - 1) & 1);
+      if (!ok) break;
+      request(&ta.tmap_k, &ta.tmap_k16, sbase + C::kOffK + ks * C::kUnitBytes, bar(C::kBarKFull + ks), true);
+      if (vu > 0) ok = warp_wait(bar(C::kBarVEmpty + vs), (vu - 1) & 1);
+      if (!ok) break;
+      request(&ta.tmap_v, &ta.tmap_v16, sbase + C::kOffV + vs * C::kUnitBytes, bar(C::kBarVFull + vs), false);
+    }
+  }
+  // as in the score role: the releases of the last V slots
+  for (uint32_t t = T < C::kVSlots ? 0 : T - C::kVSlots; t < T && ok; ++t)
+    ok = warp_wait(bar(C::kBarVEmpty + t % C::kVSlots), (t / C::kVSlots) & 1);
+  if (!ok) atomicMax(&g_status, (unsigned)kTimeoutProducer);
+}
+
+// ------------------------------------------------------------------ value MMAs (one warp per pair of heads)
+// Lane 0 and lane 1 serve one head each: they wait for the digit planes of the head's four warps and issue the
+// head's value MMAs (one per warp of 32 tokens, each into its own 8 columns of tensor memory); two commits
+// then tell the epilogue warps (D full) and the copying warp (V empty) when the MMAs have completed.
+__device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, uint32_t sbase, const uint8_t* sm,
+                                           uint32_t tmem, int pair) {
+  using C = Cfg;
+  const WsvdLatentDecodeParams& p = ta.k.p;
+  const int lane = threadIdx.x & 31;
+  const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG, gqa = p.n_q_heads / p.n_kv_heads;
+  auto bar = [&](int i) { return sbase + C::kOffBar + 8u * i; };
+  const int g = 2 * pair + lane;
+  const uint32_t idesc = instr_desc_i8(64, 8);
+  const uint64_t pdesc0 = smem_desc_k_plain(sbase + C::kOffPlanes + 2 * g * C::kPlaneBytes);
+  const uint32_t d_tmem = tmem + C::kTmemD + 32 * g;
+  const volatile int* mode = reinterpret_cast<const volatile int*>(sm + C::kOffMode);
+  const uint64_t vdesc0 = smem_desc_mn_sw64(sbase + C::kOffV);
+  Walk w;
+  bool ok = true;
+  uint32_t T = 0, mine = 0;  // tiles so far, and those this head took part in
+  if (lane < 2) {
+    for (bool more = w.start(ta, sh, n_hg); more && ok; more = w.next(p, n_hg)) {
+      const int h0 = w.hg * C::kG, G = min(C::kG, p.n_q_heads - h0);
+      if (g >= G) {
+        T += w.ntiles;
+        continue;
+      }
+      const int sub = (h0 + g) / gqa - h0 / gqa;
+      for (int t = 0; t < w.ntiles && ok; ++t, ++T, ++mine) {
+        const uint32_t vslot = T % C::kVSlots;
+        // the V rows arrive long before the planes are ready: wait for them first, off the
+        // critical path from "planes ready" to "D full"
+        ok = mbar_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
+        if (ok) ok = mbar_wait(bar(C::kBarPlanes + g), mine & 1);
+        if (ok) {
+          tc_fence_after();
+          // copied rows sit at the head's KV head, gathered ones at the head itself
+          const uint32_t region = vslot * C::kUnitBytes + (mode[T & 3] == kTileGather ? g : sub) * C::kHeadBytes;
+#pragma unroll
+          for (int w4 = 0; w4 < 4; ++w4) {
+            const uint32_t voff = region + w4 * 2048;  // the 32 tokens of warp w4: 32 rows of 64 bytes
+            umma_i8(d_tmem + 8 * w4, vdesc0 + (voff >> 4), pdesc0 + (((w4 >> 1) * C::kPlaneBytes) >> 4), idesc, 0);
+          }
+          umma_commit(bar(C::kBarDFull + g));
+          umma_commit(bar(C::kBarVEmpty + vslot));
+          if (g == 0 && G < C::kG) mbar_arrive_n(bar(C::kBarVEmpty + vslot), C::kG - G);  // for the heads that are not there
+        }
+      }
+    }
+  }
+  if (!ok) atomicMax(&g_status, (unsigned)kTimeoutProducer);
+}
+
+// ------------------------------------------------------------------ epilogue (four warps per head)
+// Where chunk ic (8 frequencies) of rank r of head g sits in either half of the B operand.
+__device__ __forceinline__ uint32_t pq_off(int g, int r, int ic) {
+  const int nrow = g * kRkMax + r;
+  return nrow * 128 + ((ic ^ (nrow & 7)) << 4);
+}
+
+// Asks for what the [P;Q] build of an item needs from memory: the head's slice of wk goes, without passing
+// through registers, to the places in the B operand that the thread which asked for it will overwrite with P
+// and Q; the page entries of the first two tiles go to L1.
+__device__ __forceinline__ void request_pq(const TcArgs& ta, uint32_t sbase, const Walk& w, int g, bool wk_vec) {
+  using C = Cfg;
+  const WsvdLatentDecodeParams& p = ta.k.p;
+  const int gqa = p.n_q_heads / p.n_kv_heads, hk = (w.hg * C::kG + g) / gqa;
+  const bool il = p.rope_layout == WSVD_ROPE_INTERLEAVED, wk_i8 = p.wk_dtype == WSVD_I8;
+  const int tid = threadIdx.x & 127, ic = tid & 7;
+  const int d0 = il ? ic * 16 : ic * 8, d1 = il ? ic * 16 + 8 : 64 + ic * 8;
+  if (wk_vec) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = (tid + 128 * i) >> 3;
+      if (r >= p.rank_k) continue;
+      const uint32_t dst = sbase + C::kOffB + pq_off(g, r, ic);
+      const int64_t at = (int64_t)r * p.wk_stride_r + (int64_t)hk * 128;
+      if (wk_i8) {
+        const int8_t* s = reinterpret_cast<const int8_t*>(p.wk) + at;
+        cp_async8(dst, s + d0);
+        cp_async8(dst + C::kBHalfBytes, s + d1);
+      } else {
+        const __half* s = reinterpret_cast<const __half*>(p.wk) + at;
+        cp_async16(dst, s + d0);
+        cp_async16(dst + C::kBHalfBytes, s + d1);
+      }
+    }
+  }
+  const int32_t* page = p.req_to_token + (int64_t)w.req * p.rtt_stride;
+  const int s_first = w.lo + tid;
+  if (s_first < w.hi) asm volatile("prefetch.global.L1 [%0];" ::"l"(page + s_first));
+  if (s_first + kTile < w.hi) asm volatile("prefetch.global.L1 [%0];" ::"l"(page + s_first + kTile));
+}
+
+// B operand: P (cos coefficients) and Q (sin coefficients) of head g of the group, f16, rows n = g*64 + r, 64
+// frequencies per row, 128-byte swizzle; rows r >= rank_k are zero.
+__device__ __forceinline__ void build_pq(const TcArgs& ta, uint8_t* sm, int b, int h, int hk, int g, bool wk_vec) {
+  using C = Cfg;
   const KArgs& a = ta.k;
   const WsvdLatentDecodeParams& p = a.p;
-  const int gqa = p.n_q_heads / p.n_kv_heads;
-  const int Rk = p.rank_k, Rv = p.rank_v;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_hg = (p.n_q_heads + kG - 1) / kG;
+  const bool interleaved = p.rope_layout == WSVD_ROPE_INTERLEAVED, wk_i8 = p.wk_dtype == WSVD_I8;
+  const int tid = threadIdx.x & 127;
+  uint4 qv0, qv1;  // the 16 query values of this thread's chunk of 8 frequencies
+  {
+    const int ic = tid & 7;
+    const __half* qp = reinterpret_cast<const __half*>(p.q) + (int64_t)b * p.q_stride_b + (int64_t)h * p.q_stride_h;
+    qv0 = *reinterpret_cast<const uint4*>(qp + (interleaved ? ic * 16 : ic * 8));
+    qv1 = *reinterpret_cast<const uint4*>(qp + (interleaved ? ic * 16 + 8 : 64 + ic * 8));
+  }
+  cp_async_wait_all();  // this thread's own pieces of wk
+  // q * sm_scale * log2(e) (scores come out in the log2 domain): qlo[e] pairs with dimension
+  // d0 and qhi[e] with its rotation partner d1 of frequency ic*8 + e
+  float qlo[8], qhi[8];
+  {
+    const float qscale = a.sm_scale * 1.4426950408889634f;
+    const __half* q0 = reinterpret_cast<const __half*>(&qv0);
+    const __half* q1 = reinterpret_cast<const __half*>(&qv1);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if (interleaved) {
+        const __half* src = e < 4 ? q0 : q1;
+        qlo[e] = __half2float(src[(2 * e) & 7]) * qscale;
+        qhi[e] = __half2float(src[(2 * e + 1) & 7]) * qscale;
+      } else {
+        qlo[e] = __half2float(q0[e]) * qscale;
+        qhi[e] = __half2float(q1[e]) * qscale;
+      }
+    }
+  }
+  const int64_t col = (int64_t)hk * 128;
+  if (wk_vec && !wk_i8 && !interleaved) {
+    // Common case (f16 wk, half-split pairing): packed f16 arithmetic.  The operands are
+    // rounded to f16 for the MMA anyway; forming them with one extra f16 rounding of a
+    // product keeps the error of the scores within a few 1e-5.  This thread's chunk of 8
+    // frequencies is the same for its four ranks, so q is converted once.
+    const int ic = tid & 7;
+    __half2 qa[4], qb[4], nqa[4];
+    {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        qa[e] = __floats2half2_rn(qlo[2 * e], qlo[2 * e + 1]);
+        qb[e] = __floats2half2_rn(qhi[2 * e], qhi[2 * e + 1]);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) nqa[e] = __hneg2(qa[e]);
+    }
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int r = (tid + 128 * it) >> 3;
+      const uint32_t off = pq_off(g, r, ic);
+      uint4 u_lo = make_uint4(0u, 0u, 0u, 0u), u_hi = u_lo;
+      if (r < p.rank_k) {
+        u_lo = *reinterpret_cast<const uint4*>(sm + C::kOffB + off);
+        u_hi = *reinterpret_cast<const uint4*>(sm + C::kOffB + C::kBHalfBytes + off);
+      }
+      const __half2* ua = reinterpret_cast<const __half2*>(&u_lo);  // U[d = ic*8 .. +7]
+      const __half2* ub = reinterpret_cast<const __half2*>(&u_hi);  // U[64 + ic*8 .. +7]
+      __align__(16) __half2 pv[4];
+      __align__(16) __half2 qv[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        pv[e] = __hfma2(qa[e], ua[e], __hmul2(qb[e], ub[e]));   // P = q_i U_i + q_{i+64} U_{i+64}
+        qv[e] = __hfma2(nqa[e], ub[e], __hmul2(qb[e], ua[e]));  // Q = q_{i+64} U_i - q_i U_{i+64}
+      }
+      *reinterpret_cast<uint4*>(sm + C::kOffB + off) = *reinterpret_cast<const uint4*>(pv);
+      *reinterpret_cast<uint4*>(sm + C::kOffB + C::kBHalfBytes + off) = *reinterpret_cast<const uint4*>(qv);
+    }
+  } else if (wk_vec && wk_i8) {
+    // int8 wk in vectors of eight; the columns' scales are this thread's for all four ranks.  fp32 throughout.
+    const int ic = tid & 7;
+    const __half* ws = reinterpret_cast<const __half*>(p.wk_scale) + col;
+    const uint4 s0v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 : ic * 8));
+    const uint4 s1v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 + 8 : 64 + ic * 8));
+    const __half* s0h = reinterpret_cast<const __half*>(&s0v);
+    const __half* s1h = reinterpret_cast<const __half*>(&s1v);
+#pragma unroll 1
+    for (int it = 0; it < 4; ++it) {
+      const int r = (tid + 128 * it) >> 3;
+      const uint32_t off = pq_off(g, r, ic);
+      uint2 b0 = make_uint2(0u, 0u), b1 = b0;
+      if (r < p.rank_k) {
+        b0 = *reinterpret_cast<const uint2*>(sm + C::kOffB + off);
+        b1 = *reinterpret_cast<const uint2*>(sm + C::kOffB + C::kBHalfBytes + off);
+      }
+      __align__(16) __half pv[8];
+      __align__(16) __half qv[8];
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        // bytes of dimension d0 and d1 of four frequencies
+        uint32_t w0, w1;
+        if (interleaved) {
+          const uint2 src = half == 0 ? b0 : b1;
+          w0 = __byte_perm(src.x, src.y, 0x6420);
+          w1 = __byte_perm(src.x, src.y, 0x7531);
+        } else {
+          w0 = half == 0 ? b0.x : b0.y;
+          w1 = half == 0 ? b1.x : b1.y;
+        }
+        const __half* pair = half == 0 ? s0h : s1h;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int e = 4 * half + j;
+          const float s0 = __half2float(interleaved ? pair[(2 * e) & 7] : s0h[e]);
+          const float s1 = __half2float(interleaved ? pair[(2 * e + 1) & 7] : s1h[e]);
+          const float u0 = (float)(int8_t)(w0 >> (8 * j)) * s0, u1 = (float)(int8_t)(w1 >> (8 * j)) * s1;
+          pv[e] = __float2half_rn(qlo[e] * u0 + qhi[e] * u1);
+          qv[e] = __float2half_rn(qhi[e] * u0 - qlo[e] * u1);
+        }
+      }
+      *reinterpret_cast<uint4*>(sm + C::kOffB + off) = *reinterpret_cast<const uint4*>(pv);
+      *reinterpret_cast<uint4*>(sm + C::kOffB + C::kBHalfBytes + off) = *reinterpret_cast<const uint4*>(qv);
+    }
+  } else
+#pragma unroll 1
+  for (int it = 0; it < 4; ++it) {
+    const int task = tid + 128 * it;
+    const int r = task >> 3, ic = task & 7;  // rank, chunk of 8 frequencies
+    float u0[8], u1[8];
+    if (r >= p.rank_k) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) u0[e] = u1[e] = 0.f;
+    } else if (wk_vec) {
+      // half layout: dims ic*8.. and 64+ic*8..; interleaved: 16 consecutive dims
+      const uint4 a0 = *reinterpret_cast<const uint4*>(sm + C::kOffB + pq_off(g, r, ic));
+      const uint4 a1 = *reinterpret_cast<const uint4*>(sm + C::kOffB + C::kBHalfBytes + pq_off(g, r, ic));
+      const __half* h0p = reinterpret_cast<const __half*>(&a0);
+      const __half* h1p = reinterpret_cast<const __half*>(&a1);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        if (interleaved) {
+          const __half* src = e < 4 ? h0p : h1p;
+          u0[e] = __half2float(src[(2 * e) & 7]);
+          u1[e] = __half2float(src[(2 * e + 1) & 7]);
+        } else {
+          u0[e] = __half2float(h0p[e]);
+          u1[e] = __half2float(h1p[e]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int i = ic * 8 + e;
+        const int d0 = interleaved ? 2 * i : i, d1 = interleaved ? 2 * i + 1 : i + 64;
+        if (p.wk_dtype == WSVD_I8) {
+          const int8_t* w = reinterpret_cast<const int8_t*>(p.wk) + (int64_t)r * p.wk_stride_r + col;
+          const __half* ws = reinterpret_cast<const __half*>(p.wk_scale) + col;
+          u0[e] = (float)w[d0] * __half2float(ws[d0]);
+          u1[e] = (float)w[d1] * __half2float(ws[d1]);
+        } else {
+          const __half* w = reinterpret_cast<const __half*>(p.wk) + (int64_t)r * p.wk_stride_r + col;
+          u0[e] = __half2float(w[d0]);
+          u1[e] = __half2float(w[d1]);
+        }
+      }
+    }
+    __align__(16) __half pv[8];
+    __align__(16) __half qv[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      pv[e] = __float2half_rn(qlo[e] * u0[e] + qhi[e] * u1[e]);
+      qv[e] = __float2half_rn(qhi[e] * u0[e] - qlo[e] * u1[e]);
+    }
+    const uint32_t off = pq_off(g, r, ic);
+    *reinterpret_cast<uint4*>(sm + C::kOffB + off) = *reinterpret_cast<const uint4*>(pv);
+    *reinterpret_cast<uint4*>(sm + C::kOffB + C::kBHalfBytes + off) = *reinterpret_cast<const uint4*>(qv);
+  }
+}
 
+// What a head's warps know of an item lives in shared memory ([head][item parity], every warp of the head writes
+// the same values): the registers are needed for the tile loop and the [P;Q] build, and state that is kept
+// in registers across both comes back as reloads from local memory inside the tile loop.
+enum ItemField { kItB, kItHg, kItLeft, kItBefore, kItN, kItReq, kItTilesB, kItLo, kItHi, kItTiles, kItT, kItUnits, kItMine, kItParts, kItFirst };
+
+__device__ __forceinline__ void put_item(volatile int* st, const Walk& w, uint32_t T, uint32_t units, uint32_t mine) {
+  if ((threadIdx.x & 31) == 0) {
+    st[kItB] = w.b, st[kItHg] = w.hg, st[kItLeft] = w.tiles_left, st[kItBefore] = w.before_b, st[kItN] = w.n, st[kItReq] = w.req;
+    st[kItTilesB] = w.tiles_b, st[kItLo] = w.lo, st[kItHi] = w.hi, st[kItTiles] = w.ntiles;
+    st[kItT] = (int)T, st[kItUnits] = (int)units, st[kItMine] = (int)mine;
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ Walk get_item(const volatile int* st) {
+  Walk w;
+  w.b = st[kItB], w.hg = st[kItHg], w.tiles_left = st[kItLeft], w.before_b = st[kItBefore], w.n = st[kItN], w.req = st[kItReq];
+  w.tiles_b = st[kItTilesB], w.lo = st[kItLo], w.hi = st[kItHi], w.ntiles = st[kItTiles], w.t_first = 0;
+  return w;
+}
+
+// Merges, projects and writes the output rows of a head whose last partial this CTA has delivered (or that it
+// covered alone: the latent-space row is in shared memory then).  Run by the head's 128 threads.
+// `seen`: for thread 0 of the head, the arrivals before this CTA's.
+__device__ __forceinline__ void finish_head(const TcArgs& ta, uint8_t* sm, int g, const volatile int* st, unsigned int seen) {
+  using C = Cfg;
+  const KArgs& a = ta.k;
+  const WsvdLatentDecodeParams& p = a.p;
+  const int d = threadIdx.x & 127, Rv = p.rank_v;
+  const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG;
+  struct { int b, hg, n_parts, c_first; } const f = {st[kItB], st[kItHg], st[kItParts], st[kItFirst]};
+  const int h = f.hg * C::kG + g, hk = h / (p.n_q_heads / p.n_kv_heads);
+  float* o_row = reinterpret_cast<float*>(sm + C::kOffPlanes + 2 * g * C::kPlaneBytes);
+  int* verdict = reinterpret_cast<int*>(sm + C::kOffSum) + g * 8;  // the head's (max, sum) pairs were read before
+  auto head_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(128) : "memory"); };
+  if (f.n_parts > 1) {
+    // the CTA that adds the head's last partial merges them all
+    if (d == 0) {
+      __threadfence();
+      verdict[0] = seen + 1u == (unsigned int)f.n_parts;
+    }
+    head_sync();
+    if (verdict[0] == 0) return;
+    const int64_t slot0 = ((int64_t)f.b * n_hg + f.hg + f.c_first) * C::kG + g;
+    // the first four partials (a head is rarely shared by more CTAs) are requested at once
+    float ls[4], mo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      ls[i] = i < f.n_parts ? __ldcg(a.lse + slot0 + (int64_t)i * C::kG) : -INFINITY;
+      mo[i] = i < f.n_parts && d < Rv ? __ldcg(a.mid_o + (slot0 + (int64_t)i * C::kG) * Rv + d) : 0.f;
+    }
+    float m = fmaxf(fmaxf(ls[0], ls[1]), fmaxf(ls[2], ls[3]));
+    for (int i = 4; i < f.n_parts; ++i) m = fmaxf(m, __ldcg(a.lse + slot0 + (int64_t)i * C::kG));
+    float wsum = 0.f, osum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float w = ls[i] > -INFINITY ? __expf(ls[i] - m) : 0.f;
+      wsum += w;
+      osum = fmaf(w, mo[i], osum);
+    }
+    for (int i = 4; i < f.n_parts; ++i) {
+      const float w = __expf(__ldcg(a.lse + slot0 + (int64_t)i * C::kG) - m);
+      wsum += w;
+      if (d < Rv) osum = fmaf(w, __ldcg(a.mid_o + (slot0 + (int64_t)i * C::kG) * Rv + d), osum);
+    }
+    if (d < Rv) o_row[d] = osum / wsum;
+  }
+  head_sync();
+  // with peers the finished row is staged (second half of the head's plane area) and leaves as
+  // 16-byte stores, one per thread per peer
+  __half* stage = reinterpret_cast<__half*>(sm + C::kOffPlanes + 2 * g * C::kPlaneBytes + C::kPlaneBytes);
+  __half* out = ta.has_peers ? stage
+                             : reinterpret_cast<__half*>(p.out) + (int64_t)f.b * p.out_stride_b + (int64_t)h * p.out_stride_h;
+  if (p.wv == nullptr) {
+    if (d < Rv) out[d] = __float2half_rn(o_row[d]);
+  } else {
+    // out[d] = sum_r O_lat[r] U_v[r, hk*128 + d]: consecutive d in consecutive lanes, four sums and
+    // 32 loads of U_v (L2) in flight
+    const __half* w = reinterpret_cast<const __half*>(p.wv) + (int64_t)hk * p.head_dim + d;
+    float y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < Rv; k += 4) {
+      y0 = fmaf(o_row[k], __half2float(__ldg(w + (int64_t)k * p.wv_stride_r)), y0);
+      y1 = fmaf(o_row[k + 1], __half2float(__ldg(w + (int64_t)(k + 1) * p.wv_stride_r)), y1);
+      y2 = fmaf(o_row[k + 2], __half2float(__ldg(w + (int64_t)(k + 2) * p.wv_stride_r)), y2);
+      y3 = fmaf(o_row[k + 3], __half2float(__ldg(w + (int64_t)(k + 3) * p.wv_stride_r)), y3);
+    }
+    out[d] = __float2half_rn((y0 + y1) + (y2 + y3));
+  }
+  head_sync();  // o_row has been read (and the staged row is complete): the next item's planes may go there
+  if (ta.has_peers) {
+    const int chunks = (p.wv == nullptr ? Rv : p.head_dim) >> 3;
+    const int64_t doff = (int64_t)f.b * ta.peers.out_stride_b + (int64_t)(h + ta.peers.head_offset) * ta.peers.out_stride_h;
+    for (int idx = d; idx < chunks * ta.peers.n_peers; idx += 128) {
+      const int peer = idx / chunks, c = idx - peer * chunks;
+      *reinterpret_cast<uint4*>(ta.peers.out[peer] + doff + 8 * c) = reinterpret_cast<const uint4*>(stage)[c];
+    }
+    head_sync();
+  }
+}
+
+__device__ __forceinline__ volatile int* item_state(uint8_t* sm, int g, uint32_t item) {
+  return reinterpret_cast<volatile int*>(sm + Cfg::kOffItem) + (g * 2 + (item & 1)) * 16;
+}
+
+// One head's running sums over the tiles of an item.
+struct HeadSums {
+  float m_run, l_lane;  // softmax denominator of this lane's tokens, under the warp's running maximum of z
+  float big_m, acc;     // value sum of rank 16*q4 + lane (lanes 0..15), all four warps' tokens, under the running
+                        // reference big_m (max y of every (tile, warp) folded in so far)
+};
+
+// Fold in the value sums of the head's tile number tp: D[rank][8*w + 0..2] are the three digit-plane sums over
+// the 32 tokens of warp w, whose weights were taken relative to refs[tp & 1][w].
+__device__ __forceinline__ void fold_values(HeadSums& hs, uint32_t d_addr, const float* refs, uint32_t tp) {
+  uint32_t d[4][4];
+#pragma unroll
+  for (int w4 = 0; w4 < 4; ++w4) tmem_ld4(d_addr + 8 * w4 + 3 * (w4 & 1), d[w4]);
+  const float4 rf = *reinterpret_cast<const float4*>(refs + (tp & 1) * 4);
+  const float ref[4] = {rf.x, rf.y, rf.z, rf.w};
+  tmem_wait_ld();
+  float m_new = hs.big_m;
+#pragma unroll
+  for (int w4 = 0; w4 < 4; ++w4) m_new = fmaxf(m_new, ref[w4]);
+  if (m_new > -INFINITY) {
+    hs.acc *= fast_exp2(hs.big_m - m_new);  // big_m = -inf -> factor 0
+#pragma unroll
+    for (int w4 = 0; w4 < 4; ++w4) {
+      if (ref[w4] > -INFINITY) {  // (a warp without tokens in this tile has no MMA and reference -inf)
+        // the two low digit sums are combined as integers (|d| <= 32 * 255 * 128 < 2^21)
+        const float v = fmaf((float)(int32_t)d[w4][2], 65536.f, (float)((int32_t)d[w4][1] * 256 + (int32_t)d[w4][0]));
+        hs.acc = fmaf(v, fast_exp2(ref[w4] - m_new) * (1.f / kPlaneScale), hs.acc);
+      }
+    }
+    hs.big_m = m_new;
+  }
+}
+
+// The tiles of an item, for one warp of a head that is there.
+__device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_t item, HeadSums& hs) {
+  using C = Cfg;
+  const WsvdLatentDecodeParams& p = ta.k.p;
+  const int tid = fresh_tid(), lane = tid & 31, g = tid >> 7, row = tid & 127, q4 = row >> 5;
   const uint32_t sbase = smem_u32(sm);
-  const uint32_t sB = sbase + kOffB, sA = sbase + kOffA, sV = sbase + kOffV, sK = sbase + kOffK;
-  const uint32_t sPl = sbase + kOffPlanes;
-  uint32_t bars = sbase + kOffBar;
-  auto bar = [&](int i) { return bars + 8u * i; };
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + kOffTmemSlot);
+  auto bar = [&](int i) { return sbase + C::kOffBar + 8u * i; };
+  const int gqa = p.n_q_heads / p.n_kv_heads, Rv = p.rank_v;
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + C::kOffTmemSlot);
+  const volatile int* st = item_state(sm, g, item);
+  const volatile int* mode = reinterpret_cast<const volatile int*>(sm + C::kOffMode);
+  float* refs = reinterpret_cast<float*>(sm + C::kOffRef) + g * 8;  // [tile parity][warp]: max y the warp's planes refer to
+  // Digit planes: the two warps of half a tile share one 8-row block (the MMA's B operand has 8
+  // rows): rows 0..2 hold the even warp's digits, rows 3..5 the odd warp's.  Each warp's MMA reads
+  // the whole block, so its columns 3..5 (or 0..2) are the other warp's weights times this warp's
+  // V rows: garbage that nobody reads.  Rows 6 and 7 are never written.
+  const uint32_t my_planes = sbase + C::kOffPlanes + (2 * g + (q4 >> 1)) * C::kPlaneBytes + (lane >> 4) * 128 + (q4 & 1) * 48 + (lane & 15);
+  const uint32_t d_addr = tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 32 * g;
+  const int h0 = st[kItHg] * C::kG, G = min(C::kG, p.n_q_heads - h0), npairs = (G + 1) >> 1;
+  bool ok = true;
+  const int hk = (h0 + g) / gqa;
+  const int pr = g >> 1, sub = hk - h0 / gqa;  // sub: this head's KV head inside a unit
+  const int lo = st[kItLo], hi = st[kItHi], ntiles = st[kItTiles];
+  int slot_c, slot_n;
+  unsigned short sk_raw = 0, sv_raw = 0;
+  const uint32_t T = st[kItT], ub = st[kItUnits], mine = st[kItMine];
+  const int32_t* page = p.req_to_token + (int64_t)st[kItReq] * p.rtt_stride;
+  const __half* ksc = reinterpret_cast<const __half*>(p.k_scale) + (int64_t)hk * p.ks_stride_h;
+  const __half* vsc = reinterpret_cast<const __half*>(p.v_scale) + (int64_t)hk * p.vs_stride_h;
+  // counts that stay the same when the last group is not full: its first head arrives for the missing
+  // ones, and a pair that holds a single head arrives twice
+  const uint32_t k_arrivals = g == 0 ? 1u + (C::kG - G) : 1u;
+  const uint32_t w_arrivals = (G - 2 * pr) >= 2 ? 1u : 2u;
+  // this lane's first token and its next one (the lines were asked for with the item's other loads)
+  slot_c = lo + row < hi ? page[lo + row] : -1;
+  slot_n = lo + kTile + row < hi ? page[lo + kTile + row] : -1;
+  if (slot_c >= 0) {
+    sk_raw = reinterpret_cast<const unsigned short*>(ksc)[(int64_t)slot_c * p.ks_stride_t];
+    sv_raw = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_c * p.vs_stride_t];
+  }
+  for (int t = 0; t < ntiles && ok; ++t) {
+    const int s = lo + t * kTile + row;
+    const bool valid = s < hi;
+    const uint32_t Tt = T + t, u = ub + t * npairs + pr, wb = u % C::kWBufs, mt = mine + t;
+    // ---- the next tile's scales and the page entry of the tile after it: requested a whole
+    //      tile before they are used
+    unsigned short sk_n = 0, sv_n = 0;
+    if (slot_n >= 0) {
+      sk_n = reinterpret_cast<const unsigned short*>(ksc)[(int64_t)slot_n * p.ks_stride_t];
+      sv_n = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_n * p.vs_stride_t];
+    }
+    const int slot_t = slot_c;
+    slot_c = slot_n;
+    slot_n = -1;
+    if (s + 2 * kTile < hi) slot_n = page[s + 2 * kTile];
+    // ---- this warp's 32 K rows (lane = token) go from the ring slot to registers at once and
+    //      the slot is handed back: its refill has the whole tile to arrive
+    uint4 kreg[4];
+    const uint32_t kslot = Tt % C::kKSlots;
+    ok = mbar_wait(bar(C::kBarKFull + kslot), (Tt / C::kKSlots) & 1);
+    if (!ok) break;
+    const bool gather = mode[Tt & 3] == kTileGather;
+    if (!gather) {
+      const uint32_t krows = sbase + C::kOffK + kslot * C::kUnitBytes + sub * C::kHeadBytes;
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(kreg[c].x), "=r"(kreg[c].y), "=r"(kreg[c].z), "=r"(kreg[c].w)
+                     : "r"(krows + latent_off(row, c)));
+    } else {
+      const uint8_t* src = reinterpret_cast<const uint8_t*>(p.latent_k) + (int64_t)slot_t * p.k_stride_t + (int64_t)hk * p.k_stride_h;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        kreg[c] = make_uint4(0u, 0u, 0u, 0u);
+        if (valid && c * 16 < p.rank_k) kreg[c] = __ldg(reinterpret_cast<const uint4*>(src) + c);
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive_n(bar(C::kBarKEmpty + kslot), k_arrivals);
+    ok = mbar_wait(bar(C::kBarWFull + wb), (u / C::kWBufs) & 1);
+    if (!ok) break;
+    tc_fence_after();
+
+    // ---- score: dot of this token's int8 K row with its row of W, 16 ranks at a time
+    const uint32_t taddr = tmem + ((uint32_t)(q4 * 32) << 16) + wb * 128 + (g & 1) * kRkMax;
+    float2 dot0 = make_float2(0.f, 0.f), dot1 = make_float2(0.f, 0.f);
+    // two 16-column loads in flight alternately: the next chunk of W travels while this one is used
+    uint32_t wa[16], wb16[16];
+    auto mac16 = [&](const uint32_t (&wv)[16], const uint4 kq) {
+      const uint32_t kws[4] = {kq.x ^ 0x80808080u, kq.y ^ 0x80808080u, kq.z ^ 0x80808080u, kq.w ^ 0x80808080u};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float2 x01, x23;
+        cvt4(kws[j], x01, x23);
+        dot0 = __ffma2_rn(x01, make_float2(__uint_as_float(wv[4 * j]), __uint_as_float(wv[4 * j + 1])), dot0);
+        dot1 = __ffma2_rn(x23, make_float2(__uint_as_float(wv[4 * j + 2]), __uint_as_float(wv[4 * j + 3])), dot1);
+      }
+    };
+    tmem_ld16(taddr, wa);
+    tmem_wait_ld();
+    tmem_ld16(taddr + 16, wb16);
+    mac16(wa, kreg[0]);
+    tmem_wait_ld();
+    tmem_ld16(taddr + 32, wa);
+    mac16(wb16, kreg[1]);
+    tmem_wait_ld();
+    tmem_ld16(taddr + 48, wb16);
+    mac16(wa, kreg[2]);
+    tmem_wait_ld();
+    mac16(wb16, kreg[3]);
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive_n(bar(C::kBarWEmpty + wb), w_arrivals);  // this warp has read its rows of W
+    if (gather) {  // the V row of this token: requested now, stored once the slot is known to be free
+#pragma unroll
+      for (int c = 0; c < 4; ++c) kreg[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (valid) {
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(p.latent_v) + (int64_t)slot_t * p.v_stride_t + (int64_t)hk * p.v_stride_h;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (c * 16 < Rv) kreg[c] = __ldg(reinterpret_cast<const uint4*>(src) + c);
+      }
+    }
+    const float2 dsum = __fadd2_rn(dot0, dot1);
+    const float sk = __half2float(__ushort_as_half(sk_raw)), sv = __half2float(__ushort_as_half(sv_raw));
+    const float z = valid ? (dsum.x + dsum.y) * sk : -INFINITY;
+    const float y = valid ? z + fast_log2(sv) : -INFINITY;  // log2(0) = -inf: a zero scale drops the token's value
+    sk_raw = sk_n;
+    sv_raw = sv_n;
+
+    // ---- softmax denominator under this warp's own running max (fp32, by the owner threads)
+    const float mz_w = warp_max_redux(z), my_w = warp_max_redux(y);
+    if (mz_w > -INFINITY) {
+      const float m_new = fmaxf(hs.m_run, mz_w);
+      hs.l_lane = fmaf(hs.l_lane, fast_exp2(hs.m_run - m_new), fast_exp2(z - m_new));  // 2^-inf = 0: hs.m_run = -inf, masked tokens
+      hs.m_run = m_new;
+    }
+
+    // ---- the previous tile's value sums are in tensor memory by now: fold them in.  This also
+    //      orders this warp's reads of D and of the references (and, through the MMAs' completion,
+    //      the MMAs' reads of its digit planes and V rows) before those of this tile are written.
+    if (t > 0) {
+      ok = mbar_wait(bar(C::kBarDFull + g), (mt - 1) & 1);
+      if (!ok) break;
+      tc_fence_after();
+      fold_values(hs, d_addr, refs, mt - 1);
+    }
+    if (gather) {
+      // the copying warp's arrival says that every head's value MMAs on the slot are complete
+      ok = mbar_wait(bar(C::kBarVFull + Tt % C::kVSlots), (Tt / C::kVSlots) & 1);
+      if (!ok) break;
+      const uint32_t vrow = sbase + C::kOffV + (Tt % C::kVSlots) * C::kUnitBytes + g * C::kHeadBytes;
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(vrow + latent_off(row, c)), "r"(kreg[c].x),
+                     "r"(kreg[c].y), "r"(kreg[c].z), "r"(kreg[c].w)
+                     : "memory");
+    }
+
+    // ---- this token's weight for the value MMA, relative to the warp's largest, as three 8-bit digits
+    {
+      const float wgt = y > -INFINITY ? fast_exp2(y - my_w) : 0.f;  // <= 1
+      const uint32_t nq = __float2uint_rn(wgt * kPlaneScale);
+      asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes), "r"(nq) : "memory");
+      asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 16), "r"(nq >> 8) : "memory");
+      asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 32), "r"(nq >> 16) : "memory");
+    }
+    fence_proxy_async();
+    tc_fence_before();
+    if (lane == 0) refs[(mt & 1) * 4 + q4] = my_w;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(C::kBarPlanes + g));
+  }
+  return ok;
+}
+
+__device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh, uint8_t* sm, uint32_t sbase, uint32_t tmem) {
+  using C = Cfg;
+  const KArgs& a = ta.k;
+  const WsvdLatentDecodeParams& p = a.p;
+  const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG, gqa = p.n_q_heads / p.n_kv_heads;
+  const int Rv = p.rank_v;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = warp >> 2, q4 = warp & 3, row = q4 * 32 + lane;
+  auto bar = [&](int i) { return sbase + C::kOffBar + 8u * i; };
+  auto head_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(128) : "memory"); };
+  const bool balanced = ta.balanced != 0, fused = balanced && ta.arrivals != nullptr;
   // vector loads of eight values of wk need rows aligned to them: 16 bytes for f16, 8 bytes for int8
   // (whose scales are then read as 16-byte vectors too)
   const bool wk_i8 = p.wk_dtype == WSVD_I8;
   const bool wk_vec = (p.wk_stride_r & 7) == 0 &&
                       (wk_i8 ? (reinterpret_cast<uintptr_t>(p.wk) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.wk_scale) & 15) == 0
                              : (reinterpret_cast<uintptr_t>(p.wk) & 15) == 0);
+  auto state = [&](uint32_t i) { return item_state(sm, g, i); };
+  bool ok = true;  // after a wait that timed out: tiles are skipped, results are NaN
+  bool pending = false;  // the item before is still to be finished
+  unsigned int seen = 0;
+  {
+    Walk w;
+    if (!w.start(ta, sh, n_hg)) return;
+    if (g < p.n_q_heads - w.hg * C::kG) request_pq(ta, sbase, w, g, wk_vec);
+    put_item(state(0), w, 0, 0, 0);
+  }
+  for (uint32_t item = 0;; ++item) {
+    volatile int* st = state(item);
+    const int h0 = st[kItHg] * C::kG, G = min(C::kG, p.n_q_heads - h0), npairs = (G + 1) >> 1;
+    const bool active = g < G;
+    if (active) {
+      const int hk = (h0 + g) / gqa;
+      // The rows of this head in the B operand are free: this warp has seen W of the head's last tile, and
+      // with it the completion of every score MMA that read them.
+      build_pq(ta, sm, st[kItB], h0 + g, hk, g, wk_vec);
+      fence_proxy_async();
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(C::kBarPq));
+    // a warp whose head is not there must not arrive for the next item before this one's phase is over
+    if (!active && ok) ok = warp_wait(bar(C::kBarPq), item & 1);
+    if (pending) finish_head(ta, sm, g, state(item + 1), seen);  // the item before, while the first score MMAs of this one run
+    pending = false;
 
-  uint32_t tmem = 0;
-  // ---- this CTA's work: every thread walks the same items (uniform loads, no broadcast needed)
-  const bool balanced = ta.balanced != 0;
-  const bool fused = balanced && ta.arrivals != nullptr;
-  int b = 0, hg = 0, t_first = 0, tiles_left = 0, split = 0;
-  int before_b = 0;     // balanced mode: tiles in the sequences before b
-  int64_t total = 0;    // balanced mode: entries of the tile list
-  int shares = 0;       // balanced mode: CTAs that have a share
+    HeadSums hs = {-INFINITY, 0.f, -INFINITY, 0.f};
+    if (active && ok) ok = run_tiles(ta, sm, item, hs);
+
+    // ---- the item's end.  What the next item needs is requested before the last value sums are waited for.
+    bool more;
+    int n_parts = 1;
+    {
+      Walk w = get_item(st);
+      const uint32_t mine = st[kItMine] + (active ? w.ntiles : 0);
+      const uint32_t T = st[kItT] + w.ntiles, units = st[kItUnits] + w.ntiles * npairs;
+      if (fused && active) {  // the CTAs that share this (sequence, head group)
+        const int64_t first = (int64_t)w.before_b * n_hg + (int64_t)w.hg * w.tiles_b;
+        const int c_first = share_owner(first, sh.total, sh.shares);
+        n_parts = share_owner(first + w.tiles_b - 1, sh.total, sh.shares) - c_first + 1;
+        if (lane == 0) st[kItParts] = n_parts, st[kItFirst] = c_first;
+      }
+      more = w.next(p, n_hg);
+      if (more) {
+        if (g < p.n_q_heads - w.hg * C::kG) request_pq(ta, sbase, w, g, wk_vec);
+        put_item(state(item + 1), w, T, units, mine);
+      }
+    }
+    if (active) {
+      const uint32_t last = st[kItMine] + st[kItTiles] - 1;  // count of the head's last tile
+      const int b = st[kItB], hg = st[kItHg], h = h0 + g;
+      if (ok) {
+        ok = warp_wait(bar(C::kBarDFull + g), last & 1);
+        if (ok) {
+          tc_fence_after();
+          fold_values(hs, tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 32 * g, reinterpret_cast<const float*>(sm + C::kOffRef) + g * 8, last);
+          tc_fence_before();
+        }
+      }
+      if (!ok) atomicMax(&g_status, (unsigned)kTimeoutEpilogue);
+
+      // ---- the head's denominator: the four warps' (max z, sum) pairs under a common maximum
+      const float l_w = warp_sum(hs.l_lane);
+      float2* sums = reinterpret_cast<float2*>(sm + C::kOffSum) + g * 4;
+      if (lane == 0) sums[q4] = make_float2(hs.m_run, l_w);
+      head_sync();
+      float m_all = -INFINITY;
+#pragma unroll
+      for (int w4 = 0; w4 < 4; ++w4) m_all = fmaxf(m_all, sums[w4].x);
+      float l_tot = 0.f;
+#pragma unroll
+      for (int w4 = 0; w4 < 4; ++w4)
+        if (sums[w4].x > -INFINITY) l_tot = fmaf(sums[w4].y, fast_exp2(sums[w4].x - m_all), l_tot);
+      const int64_t slot = balanced ? ((int64_t)b * n_hg + hg + blockIdx.x) * C::kG + g
+                                    : ((int64_t)b * p.n_q_heads + h) * a.n_splits + blockIdx.x % a.n_splits;
+      const int r = 16 * q4 + lane;
+      // sum_s 2^z sv Lv / sum_s 2^z  =  acc * 2^(big_m - m_all) / l
+      // (after a wait that timed out the item's result is poisoned: NaN here propagates through the
+      // merge into the output row, so a time-out cannot pass for a valid result)
+      const float o = !ok ? __int_as_float(0x7fc00000) : hs.big_m > -INFINITY ? hs.acc * fast_exp2(hs.big_m - m_all) / l_tot : 0.f;
+      if (!fused || n_parts > 1) {
+        if (lane < 16 && r < Rv) a.mid_o[slot * Rv + r] = o;
+        // natural-log lse, as the merge kernel expects (stage1.py:216)
+        if (q4 == 0 && lane == 0) a.lse[slot] = m_all * 0.6931471805599453f + logf(l_tot);
+      } else if (lane < 16 && r < Rv) {
+        // this CTA covered the whole (sequence, head): no partials.  The latent-space row goes to shared
+        // memory (the head's plane area: its value MMAs are complete).
+        reinterpret_cast<float*>(sm + C::kOffPlanes + 2 * g * C::kPlaneBytes)[r] = o;
+      }
+      if (fused) {
+        if (n_parts > 1) __threadfence();
+        head_sync();  // the partial is out, the (max, sum) pairs have been read
+        // the counter's answer is needed only after the next item's [P;Q] build
+        if (n_parts > 1 && row == 0) seen = atomicAdd(ta.arrivals + (int64_t)b * p.n_q_heads + h, 1u);
+        pending = true;
+      }
+    }
+    if (!more) {
+      if (pending) finish_head(ta, sm, g, st, seen);
+      break;
+    }
+  }
+}
+
+// ------------------------------------------------------------------ the kernel
+__global__ void __launch_bounds__(Cfg::kThreads, 1) stage1_tc_kernel(const __grid_constant__ TcArgs ta) {
+  using C = Cfg;
+  const KArgs& a = ta.k;
+  const WsvdLatentDecodeParams& p = a.p;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t sbase = smem_u32(smem_raw);
+  uint8_t* sm = smem_raw;
+  if ((sbase & 1023u) != 0) {  // the swizzled operand tiles need a 1024-byte aligned base
+    if (threadIdx.x == 0) atomicMax(&g_status, (unsigned)kBadSmemAlignment);
+    return;
+  }
+  const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG;
+  const bool balanced = ta.balanced != 0, fused = balanced && ta.arrivals != nullptr;
+  auto tiles_of = [&](int i) {
+    const int n = i < p.batch ? p.b_seq_len[i] : 0;
+    return n > 0 ? (n + kTile - 1) / kTile : 0;
+  };
+  int mine = 0;  // balanced mode: tiles of the sequences this thread counts (requested before the set-up below)
+  if (balanced)
+    for (int i = threadIdx.x; i < p.batch; i += C::kThreads) mine += tiles_of(i);
+
+  // ---- once per CTA: tensor memory, barriers, descriptor prefetch
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + C::kOffTmemSlot);
+  if (warp == C::kMmaWarp) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
+    tmem_relinquish();
+    tc_fence_before();
+  } else if (warp == C::kLoadWarp) {
+    for (int i = lane; i < C::kNumBars; i += 32) {
+      uint32_t count = 1;                                                       // one copy, or one commit
+      if (i >= C::kBarVEmpty && i < C::kBarKEmpty) count = C::kG;               // a commit per head, after its value MMAs on the slot
+      else if (i >= C::kBarKEmpty && i < C::kBarAFull) count = 4 * C::kG;       // every warp that copies rows out of the slot
+      else if (i >= C::kBarWEmpty && i < C::kBarDFull) count = 8;               // the warps of a pair of heads
+      else if (i >= C::kBarPlanes && i < C::kBarPq) count = 4;                  // the head's four warps
+      else if (i == C::kBarPq) count = 4 * C::kG;
+      mbar_init(sbase + C::kOffBar + 8u * i, count);
+    }
+    fence_barrier_init();
+  } else if (warp == C::kValWarp && lane == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ta.tmap_table)) : "memory");
+    if (ta.use_tma) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ta.tmap_k)) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ta.tmap_v)) : "memory");
+    }
+  }
+
+  Share sh = {};
   if (balanced) {
     // Tiles per sequence -> block-wide sums -> this CTA's share [begin, end) of the tile list and the
     // (sequence, head group, tile) it starts at.  Scratch: the reference/sum area, unused until the
     // first tile.
-    int* plan_sm = reinterpret_cast<int*>(sm + kOffRef);  // [0, 20): per-warp sums; [24], [25]: start sequence, tiles before it
-    constexpr int kWarps = kThreads / 32;
-    auto tiles_of = [&](int i) {
-      const int n = i < p.batch ? p.b_seq_len[i] : 0;
-      return n > 0 ? (n + kTile - 1) / kTile : 0;
-    };
-    int mine = 0;
-    for (int i = threadIdx.x; i < p.batch; i += kThreads) mine += tiles_of(i);
+    int* plan_sm = reinterpret_cast<int*>(sm + C::kOffRef);  // [0, 20): per-warp sums; [24], [25]: start sequence, tiles before it
+    constexpr int kWarps = C::kThreads / 32;
+    static_assert(C::kOffMode - C::kOffRef >= 26 * 4 && kWarps <= 24, "plan scratch");
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
     if (lane == 0) plan_sm[warp] = mine;
@@ -399,14 +1357,14 @@ __device__ __forceinline__ void run_share(const TcArgs& ta, uint8_t* sm) {
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) all_tiles += plan_sm[w];
     __syncthreads();
-    total = (int64_t)all_tiles * n_hg;
-    shares = (int)min((int64_t)gridDim.x, total);
-    const bool has_share = (int)blockIdx.x < shares;
-    const int64_t begin = has_share ? share_begin(blockIdx.x, total, shares) : 0;
-    if (has_share) tiles_left = (int)(share_begin(blockIdx.x + 1, total, shares) - begin);
+    sh.total = (int64_t)all_tiles * n_hg;
+    sh.shares = (int)min((int64_t)gridDim.x, sh.total);
+    const bool has_share = (int)blockIdx.x < sh.shares;
+    const int64_t begin = has_share ? share_begin(blockIdx.x, sh.total, sh.shares) : 0;
+    if (has_share) sh.tiles_left = (int)(share_begin(blockIdx.x + 1, sh.total, sh.shares) - begin);
     if (has_share || (blockIdx.x == 0 && ta.prefix_out != nullptr)) {
       int carry = 0;
-      for (int base = 0; base < p.batch; base += kThreads) {
+      for (int base = 0; base < p.batch; base += C::kThreads) {
         const int i = base + threadIdx.x;
         const int v = tiles_of(i);
         int incl = v;
@@ -435,25 +1393,23 @@ __device__ __forceinline__ void run_share(const TcArgs& ta, uint8_t* sm) {
       }
       if (blockIdx.x == 0 && ta.prefix_out != nullptr && threadIdx.x == 0) {
         ta.prefix_out[p.batch] = all_tiles;
-        ta.prefix_out[p.batch + 1] = shares;
+        ta.prefix_out[p.batch + 1] = sh.shares;
       }
       if (has_share) {
-        b = plan_sm[24];
-        before_b = plan_sm[25];
-        const int tiles_b = tiles_of(b);
-        const int64_t rem = begin - (int64_t)before_b * n_hg;
-        hg = (int)(rem / tiles_b);
-        t_first = (int)(rem % tiles_b);
+        sh.b = plan_sm[24];
+        sh.before_b = plan_sm[25];
+        const int tiles_b = tiles_of(sh.b), rem = (int)(begin - (int64_t)sh.before_b * n_hg);
+        sh.hg = rem / tiles_b;
+        sh.t_first = rem % tiles_b;
       }
-      __syncthreads();  // the scratch area is handed back
     }
     // sequences without tokens belong to no share: their output rows are zeros
     if (fused) {
-      const int n_out = p.wv != nullptr ? p.head_dim : Rv;
+      const int n_out = p.wv != nullptr ? p.head_dim : p.rank_v;
       for (int bb = blockIdx.x; bb < p.batch; bb += gridDim.x) {
         if (p.b_seq_len[bb] > 0) continue;
         if (ta.has_peers) {
-          for (int i = threadIdx.x; i < p.n_q_heads * n_out * ta.peers.n_peers; i += kThreads) {
+          for (int i = threadIdx.x; i < p.n_q_heads * n_out * ta.peers.n_peers; i += C::kThreads) {
             const int peer = i / (p.n_q_heads * n_out), j = i % (p.n_q_heads * n_out);
             ta.peers.out[peer][(int64_t)bb * ta.peers.out_stride_b +
                                (int64_t)(j / n_out + ta.peers.head_offset) * ta.peers.out_stride_h + j % n_out] =
@@ -461,815 +1417,40 @@ __device__ __forceinline__ void run_share(const TcArgs& ta, uint8_t* sm) {
           }
         } else {
           __half* orow = reinterpret_cast<__half*>(p.out) + (int64_t)bb * p.out_stride_b;
-          for (int i = threadIdx.x; i < p.n_q_heads * n_out; i += kThreads)
+          for (int i = threadIdx.x; i < p.n_q_heads * n_out; i += C::kThreads)
             orow[(int64_t)(i / n_out) * p.out_stride_h + i % n_out] = __float2half_rn(0.f);
         }
       }
     }
-  } else {
-    split = blockIdx.x % a.n_splits, hg = (blockIdx.x / a.n_splits) % n_hg, b = blockIdx.x / (a.n_splits * n_hg);
-    tiles_left = 1;
   }
-  // The barriers of an item are re-made for the next one.  Two sets are used in turn, so that a set
-  // is invalidated and re-initialised a whole item after its last use.
-  for (int round = 0; tiles_left > 0 && b < p.batch; ++round) {
-  const int req = p.b_req_idx[b];  // requested together with the length: one round trip, not two
-  const int n = p.b_seq_len[b];
-  int lo, hi;
-  int tiles_b = 0, n_parts = 1, c_first = 0;  // balanced mode: the CTAs that share this (sequence, head group)
-  if (balanced) {
-    tiles_b = (n + kTile - 1) / kTile;
-    const int seg = min(tiles_left, tiles_b - t_first);
-    lo = t_first * kTile;
-    hi = min(n, (t_first + seg) * kTile);
-    tiles_left -= seg;
-    const int64_t first = (int64_t)before_b * n_hg + (int64_t)hg * tiles_b;
-    c_first = share_owner(first, total, shares);
-    n_parts = share_owner(first + tiles_b - 1, total, shares) - c_first + 1;
-  } else {
-    lo = split * a.split_len;
-    hi = min(n, lo + a.split_len);
-    tiles_left = 0;
-  }
-  if (hi <= lo) break;  // an empty split writes nothing (a balanced share never holds an empty item)
-  bars = sbase + kOffBar + (round & 1) * (kNumBars * 8);
-  const int h0 = hg * kG;
-  const int G = min(kG, p.n_q_heads - h0);
-  const int npairs = (G + 1) >> 1;
-  const int ntiles = (hi - lo + kTile - 1) / kTile;
-  const int pos0 = (p.pos_offset != nullptr ? p.pos_offset[b] : 0) + lo;  // RoPE position of token lo
-
-  const int32_t* page = p.req_to_token + (int64_t)req * p.rtt_stride;
-
-  uint4 wpre[8], qpre[2];
-  // requested during set-up so that their latency is hidden behind it
-  int slot_n = -1;
-  unsigned short sk_raw = 0, sv_raw = 0;
-  int slot0 = -1;  // epilogue: token slot of this lane's first token
-  int ent[4];      // requesting warp: page entries of the tile it requests next (see check_run)
-
-  // ---- set-up of the item: barriers (MMA warp), first loads (the others).  Nothing here waits for
-  //      a load: what was requested is used after the barrier, so that the barrier is reached after
-  //      one round trip (the sequence length) and not after the three of the page-table look-ups.
-  if constexpr (!kEpi) {
-  if (warp == kMmaWarp) {
-    for (int i = lane; i < kNumBars; i += 32) {
-      if (round >= 2) mbar_inval(bar(i));
-      uint32_t count = 1;                                    // one TMA or commit arrival
-      if (i < kBarVEmpty) count = 32;                        // V/K full: one arrive per lane of the copying warp
-      else if (i < kBarKEmpty) count = G;                    // V empty: one commit per head, after the head's value MMAs on the slot
-      else if (i < kBarAFull) count = 4 * G;                 // K empty: every warp that copies rows out of the slot
-      else if (i >= kBarWEmpty && i < kBarDFull) count = 8;  // W empty: 8 warp arrivals (see w_empty_arrivals)
-      else if (i >= kBarPlanes && i < kBarPq) count = 4;     // planes ready: the head's four warps
-      else if (i == kBarPq) count = 4 * G;
-      mbar_init(bar(i), count);
-    }
-    fence_barrier_init();
-  } else if (warp == kMmaWarp + 1) {
-    // page entries of tile 0, for the run check that precedes the first copies
-    const int s0 = lo + 4 * lane;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) ent[j] = s0 + j < hi ? page[s0 + j] : -1;
-  }
-  } else {
-  if (warp < 4 * G) {
-    const int hk_pre = (h0 + (warp >> 2)) / gqa;
-    // the head's slice of wk for the [P;Q] build: requested now, used after the barrier
-    if (wk_vec) {
-      const bool il = p.rope_layout == WSVD_ROPE_INTERLEAVED;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int task = (threadIdx.x & 127) + 128 * i, r = task >> 3, ic = task & 7;
-        wpre[2 * i] = make_uint4(0u, 0u, 0u, 0u);
-        wpre[2 * i + 1] = make_uint4(0u, 0u, 0u, 0u);
-        if (r < Rk && wk_i8) {
-          const int8_t* w = reinterpret_cast<const int8_t*>(p.wk) + (int64_t)r * p.wk_stride_r + (int64_t)hk_pre * 128;
-          const uint2 a0 = *reinterpret_cast<const uint2*>(w + (il ? ic * 16 : ic * 8));
-          const uint2 a1 = *reinterpret_cast<const uint2*>(w + (il ? ic * 16 + 8 : 64 + ic * 8));
-          wpre[2 * i].x = a0.x;
-          wpre[2 * i].y = a0.y;
-          wpre[2 * i + 1].x = a1.x;
-          wpre[2 * i + 1].y = a1.y;
-        } else if (r < Rk) {
-          const __half* w = reinterpret_cast<const __half*>(p.wk) + (int64_t)r * p.wk_stride_r + (int64_t)hk_pre * 128;
-          wpre[2 * i] = *reinterpret_cast<const uint4*>(w + (il ? ic * 16 : ic * 8));
-          wpre[2 * i + 1] = *reinterpret_cast<const uint4*>(w + (il ? ic * 16 + 8 : 64 + ic * 8));
-        }
-      }
-    }
-    // the 16 query values this thread's chunk of 8 frequencies needs (two 16-byte loads)
-    {
-      const bool il = p.rope_layout == WSVD_ROPE_INTERLEAVED;
-      const int ic = threadIdx.x & 7;
-      const __half* qp = reinterpret_cast<const __half*>(p.q) + (int64_t)b * p.q_stride_b +
-                         (int64_t)(h0 + (warp >> 2)) * p.q_stride_h;
-      qpre[0] = *reinterpret_cast<const uint4*>(qp + (il ? ic * 16 : ic * 8));
-      qpre[1] = *reinterpret_cast<const uint4*>(qp + (il ? ic * 16 + 8 : 64 + ic * 8));
-    }
-    {
-      // this lane's first token and its next one: page entries (the first token's scales are
-      // requested once its entry is here, after the [P;Q] build)
-      const int s_first = lo + (warp & 3) * 32 + lane;
-      if (s_first < hi) slot0 = page[s_first];
-      if (s_first + kTile < hi) slot_n = page[s_first + kTile];
-    }
-  }
-  }
-  __syncthreads();
+  __syncthreads();  // barriers, tensor memory; the scratch area is handed back
   tc_fence_after();
-  tmem = *tmem_slot;
-
-  if constexpr (!kEpi) {
-  if (warp == kMmaWarp) {
-    // ================================================================= score MMAs
-    if (lane == 0) {
-      // descriptors: only the start-address field changes between k-steps, buffers and pairs
-      const uint64_t adesc0 = smem_desc_sw128(sA), bdesc0 = smem_desc_sw128(sB);
-      bool ok = mbar_wait(bar(kBarPq), 0);
-      int u = 0;  // running count of (tile, pair) units: unit u uses W buffer u % kWBufs
-      for (int t = 0; t < ntiles && ok; ++t) {
-        const int buf = t & 1;
-        ok = mbar_wait(bar(kBarAFull + buf), (t >> 1) & 1);
-        for (int pr = 0; pr < npairs && ok; ++pr, ++u) {
-          const int wb = u % kWBufs;
-          if (u >= kWBufs) ok = mbar_wait(bar(kBarWEmpty + wb), ((u / kWBufs) - 1) & 1);
-          if (!ok) break;
-          tc_fence_after();
-          const int heads = min(2, G - 2 * pr);
-          const uint32_t idesc = instr_desc_f16(kTile, kRkMax * heads);
-          const uint32_t d_tmem = tmem + wb * 128;
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            const uint32_t koff = (kk & 3) * 32;
-            const uint64_t ad = adesc0 + ((buf * kABufBytes + (kk >> 2) * kAHalfBytes + koff) >> 4);
-            const uint64_t bd = bdesc0 + (((kk >> 2) * kBHalfBytes + pr * (2 * kRkMax * 128) + koff) >> 4);
-            umma_f16(d_tmem, ad, bd, idesc, kk > 0);
-          }
-          umma_commit(bar(kBarWFull + wb));
-        }
-        if (ok) umma_commit(bar(kBarAEmpty + buf));
-      }
-      // nothing may still be on its way to a barrier when the next item re-makes them: the releases
-      // of the last two table buffers are the only arrivals nobody else waits for
-      for (int t = max(0, ntiles - 2); t < ntiles && ok; ++t) ok = mbar_wait(bar(kBarAEmpty + (t & 1)), (t >> 1) & 1);
-      if (!ok) atomicMax(&g_status, (unsigned)kTimeoutMma);
-    }
-    __syncwarp();
-  } else {
-    // ================================================================= copies, value MMAs
-    // Latent rows travel in units of one tile (128 tokens) of all the group's KV heads; tile n uses
-    // ring slot n % kKSlots (K) or n % kVSlots (V); KV head hk0 + j sits at j * kHeadBytes inside
-    // the slot.  Warp 17 requests the table tiles and the K and V tiles: a K slot is free again once
-    // every warp has copied its rows to registers, at the top of the tile; a V slot once every
-    // head's value MMAs on it are complete.  Warps 18 and 19 each serve one pair of heads (lane 0
-    // and lane 1 one head each): they wait for the digit planes of the head's four warps and issue
-    // the head's value MMAs (one per warp of 32 tokens, each into its own 8 columns of tensor
-    // memory); two commits then tell the epilogue warps (D full) and the requesting warp (V empty)
-    // when the MMAs have completed.
-    const int pw = warp - kMmaWarp - 1;
-    const bool is_loader = pw == 0;
-    const int hk0 = h0 / gqa, nkv = (h0 + G - 1) / gqa - hk0 + 1;  // the group's KV heads
-    bool ok = true;
-    // A tensor copy needs the tile's token slots to be one run of consecutive slots (true for a cache
-    // laid out sequence by sequence, and for every tile inside a page of a paged cache).  The
-    // requesting warp checks that tile by tile: lane l holds the page entries of tokens 4l..4l+3 of
-    // the tile it will request next (fetched one tile ahead), and the warp votes.  `run_first`: the
-    // slot of the tile's first token.
-    int run_tile = -1, run_first = 0;
-    bool run_ok = false;
-    auto fetch_entries = [&](int nu) {
-      const int s0 = lo + nu * kTile + 4 * lane;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) ent[j] = (nu < ntiles && s0 + j < hi) ? page[s0 + j] : -1;
-    };
-    auto check_run = [&](int nu) {  // tiles are asked for in order, each at most twice in a row
-      if (nu == run_tile) return;
-      run_first = __shfl_sync(0xffffffffu, ent[0], 0);
-      bool good = true;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) good = good && (ent[j] < 0 || ent[j] == run_first + 4 * lane + j);
-      run_ok = __all_sync(0xffffffffu, good) && ta.use_tma != 0;
-      run_tile = nu;
-      fetch_entries(nu + 1);
-    };
-    // Request tile `nu` of K (is_k) or V once its ring slot is free.
-    auto load_unit = [&](int nu, bool is_k) {
-      check_run(nu);
-      const int nslots = is_k ? kKSlots : kVSlots;
-      const int bar_full = is_k ? kBarKFull : kBarVFull, bar_empty = is_k ? kBarKEmpty : kBarVEmpty;
-      const int slot = nu % nslots, use = nu / nslots;
-      if (use > 0) ok = warp_wait(bar(bar_empty + slot), (use - 1) & 1);
-      if (!ok) return;
-      const uint32_t dst = (is_k ? sK : sV) + slot * kUnitBytes, full = bar(bar_full + slot);
-      if (run_ok) {
-        // one copy for all heads, or one per KV head (lane j: head hk0 + j)
-        const int copies = ta.box_heads > 1 ? 1 : nkv;
-        if (lane < copies) {
-          const int hk = hk0 + lane, first = run_first;
-          const int c1 = ta.slot_axis == 1 ? first : hk, c2 = ta.slot_axis == 1 ? hk : first;
-          mbar_expect_tx(full, ta.box_heads * kHeadBytes);
-          tma_load_3d(dst + lane * kHeadBytes, is_k ? &ta.tmap_k : &ta.tmap_v, 0, c1, c2, full);
-        }
-        if (lane == 0) mbar_arrive_n(full, 32 - copies);  // the arrivals the gather path makes lane by lane
-      } else {
-        // Gather through the page table, head after head: lane (r0 = lane/4, c = lane%4) copies
-        // 16-byte chunk c of rows r0 + 8k to where the tensor copy would have placed it.  Rows past
-        // the end and chunks past the rank are zero-filled.
-        const int R = is_k ? Rk : Rv;
-        const int64_t stride_t = is_k ? p.k_stride_t : p.v_stride_t, stride_h = is_k ? p.k_stride_h : p.v_stride_h;
-        const uint8_t* latent = reinterpret_cast<const uint8_t*>(is_k ? p.latent_k : p.latent_v);
-        const int c = lane & 3, r0 = lane >> 2;
-        const bool c_on = c * 16 < R;
-#pragma unroll 1
-        for (int half = 0; half < 2; ++half) {
-          const int s0 = lo + nu * kTile + half * 64 + r0;
-          int64_t sl[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) sl[k] = (c_on && s0 + 8 * k < hi) ? page[s0 + 8 * k] : -1;
-          for (int j = 0; j < nkv; ++j) {
-            const uint8_t* base = latent + (int64_t)(hk0 + j) * stride_h;
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-              cp_async16(dst + j * kHeadBytes + latent_off(half * 64 + r0 + 8 * k, c),
-                         base + (sl[k] >= 0 ? c * 16 + sl[k] * stride_t : 0), sl[k] >= 0 ? 16u : 0u);
-          }
-        }
-        cp_async_arrive_noinc(full);
-      }
-    };
-    if (is_loader) {
-      auto issue_table = [&](int t) {
-        if (lane == 0) {
-          const int buf = t & 1;
-          mbar_expect_tx(bar(kBarAFull + buf), kABufBytes);
-          tma_load_3d(sA + buf * kABufBytes, &ta.tmap_table, 0, pos0 + t * kTile, 0, bar(kBarAFull + buf));
-        }
-      };
-      // start: K of tile 0, table tiles 0 and 1, V of tiles 0 and 1 (tile 0's page entries were
-      // requested before the barrier)
-      load_unit(0, true);
-      issue_table(0);
-      load_unit(0, false);
-      if (ntiles > 1) {
-        load_unit(1, false);
-        issue_table(1);
-      }
-      for (int t = 0; t < ntiles && ok; ++t) {
-        // In the order in which their slots come free during tile t: the table tile of t+2 (the
-        // score MMAs of tile t have read its buffer), K of tile t+1 (tile t's rows were copied to
-        // registers at the top of the tile), V of tile t+1 (tile t-1's value MMAs completed shortly
-        // after the end of tile t-1).
-        if (t + 2 < ntiles) {
-          ok = warp_wait(bar(kBarAEmpty + (t & 1)), (t >> 1) & 1);
-          if (!ok) break;
-          issue_table(t + 2);
-        }
-        if (t + 1 < ntiles) load_unit(t + 1, true);
-        if (t >= 1 && t + 1 < ntiles && ok) load_unit(t + 1, false);
-      }
-    } else if (2 * (pw - 1) < G) {
-      // Value MMAs of one pair of heads: lane 0 and lane 1 one head each.
-      const int g = 2 * (pw - 1) + lane;
-      const bool agent = lane < 2 && g < G;
-      const int sub = agent ? (h0 + g) / gqa - hk0 : 0;
-      const uint32_t idesc = instr_desc_i8(64, 8);
-      const uint64_t vdesc0 = smem_desc_mn_sw64(sV + sub * kHeadBytes);
-      const uint64_t pdesc0 = smem_desc_k_plain(sPl + 2 * g * kPlaneBytes);
-      const uint32_t d_tmem = tmem + kTmemD + 32 * g;
-      for (int t = 0; t < ntiles && ok; ++t) {
-        if (agent) {
-          const int vslot = t % kVSlots;
-          // the V rows arrive long before the planes are ready: wait for them first, off the
-          // critical path from "planes ready" to "D full"
-          ok = mbar_wait(bar(kBarVFull + vslot), (t / kVSlots) & 1);
-          if (ok) ok = mbar_wait(bar(kBarPlanes + g), t & 1);
-          if (ok) {
-            tc_fence_after();
-#pragma unroll
-            for (int w4 = 0; w4 < 4; ++w4) {
-              const uint32_t voff = vslot * kUnitBytes + w4 * 2048;  // the 32 tokens of warp w4: 32 rows of 64 bytes
-              umma_i8(d_tmem + 8 * w4, vdesc0 + (voff >> 4), pdesc0 + (((w4 >> 1) * kPlaneBytes) >> 4), idesc, 0);
-            }
-            // completion of the MMAs tells the epilogue warps (D full) and hands the V slot back
-            umma_commit(bar(kBarDFull + g));
-            umma_commit(bar(kBarVEmpty + vslot));
-          }
-        }
-        ok = __all_sync(0xffffffffu, ok);
-      }
-    }
-    if (!ok) atomicMax(&g_status, (unsigned)kTimeoutProducer);
-  }
-  } else {
-  if (warp < 4 * G) {
-    // ================================================================= epilogue
-    const int g = warp >> 2, q4 = warp & 3;
-    const int h = h0 + g, hk = h / gqa;
-    const int pr = g >> 1;
-    const int row = q4 * 32 + lane;
-    const bool interleaved = p.rope_layout == WSVD_ROPE_INTERLEAVED;
-
-    // ---- B operand: P (cos coefficients) and Q (sin coefficients) of this head, f16,
-    //      rows n = g*64 + r, 64 frequencies per row, 128-byte swizzle; rows r >= rank_k are zero
-    {
-      const int tid = threadIdx.x & 127;
-      // q * sm_scale * log2(e) (scores come out in the log2 domain): qlo[e] pairs with dimension
-      // d0 and qhi[e] with its rotation partner d1 of frequency ic*8 + e
-      float qlo[8], qhi[8];
-      {
-        const float qscale = a.sm_scale * 1.4426950408889634f;
-        const __half* q0 = reinterpret_cast<const __half*>(&qpre[0]);
-        const __half* q1 = reinterpret_cast<const __half*>(&qpre[1]);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          if (interleaved) {
-            const __half* src = e < 4 ? q0 : q1;
-            qlo[e] = __half2float(src[(2 * e) & 7]) * qscale;
-            qhi[e] = __half2float(src[(2 * e + 1) & 7]) * qscale;
-          } else {
-            qlo[e] = __half2float(q0[e]) * qscale;
-            qhi[e] = __half2float(q1[e]) * qscale;
-          }
-        }
-      }
-      const int64_t col = (int64_t)hk * 128;
-      if (wk_vec && !wk_i8 && !interleaved) {
-        // Common case (f16 wk, half-split pairing): packed f16 arithmetic.  The operands are
-        // rounded to f16 for the MMA anyway; forming them with one extra f16 rounding of a
-        // product keeps the error of the scores within a few 1e-5.  This thread's chunk of 8
-        // frequencies is the same for its four ranks, so q is converted once.
-        const int ic = tid & 7;
-        __half2 qa[4], qb[4], nqa[4];
-        {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            qa[e] = __floats2half2_rn(qlo[2 * e], qlo[2 * e + 1]);
-            qb[e] = __floats2half2_rn(qhi[2 * e], qhi[2 * e + 1]);
-          }
-#pragma unroll
-          for (int e = 0; e < 4; ++e) nqa[e] = __hneg2(qa[e]);
-        }
-#pragma unroll
-        for (int it = 0; it < 4; ++it) {
-          const int r = (tid + 128 * it) >> 3;
-          const __half2* ua = reinterpret_cast<const __half2*>(&wpre[2 * it]);      // U[d = ic*8 .. +7]
-          const __half2* ub = reinterpret_cast<const __half2*>(&wpre[2 * it + 1]);  // U[64 + ic*8 .. +7]
-          __align__(16) __half2 pv[4];
-          __align__(16) __half2 qv[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            pv[e] = __hfma2(qa[e], ua[e], __hmul2(qb[e], ub[e]));   // P = q_i U_i + q_{i+64} U_{i+64}
-            qv[e] = __hfma2(nqa[e], ub[e], __hmul2(qb[e], ua[e]));  // Q = q_{i+64} U_i - q_i U_{i+64}
-          }
-          const int nrow = g * 64 + r;
-          const uint32_t off = nrow * 128 + ((ic ^ (nrow & 7)) << 4);
-          *reinterpret_cast<uint4*>(sm + kOffB + off) = *reinterpret_cast<const uint4*>(pv);
-          *reinterpret_cast<uint4*>(sm + kOffB + kBHalfBytes + off) = *reinterpret_cast<const uint4*>(qv);
-        }
-      } else if (wk_vec && wk_i8) {
-        // int8 wk in vectors of eight: the columns' scales are this thread's for all four ranks and go
-        // into q once, P = (q_d0 s_d0) w_d0 + (q_d1 s_d1) w_d1, Q = (q_d1 s_d0) w_d0 - (q_d0 s_d1) w_d1,
-        // fp32 throughout.  (Byte by byte, with the scales re-read per rank, the build of an item
-        // took as long as ten tiles: 64 dependent look-ups a thread.)
-        const int ic = tid & 7;
-        const __half* ws = reinterpret_cast<const __half*>(p.wk_scale) + col;
-        const uint4 s0v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 : ic * 8));
-        const uint4 s1v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 + 8 : 64 + ic * 8));
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {  // four frequencies at a time: fewer registers
-          float p0[4], p1[4], q0[4], q1[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int e = 4 * half + j;
-            const __half* s0h = reinterpret_cast<const __half*>(&s0v);
-            const __half* s1h = reinterpret_cast<const __half*>(&s1v);
-            const __half* pair = half == 0 ? s0h : s1h;
-            const float s0 = __half2float(interleaved ? pair[(2 * e) & 7] : s0h[e]);
-            const float s1 = __half2float(interleaved ? pair[(2 * e + 1) & 7] : s1h[e]);
-            p0[j] = qlo[e] * s0;
-            p1[j] = qhi[e] * s1;
-            q0[j] = qhi[e] * s0;
-            q1[j] = qlo[e] * s1;
-          }
-#pragma unroll
-          for (int it = 0; it < 4; ++it) {
-            const int r = (tid + 128 * it) >> 3;
-            // bytes of dimension d0 and d1 of the four frequencies (rank >= rank_k: zeros)
-            uint32_t w0, w1;
-            if (interleaved) {
-              const uint4 src = wpre[2 * it + half];
-              w0 = __byte_perm(src.x, src.y, 0x6420);
-              w1 = __byte_perm(src.x, src.y, 0x7531);
-            } else {
-              w0 = half == 0 ? wpre[2 * it].x : wpre[2 * it].y;
-              w1 = half == 0 ? wpre[2 * it + 1].x : wpre[2 * it + 1].y;
-            }
-            __align__(8) __half pv[4];
-            __align__(8) __half qv[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float u0 = (float)(int8_t)(w0 >> (8 * j)), u1 = (float)(int8_t)(w1 >> (8 * j));
-              pv[j] = __float2half_rn(fmaf(p0[j], u0, p1[j] * u1));
-              qv[j] = __float2half_rn(fmaf(q0[j], u0, -(q1[j] * u1)));
-            }
-            const int nrow = g * 64 + r;
-            const uint32_t off = nrow * 128 + ((ic ^ (nrow & 7)) << 4) + 8 * half;
-            *reinterpret_cast<uint2*>(sm + kOffB + off) = *reinterpret_cast<const uint2*>(pv);
-            *reinterpret_cast<uint2*>(sm + kOffB + kBHalfBytes + off) = *reinterpret_cast<const uint2*>(qv);
-          }
-        }
-      } else
-#pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        const int task = tid + 128 * it;
-        const int r = task >> 3, ic = task & 7;  // rank, chunk of 8 frequencies
-        float u0[8], u1[8];
-        if (r >= Rk) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) u0[e] = u1[e] = 0.f;
-        } else if (wk_vec) {
-          // half layout: dims ic*8.. and 64+ic*8..; interleaved: 16 consecutive dims
-          const uint4 a0 = wpre[2 * it], a1 = wpre[2 * it + 1];
-          const __half* h0p = reinterpret_cast<const __half*>(&a0);
-          const __half* h1p = reinterpret_cast<const __half*>(&a1);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            if (interleaved) {
-              const __half* src = e < 4 ? h0p : h1p;
-              u0[e] = __half2float(src[(2 * e) & 7]);
-              u1[e] = __half2float(src[(2 * e + 1) & 7]);
-            } else {
-              u0[e] = __half2float(h0p[e]);
-              u1[e] = __half2float(h1p[e]);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const int i = ic * 8 + e;
-            const int d0 = interleaved ? 2 * i : i, d1 = interleaved ? 2 * i + 1 : i + 64;
-            if (p.wk_dtype == WSVD_I8) {
-              const int8_t* w = reinterpret_cast<const int8_t*>(p.wk) + (int64_t)r * p.wk_stride_r + col;
-              const __half* ws = reinterpret_cast<const __half*>(p.wk_scale) + col;
-              u0[e] = (float)w[d0] * __half2float(ws[d0]);
-              u1[e] = (float)w[d1] * __half2float(ws[d1]);
-            } else {
-              const __half* w = reinterpret_cast<const __half*>(p.wk) + (int64_t)r * p.wk_stride_r + col;
-              u0[e] = __half2float(w[d0]);
-              u1[e] = __half2float(w[d1]);
-            }
-          }
-        }
-        __align__(16) __half pv[8];
-        __align__(16) __half qv[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          pv[e] = __float2half_rn(qlo[e] * u0[e] + qhi[e] * u1[e]);
-          qv[e] = __float2half_rn(qhi[e] * u0[e] - qlo[e] * u1[e]);
-        }
-        const int nrow = g * 64 + r;
-        const uint32_t off = nrow * 128 + ((ic ^ (nrow & 7)) << 4);
-        *reinterpret_cast<uint4*>(sm + kOffB + off) = *reinterpret_cast<const uint4*>(pv);
-        *reinterpret_cast<uint4*>(sm + kOffB + kBHalfBytes + off) = *reinterpret_cast<const uint4*>(qv);
-      }
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(kBarPq));
-    }
-    if (slot0 >= 0) {
-      sk_raw = reinterpret_cast<const unsigned short*>(p.k_scale)[(int64_t)hk * p.ks_stride_h + (int64_t)slot0 * p.ks_stride_t];
-      sv_raw = reinterpret_cast<const unsigned short*>(p.v_scale)[(int64_t)hk * p.vs_stride_h + (int64_t)slot0 * p.vs_stride_t];
-    }
-
-    const __half* ksc = reinterpret_cast<const __half*>(p.k_scale) + (int64_t)hk * p.ks_stride_h;
-    const __half* vsc = reinterpret_cast<const __half*>(p.v_scale) + (int64_t)hk * p.vs_stride_h;
-    float* refs = reinterpret_cast<float*>(sm + kOffRef) + g * 8;  // [tile parity][warp]: max y the warp's planes refer to
-    // Digit planes: the two warps of half a tile share one 8-row block (the MMA's B operand has 8
-    // rows): rows 0..2 hold the even warp's digits, rows 3..5 the odd warp's.  Each warp's MMA reads
-    // the whole block, so its columns 3..5 (or 0..2) are the other warp's weights times this warp's
-    // V rows: garbage that nobody reads.  Rows 6 and 7 are never written.
-    const uint32_t my_planes = sPl + (2 * g + (q4 >> 1)) * kPlaneBytes + (lane >> 4) * 128 + (q4 & 1) * 48 + (lane & 15);
-    const int sub = hk - h0 / gqa;  // this head's KV head inside a unit
-    // A W buffer serves the two pairs in turn and its "empty" barrier always counts 8 warp
-    // arrivals: the four warps of a pair that holds a single head arrive twice each.
-    const uint32_t w_empty_arrivals = (G - 2 * pr) >= 2 ? 1u : 2u;
-
-    // Running state.  Softmax denominator: l_lane under this warp's own running max m_run of z.
-    // Value sum: lanes 0..15 hold rank 16*q4 + lane of the whole head (all four warps' tokens): acc
-    // under the running reference big_m (max y of every (tile, warp) folded in so far).
-    float m_run = -INFINITY, l_lane = 0.f, big_m = -INFINITY, acc = 0.f;
-    bool ok = true;
-    const uint32_t d_addr = tmem + ((uint32_t)(q4 * 32) << 16) + kTmemD + 32 * g;
-    // Fold in the value sums of tile tp: D[rank][8*w + 0..2] are the three digit-plane sums over the
-    // 32 tokens of warp w, whose weights were taken relative to refs[tp & 1][w].
-    auto fold_values = [&](int tp) {
-      uint32_t d[4][4];
-#pragma unroll
-      for (int w4 = 0; w4 < 4; ++w4) tmem_ld4(d_addr + 8 * w4 + 3 * (w4 & 1), d[w4]);
-      const float4 rf = *reinterpret_cast<const float4*>(refs + (tp & 1) * 4);
-      const float ref[4] = {rf.x, rf.y, rf.z, rf.w};
-      tmem_wait_ld();
-      float m_new = big_m;
-#pragma unroll
-      for (int w4 = 0; w4 < 4; ++w4) m_new = fmaxf(m_new, ref[w4]);
-      if (m_new > -INFINITY) {
-        acc *= fast_exp2(big_m - m_new);  // big_m = -inf -> factor 0
-#pragma unroll
-        for (int w4 = 0; w4 < 4; ++w4) {
-          if (ref[w4] > -INFINITY) {  // (a warp without tokens in this tile has no MMA and reference -inf)
-            // the two low digit sums are combined as integers (|d| <= 32 * 255 * 128 < 2^21)
-            const float v = fmaf((float)(int32_t)d[w4][2], 65536.f,
-                                 (float)((int32_t)d[w4][1] * 256 + (int32_t)d[w4][0]));
-            acc = fmaf(v, fast_exp2(ref[w4] - m_new) * (1.f / kPlaneScale), acc);
-          }
-        }
-        big_m = m_new;
-      }
-    };
-
-    unsigned short sk_n = 0, sv_n = 0;
-    for (int t = 0; t < ntiles; ++t) {
-      const int s = lo + t * kTile + row;
-      const bool valid = s < hi;
-      const int u = t * npairs + pr, wb = u % kWBufs;
-      // ---- the next tile's scales and the page entry of the tile after it: requested a whole
-      //      tile before they are used
-      sk_n = 0;
-      sv_n = 0;
-      if (slot_n >= 0) {
-        sk_n = reinterpret_cast<const unsigned short*>(ksc)[(int64_t)slot_n * p.ks_stride_t];
-        sv_n = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_n * p.vs_stride_t];
-      }
-      slot_n = -1;
-      if (s + 2 * kTile < hi) slot_n = page[s + 2 * kTile];
-      // ---- this warp's 32 K rows (lane = token) go from the ring slot to registers at once and
-      //      the slot is handed back: its refill has the whole tile to arrive
-      uint4 kreg[4];
-      {
-        const int kslot = t % kKSlots;
-        ok = mbar_wait(bar(kBarKFull + kslot), (t / kKSlots) & 1);
-        if (!ok) break;
-        const uint32_t krows = sK + kslot * kUnitBytes + sub * kHeadBytes;
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                       : "=r"(kreg[c].x), "=r"(kreg[c].y), "=r"(kreg[c].z), "=r"(kreg[c].w)
-                       : "r"(krows + latent_off(row, c)));
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(kBarKEmpty + kslot));
-      }
-      ok = mbar_wait(bar(kBarWFull + wb), (u / kWBufs) & 1);
-      if (!ok) break;
-      tc_fence_after();
-
-      // ---- score: dot of this token's int8 K row with its row of W, 16 ranks at a time
-      const uint32_t taddr = tmem + ((uint32_t)(q4 * 32) << 16) + wb * 128 + (g & 1) * kRkMax;
-      float2 dot0 = make_float2(0.f, 0.f), dot1 = make_float2(0.f, 0.f);
-      // two 16-column loads in flight alternately: the next chunk of W travels while this one is used
-      uint32_t wa[16], wb16[16];
-      auto mac16 = [&](const uint32_t (&w)[16], const uint4 kq) {
-        const uint32_t kws[4] = {kq.x ^ 0x80808080u, kq.y ^ 0x80808080u, kq.z ^ 0x80808080u, kq.w ^ 0x80808080u};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float2 x01, x23;
-          cvt4(kws[j], x01, x23);
-          dot0 = __ffma2_rn(x01, make_float2(__uint_as_float(w[4 * j]), __uint_as_float(w[4 * j + 1])), dot0);
-          dot1 = __ffma2_rn(x23, make_float2(__uint_as_float(w[4 * j + 2]), __uint_as_float(w[4 * j + 3])), dot1);
-        }
-      };
-      tmem_ld16(taddr, wa);
-      tmem_wait_ld();
-      tmem_ld16(taddr + 16, wb16);
-      mac16(wa, kreg[0]);
-      tmem_wait_ld();
-      tmem_ld16(taddr + 32, wa);
-      mac16(wb16, kreg[1]);
-      tmem_wait_ld();
-      tmem_ld16(taddr + 48, wb16);
-      mac16(wa, kreg[2]);
-      tmem_wait_ld();
-      mac16(wb16, kreg[3]);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_n(bar(kBarWEmpty + wb), w_empty_arrivals);  // this warp has read its rows of W
-      const float2 dsum = __fadd2_rn(dot0, dot1);
-      const float sk = __half2float(__ushort_as_half(sk_raw)), sv = __half2float(__ushort_as_half(sv_raw));
-      const float z = valid ? (dsum.x + dsum.y) * sk : -INFINITY;
-      const float y = valid ? z + fast_log2(sv) : -INFINITY;  // log2(0) = -inf: a zero scale drops the token's value
-      sk_raw = sk_n;
-      sv_raw = sv_n;
-
-      // ---- softmax denominator under this warp's own running max (fp32, by the owner threads)
-      const float mz_w = warp_max_redux(z), my_w = warp_max_redux(y);
-      if (mz_w > -INFINITY) {
-        const float m_new = fmaxf(m_run, mz_w);
-        l_lane = fmaf(l_lane, fast_exp2(m_run - m_new), fast_exp2(z - m_new));  // 2^-inf = 0: m_run = -inf, masked tokens
-        m_run = m_new;
-      }
-
-      // ---- the previous tile's value sums are in tensor memory by now: fold them in.  This also
-      //      orders this warp's reads of D and of the references (and, through the MMAs' completion,
-      //      the MMAs' reads of its digit planes) before the planes of this tile are written.
-      if (t > 0) {
-        ok = mbar_wait(bar(kBarDFull + g), (t - 1) & 1);
-        if (!ok) break;
-        tc_fence_after();
-        fold_values(t - 1);
-      }
-
-      // ---- this token's weight for the value MMA, relative to the warp's largest, as three 8-bit digits
-      {
-        const float w = y > -INFINITY ? fast_exp2(y - my_w) : 0.f;  // <= 1
-        const uint32_t nq = __float2uint_rn(w * kPlaneScale);
-        asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes), "r"(nq) : "memory");
-        asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 16), "r"(nq >> 8) : "memory");
-        asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 32), "r"(nq >> 16) : "memory");
-      }
-      fence_proxy_async();
-      tc_fence_before();
-      if (lane == 0) refs[(t & 1) * 4 + q4] = my_w;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(kBarPlanes + g));
-    }
-    // ---- the last tile's value sums
-    if (ok) {
-      ok = warp_wait(bar(kBarDFull + g), (ntiles - 1) & 1);
-      if (ok) {
-        tc_fence_after();
-        fold_values(ntiles - 1);
-      }
-    }
-    if (!ok) atomicMax(&g_status, (unsigned)kTimeoutEpilogue);
-
-    // ---- the head's denominator: the four warps' (max z, sum) pairs under a common maximum
-    const float l_w = warp_sum(l_lane);
-    float2* sums = reinterpret_cast<float2*>(sm + kOffSum) + g * 4;
-    if (lane == 0) sums[q4] = make_float2(m_run, l_w);
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(128) : "memory");
-    float m_all = -INFINITY;
-#pragma unroll
-    for (int w4 = 0; w4 < 4; ++w4) m_all = fmaxf(m_all, sums[w4].x);
-    float l_tot = 0.f;
-#pragma unroll
-    for (int w4 = 0; w4 < 4; ++w4)
-      if (sums[w4].x > -INFINITY) l_tot = fmaf(sums[w4].y, fast_exp2(sums[w4].x - m_all), l_tot);
-    const int64_t slot = balanced ? ((int64_t)b * n_hg + hg + blockIdx.x) * kG + g
-                                  : ((int64_t)b * p.n_q_heads + h) * a.n_splits + split;
-    const int r = 16 * q4 + lane;
-    // sum_s 2^z sv Lv / sum_s 2^z  =  acc * 2^(big_m - m_all) / l
-    // (after a wait that timed out the item's result is poisoned: NaN here propagates through the
-    // merge into the output row, so a time-out cannot pass for a valid result)
-    const float o = !ok ? __int_as_float(0x7fc00000) : big_m > -INFINITY ? acc * fast_exp2(big_m - m_all) / l_tot : 0.f;
-    const bool alone = fused && n_parts == 1;  // this CTA covered the whole (sequence, head): no partials
-    if (!alone) {
-      if (lane < 16 && r < Rv) a.mid_o[slot * Rv + r] = o;
-      // natural-log lse, as the merge kernel expects (stage1.py:216)
-      if (q4 == 0 && lane == 0) a.lse[slot] = m_all * 0.6931471805599453f + logf(l_tot);
-    }
-    if (fused) {
-      // The head's merged latent-space row goes to shared memory (the head's digit-plane area: its
-      // value MMAs are complete), then the head's 128 threads apply U_v and write the output row.
-      float* o_row = reinterpret_cast<float*>(sm + kOffPlanes + 2 * g * kPlaneBytes);
-      int* verdict = reinterpret_cast<int*>(sm + kOffSum) + g * 8;  // the head's (max, sum) pairs were read above
-      bool finish = alone;
-      if (alone) {
-        if (lane < 16 && r < Rv) o_row[r] = o;
-      } else {
-        // the CTA that adds the head's last partial merges them all
-        __threadfence();
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(128) : "memory");
-        if (q4 == 0 && lane == 0) {
-          const unsigned int seen = atomicAdd(ta.arrivals + (int64_t)b * p.n_q_heads + h, 1u);
-          __threadfence();
-          verdict[0] = seen + 1u == (unsigned int)n_parts;
-        }
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(128) : "memory");
-        finish = verdict[0] != 0;
-        if (finish) {
-          const int64_t slot0 = ((int64_t)b * n_hg + hg + c_first) * kG + g;
-          const int rr = q4 * 32 + lane;  // one rank per thread of the head
-          // the first four partials (a head is rarely shared by more CTAs) are requested at once
-          float ls[4], mo[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            ls[i] = i < n_parts ? __ldcg(a.lse + slot0 + (int64_t)i * kG) : -INFINITY;
-            mo[i] = i < n_parts && rr < Rv ? __ldcg(a.mid_o + (slot0 + (int64_t)i * kG) * Rv + rr) : 0.f;
-          }
-          float m = fmaxf(fmaxf(ls[0], ls[1]), fmaxf(ls[2], ls[3]));
-          for (int i = 4; i < n_parts; ++i) m = fmaxf(m, __ldcg(a.lse + slot0 + (int64_t)i * kG));
-          float wsum = 0.f, osum = 0.f;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float w = ls[i] > -INFINITY ? __expf(ls[i] - m) : 0.f;
-            wsum += w;
-            osum = fmaf(w, mo[i], osum);
-          }
-          for (int i = 4; i < n_parts; ++i) {
-            const float w = __expf(__ldcg(a.lse + slot0 + (int64_t)i * kG) - m);
-            wsum += w;
-            if (rr < Rv) osum = fmaf(w, __ldcg(a.mid_o + (slot0 + (int64_t)i * kG) * Rv + rr), osum);
-          }
-          if (rr < Rv) o_row[rr] = osum / wsum;
-        }
-      }
-      if (finish) {
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(128) : "memory");
-        // with peers the finished row is staged (second half of the head's plane area) and leaves as
-        // 16-byte stores, one per thread per peer
-        __half* stage = reinterpret_cast<__half*>(sm + kOffPlanes + 2 * g * kPlaneBytes + kPlaneBytes);
-        __half* out = ta.has_peers ? stage
-                                   : reinterpret_cast<__half*>(p.out) + (int64_t)b * p.out_stride_b + (int64_t)h * p.out_stride_h;
-        const int d = q4 * 32 + lane;
-        if (p.wv == nullptr) {
-          if (d < Rv) out[d] = __float2half_rn(o_row[d]);
-        } else {
-          // out[d] = sum_r O_lat[r] U_v[r, hk*128 + d]: consecutive d in consecutive lanes, four sums and
-          // 32 loads of U_v (L2) in flight
-          const __half* w = reinterpret_cast<const __half*>(p.wv) + (int64_t)hk * p.head_dim + d;
-          float y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f;
-#pragma unroll 8
-          for (int k = 0; k < Rv; k += 4) {
-            y0 = fmaf(o_row[k], __half2float(__ldg(w + (int64_t)k * p.wv_stride_r)), y0);
-            y1 = fmaf(o_row[k + 1], __half2float(__ldg(w + (int64_t)(k + 1) * p.wv_stride_r)), y1);
-            y2 = fmaf(o_row[k + 2], __half2float(__ldg(w + (int64_t)(k + 2) * p.wv_stride_r)), y2);
-            y3 = fmaf(o_row[k + 3], __half2float(__ldg(w + (int64_t)(k + 3) * p.wv_stride_r)), y3);
-          }
-          out[d] = __float2half_rn((y0 + y1) + (y2 + y3));
-        }
-        if (ta.has_peers) {
-          asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(128) : "memory");
-          const int chunks = (p.wv == nullptr ? Rv : p.head_dim) >> 3;
-          const int64_t doff = (int64_t)b * ta.peers.out_stride_b + (int64_t)(h + ta.peers.head_offset) * ta.peers.out_stride_h;
-          for (int idx = d; idx < chunks * ta.peers.n_peers; idx += 128) {
-            const int peer = idx / chunks, c = idx - peer * chunks;
-            *reinterpret_cast<uint4*>(ta.peers.out[peer] + doff + 8 * c) = reinterpret_cast<const uint4*>(stage)[c];
-          }
-        }
-      }
-    }
-  }
-  }
-
-  // ---- end of the item: every role is done with the barriers, the rings and the tensor memory
-  tc_fence_before();
-  __syncthreads();
-  // the next item of the share: the next head group, or the next sequence that has tokens
-  t_first = 0;
-  if (++hg == n_hg) {
-    hg = 0;
-    before_b += tiles_b;
-    do ++b; while (b < p.batch && p.b_seq_len[b] <= 0);
-  }
-  }  // items
-}
-
-// ------------------------------------------------------------------ stage 1
-__global__ void __launch_bounds__(kThreads, 1) stage1_tc_kernel(const __grid_constant__ TcArgs ta) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  const uint32_t sbase = smem_u32(smem_raw);
-  uint8_t* sm = smem_raw;
-  if ((sbase & 1023u) != 0) {  // the swizzled operand tiles need a 1024-byte aligned base
-    if (threadIdx.x == 0) atomicMax(&g_status, (unsigned)kBadSmemAlignment);
-    return;
-  }
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + kOffTmemSlot);
-
-  // ---- once per CTA: tensor memory, descriptor prefetch
-  if (warp == kMmaWarp) {
-    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
-    tmem_relinquish();
-    tc_fence_before();
-  } else if (warp > kMmaWarp && lane == 0) {
-    if (warp == kMmaWarp + 1)
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ta.tmap_table)) : "memory");
-    if (ta.use_tma)
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(warp == kMmaWarp + 1 ? &ta.tmap_k : &ta.tmap_v))
-                   : "memory");
-  }
+  const uint32_t tmem = *tmem_slot;
 
   // ---- register budgets.  The launch gives every thread 96 registers (640 threads); the tile loop of
   //      the epilogue needs more and the control warps far fewer, so the control warpgroup hands
   //      registers back to the pool and the four epilogue warpgroups take them.
-  if (warp < kEpiWarps) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
-    run_share<true>(ta, sm);
+  if (warp < C::kEpiWarps) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kEpiRegs));
+    epilogue_role(ta, sh, sm, sbase, tmem);
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kCtlRegs));
-    run_share<false>(ta, sm);
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kCtlRegs));
+    if (warp == C::kMmaWarp) score_role(ta, sh, sbase, tmem);
+    else if (warp == C::kLoadWarp) copy_role(ta, sh, sbase, sm);
+    else value_role(ta, sh, sbase, sm, tmem, warp - C::kValWarp);
   }
 
   // ---- common exit
   tc_fence_before();
   if (ta.has_peers) __threadfence_system();  // this thread's peer stores are ordered before the count below
   __syncthreads();
-  if (warp == kMmaWarp) {
+  if (warp == C::kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(*tmem_slot, kTmemCols);
   }
   if (ta.has_peers) {
     // the group's barrier, run by whichever CTA finishes last
-    volatile int* last = reinterpret_cast<volatile int*>(sm + kOffSum);
+    volatile int* last = reinterpret_cast<volatile int*>(sm + C::kOffSum);
     if (threadIdx.x == 0) {
       const unsigned int done = atomicAdd(ta.peers.counter, 1u) + 1u;
       *last = done == gridDim.x;
@@ -1300,21 +1481,18 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// One latent tensor [T, Hkv, R] int8 with byte strides (st, sh) as a 3-D tensor map whose outer
-// axes are ordered by stride; box = 64 bytes x 128 token slots x `heads` KV heads (head-major caches,
-// where a head's 128 rows then sit together in shared memory) or x 1 head.  The box is wider than the
-// tensor when the rank is below 64, and may reach past the last head: the missing bytes arrive as zeros.
+// One latent tensor [T, Hkv, R] int8 with byte strides (st, sh) as a 3-D tensor map [Hkv][T][R], whatever the
+// order of the strides; box = 64 bytes x `slots` token slots x `heads` KV heads, so that a head's rows sit
+// together in shared memory.  The box is wider than the tensor when the rank is below 64, and may reach past
+// the last head: the missing bytes arrive as zeros.
 bool encode_latent(CUtensorMap* map, const void* base, int64_t st, int64_t sh, int64_t T, int Hkv, int R, int heads,
-                   int* slot_axis) {
+                   int slots) {
   EncodeTiledFn fn = encode_fn();
-  if (!fn || T <= 0 || T > 0xffffffffll) return false;
-  const bool slot_first = st <= sh;  // head-major storage: the slot axis has the smaller stride
-  if (!slot_first) heads = 1;
-  cuuint64_t dims[3] = {(cuuint64_t)R, (cuuint64_t)(slot_first ? T : Hkv), (cuuint64_t)(slot_first ? Hkv : T)};
-  cuuint64_t strides[2] = {(cuuint64_t)(slot_first ? st : sh), (cuuint64_t)(slot_first ? sh : st)};
-  cuuint32_t box[3] = {64, (cuuint32_t)(slot_first ? kTile : 1), (cuuint32_t)(slot_first ? heads : kTile)};
+  if (!fn || T <= 0 || T > 0xffffffffll || st < 0 || sh < 0) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)R, (cuuint64_t)T, (cuuint64_t)Hkv};
+  cuuint64_t strides[2] = {(cuuint64_t)st, (cuuint64_t)sh};
+  cuuint32_t box[3] = {64, (cuuint32_t)slots, (cuuint32_t)heads};
   cuuint32_t estr[3] = {1, 1, 1};
-  *slot_axis = slot_first ? 1 : 2;
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1349,32 +1527,30 @@ cudaError_t launch_rope_table(void* table, int rows, const KArgs& a, cudaStream_
 
 cudaError_t launch_stage1_tc(const KArgs& a, const void* table, int table_rows, const Stage1Work& work,
                              cudaStream_t stream) {
-  static_assert(tc::kSmemBytes <= 232448, "shared memory budget");
+  using C = tc::Cfg;
   cudaError_t e = cudaFuncSetAttribute(tc::stage1_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)tc::kSmemBytes);
+                                       (int)C::kSmemBytes);
   if (e != cudaSuccess) return e;
   tc::TcArgs ta;
   ta.k = a;
   ta.table_rows = table_rows;
   ta.use_tma = 0;
-  ta.slot_axis = 1;
   ta.box_heads = 1;
-  memset(&ta.tmap_k, 0, sizeof(CUtensorMap));
-  memset(&ta.tmap_v, 0, sizeof(CUtensorMap));
+  for (CUtensorMap* m : {&ta.tmap_k, &ta.tmap_v, &ta.tmap_k16, &ta.tmap_v16}) memset(m, 0, sizeof(CUtensorMap));
   if (!tc::encode_table(&ta.tmap_table, table, table_rows)) return cudaErrorInvalidValue;
   if (a.p.n_token_slots > 0) {
-    // KV heads one group of 4 query heads can touch (its first head is a multiple of 4)
+    // KV heads one group of query heads can touch (its first head is a multiple of the group's size, 4)
     const int gqa = a.p.n_q_heads / a.p.n_kv_heads;
     const int heads = gqa == 1 ? 4 : gqa == 2 ? 2 : gqa % 4 == 0 ? 1 : 2;
-    int ax_k = 1, ax_v = 1;
-    if (tc::encode_latent(&ta.tmap_k, a.p.latent_k, a.p.k_stride_t, a.p.k_stride_h, a.p.n_token_slots,
-                          a.p.n_kv_heads, a.p.rank_k, heads, &ax_k) &&
-        tc::encode_latent(&ta.tmap_v, a.p.latent_v, a.p.v_stride_t, a.p.v_stride_h, a.p.n_token_slots,
-                          a.p.n_kv_heads, a.p.rank_v, heads, &ax_v) &&
-        ax_k == ax_v) {
-      ta.slot_axis = ax_k;
+    auto encode = [&](CUtensorMap* m, bool is_k, int heads_in_box, int slots) {
+      return tc::encode_latent(m, is_k ? a.p.latent_k : a.p.latent_v, is_k ? a.p.k_stride_t : a.p.v_stride_t,
+                               is_k ? a.p.k_stride_h : a.p.v_stride_h, a.p.n_token_slots, a.p.n_kv_heads,
+                               is_k ? a.p.rank_k : a.p.rank_v, heads_in_box, slots);
+    };
+    if (encode(&ta.tmap_k, true, heads, tc::kTile) && encode(&ta.tmap_v, false, heads, tc::kTile) &&
+        encode(&ta.tmap_k16, true, 1, 16) && encode(&ta.tmap_v16, false, 1, 16)) {
       ta.use_tma = 1;
-      ta.box_heads = ax_k == 1 ? heads : 1;
+      ta.box_heads = heads;
     }
   }
   ta.balanced = work.n_ctas > 0;
@@ -1383,12 +1559,12 @@ cudaError_t launch_stage1_tc(const KArgs& a, const void* table, int table_rows, 
   ta.has_peers = work.arrivals != nullptr && work.peers != nullptr;
   if (ta.has_peers) ta.peers = *work.peers;
   else memset(&ta.peers, 0, sizeof(ta.peers));
-  const int grid = work.n_ctas > 0 ? work.n_ctas : a.n_splits * ((a.p.n_q_heads + tc::kG - 1) / tc::kG) * a.p.batch;
+  const int grid = work.n_ctas > 0 ? work.n_ctas : a.n_splits * ((a.p.n_q_heads + C::kG - 1) / C::kG) * a.p.batch;
   if (work.n_ctas > 0 && work.arrivals != nullptr) {
     e = cudaMemsetAsync(work.arrivals, 0, sizeof(unsigned int) * (size_t)a.p.batch * a.p.n_q_heads, stream);
     if (e != cudaSuccess) return e;
   }
-  tc::stage1_tc_kernel<<<grid, tc::kThreads, tc::kSmemBytes, stream>>>(ta);
+  tc::stage1_tc_kernel<<<grid, C::kThreads, C::kSmemBytes, stream>>>(ta);
   return cudaGetLastError();
 }
 
