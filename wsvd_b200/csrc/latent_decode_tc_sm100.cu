@@ -77,7 +77,8 @@ constexpr int kRkMax = 64;
 constexpr uint32_t kAHalfBytes = kTile * 128;       // 128 rows x 64 f16
 constexpr uint32_t kABufBytes = 2 * kAHalfBytes;    // cos half + sin half
 constexpr uint32_t kTmemCols = 512;
-constexpr float kPlaneScale = 16776960.f;           // 2^24 - 256: a weight of 1 is 0xFFFF00
+constexpr float kPlaneScale = 4294967040.f;         // 2^32 - 256: a weight of 1 is 0xFFFFFF00
+constexpr float kNone = -3.0e38f;                   // log2-domain reference of something that is still empty
 
 // Shape of the CTA.
 struct Cfg {
@@ -90,7 +91,7 @@ struct Cfg {
   static constexpr int kRowBytes = 64;             // a latent row in shared memory (rank < 64: zero-filled)
   static constexpr int kKSlots = 1;  // tiles of K: a tile's rows are copied to registers at the top of the tile
   static constexpr int kVSlots = 2;  // tiles of V: the tile whose value MMAs are pending, and the next tile in flight
-  static constexpr int kWBufs = 3;   // W accumulators of 128 columns (one pair of heads each)
+  static constexpr int kWBufs = 2;   // W accumulators of 128 columns (one pair of heads each)
   // Registers per thread after the two groups have re-balanced them.  The pool is the CTA's own: what
   // the control warpgroup hands back, (96 - 64) * 128, is exactly what the epilogue warpgroups take,
   // (104 - 96) * 512.  (A request the pool cannot satisfy would block for ever.)
@@ -104,7 +105,8 @@ struct Cfg {
   static constexpr uint32_t kUnitBytes = kG * kHeadBytes;    // a ring slot: one tile of K or V for the group's KV heads
   static constexpr uint32_t kBHalfBytes = kG * kRkMax * 128; // rows of 64 f16
   static constexpr uint32_t kPlaneBytes = 256;               // per pair of warps: 2 chunks of 16 tokens x 8 rows x 16 bytes
-  static constexpr uint32_t kTmemD = kWBufs * 128;           // first column of the value accumulators: 8 per (head, warp)
+  static constexpr uint32_t kTmemD = kWBufs * 128;           // first column of the value accumulators: 2 x 8 per (head, warp)
+  static_assert(kTmemD + kG * 64 <= kTmemCols, "tensor memory");
 
   // shared-memory map (offsets from a 1024-byte aligned base)
   static constexpr uint32_t kOffB = 0;
@@ -112,7 +114,7 @@ struct Cfg {
   static constexpr uint32_t kOffV = kOffA + 2 * kABufBytes;
   static constexpr uint32_t kOffK = kOffV + kVSlots * kUnitBytes;
   static constexpr uint32_t kOffPlanes = kOffK + kKSlots * kUnitBytes;
-  static constexpr uint32_t kOffRef = kOffPlanes + 2 * kG * kPlaneBytes;  // [head][tile parity][warp] reference max y of the planes
+  static constexpr uint32_t kOffRef = kOffPlanes + 2 * kG * kPlaneBytes;  // [head][tile parity][warp] reference that a warp left with this tile
   static constexpr uint32_t kOffSum = kOffRef + kG * 2 * 4 * 4;           // [head][warp] (max z, denominator) at the end
   static constexpr uint32_t kOffMode = kOffSum + kG * 4 * 8;              // [4] how the K and V rows of a tile arrive (ring)
   static constexpr uint32_t kOffItem = kOffMode + 16;                     // [head][item parity] ItemState
@@ -264,6 +266,13 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(taddr)
                : "memory");
+}
+// the loaded registers pass through the wait, so that nothing that uses them can be moved in front of it
+template <int N>
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[N]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // warp-wide maximum in one instruction (sm_100a)
@@ -590,52 +599,65 @@ __device__ __forceinline__ void copy_role(const TcArgs& ta, const Share& sh, uin
 }
 
 // ------------------------------------------------------------------ value MMAs (one warp per pair of heads)
-// Lane 0 and lane 1 serve one head each: they wait for the digit planes of the head's four warps and issue the
-// head's value MMAs (one per warp of 32 tokens, each into its own 8 columns of tensor memory); two commits
-// then tell the epilogue warps (D full) and the copying warp (V empty) when the MMAs have completed.
-__device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, uint32_t sbase, const uint8_t* sm,
+// One byte per warp of head g: bit 0 which of its two value accumulators this tile's sums go to, bit 1 whether
+// they are added to it.  (It sits in the unused last word of the head's first ItemState.)
+__device__ __forceinline__ volatile uint32_t* value_modes(uint8_t* sm, int g) {
+  return reinterpret_cast<volatile uint32_t*>(sm + Cfg::kOffItem + g * 128 + 60);
+}
+
+// The warp serves its two heads in turn: it waits for the digit planes of a head's four warps and issues the
+// head's value MMAs (one per warp of 32 tokens, each into 8 columns of tensor memory of its own); two commits
+// then tell the epilogue warps (D full) and the copying warp (V empty) when the MMAs have completed.  All lanes
+// hold the same operands and flags: the instruction takes them from uniform registers, and when two lanes
+// served a head each, one head's sums were now and then added to, or not, as the other's should have been.
+__device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, uint32_t sbase, uint8_t* sm,
                                            uint32_t tmem, int pair) {
   using C = Cfg;
   const WsvdLatentDecodeParams& p = ta.k.p;
-  const int lane = threadIdx.x & 31;
   const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG, gqa = p.n_q_heads / p.n_kv_heads;
   auto bar = [&](int i) { return sbase + C::kOffBar + 8u * i; };
-  const int g = 2 * pair + lane;
   const uint32_t idesc = instr_desc_i8(64, 8);
-  const uint64_t pdesc0 = smem_desc_k_plain(sbase + C::kOffPlanes + 2 * g * C::kPlaneBytes);
-  const uint32_t d_tmem = tmem + C::kTmemD + 32 * g;
   const volatile int* mode = reinterpret_cast<const volatile int*>(sm + C::kOffMode);
-  const uint64_t vdesc0 = smem_desc_mn_sw64(sbase + C::kOffV);
+  const uint64_t vdesc0 = smem_desc_mn_sw64(sbase + C::kOffV), pdesc0 = smem_desc_k_plain(sbase + C::kOffPlanes);
+  const uint32_t v_lo = (uint32_t)vdesc0, v_hi = (uint32_t)(vdesc0 >> 32), p_lo = (uint32_t)pdesc0, p_hi = (uint32_t)(pdesc0 >> 32);
+  const bool issuer = elect_one();
   Walk w;
   bool ok = true;
-  uint32_t T = 0, mine = 0;  // tiles so far, and those this head took part in
-  if (lane < 2) {
-    for (bool more = w.start(ta, sh, n_hg); more && ok; more = w.next(p, n_hg)) {
-      const int h0 = w.hg * C::kG, G = min(C::kG, p.n_q_heads - h0);
-      if (g >= G) {
-        T += w.ntiles;
-        continue;
-      }
-      const int sub = (h0 + g) / gqa - h0 / gqa;
-      for (int t = 0; t < w.ntiles && ok; ++t, ++T, ++mine) {
-        const uint32_t vslot = T % C::kVSlots;
-        // the V rows arrive long before the planes are ready: wait for them first, off the
-        // critical path from "planes ready" to "D full"
-        ok = mbar_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
-        if (ok) ok = mbar_wait(bar(C::kBarPlanes + g), mine & 1);
-        if (ok) {
-          tc_fence_after();
-          // copied rows sit at the head's KV head, gathered ones at the head itself
-          const uint32_t region = vslot * C::kUnitBytes + (mode[T & 3] == kTileGather ? g : sub) * C::kHeadBytes;
+  uint32_t T = 0, mine[2] = {0, 0};  // tiles so far, and those that each head took part in
+  for (bool more = w.start(ta, sh, n_hg); more && ok; more = w.next(p, n_hg)) {
+    const int h0 = w.hg * C::kG, G = min(C::kG, p.n_q_heads - h0);
+    if (2 * pair >= G) {
+      T += w.ntiles;
+      continue;
+    }
+    for (int t = 0; t < w.ntiles && ok; ++t, ++T) {
+      const uint32_t vslot = T % C::kVSlots;
+      // the V rows arrive long before the planes are ready: wait for them first, off the
+      // critical path from "planes ready" to "D full"
+      ok = warp_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
 #pragma unroll
-          for (int w4 = 0; w4 < 4; ++w4) {
-            const uint32_t voff = region + w4 * 2048;  // the 32 tokens of warp w4: 32 rows of 64 bytes
-            umma_i8(d_tmem + 8 * w4, vdesc0 + (voff >> 4), pdesc0 + (((w4 >> 1) * C::kPlaneBytes) >> 4), idesc, 0);
-          }
+      for (int j = 0; j < 2; ++j) {
+        const int g = 2 * pair + j;
+        if (g >= G || !ok) break;
+        ok = warp_wait(bar(C::kBarPlanes + g), mine[j] & 1);
+        if (!ok) break;
+        ++mine[j];
+        tc_fence_after();
+        const uint32_t how = *value_modes(sm, g);  // a byte per warp: which of its accumulators, added to or started
+        // copied rows sit at the head's KV head, gathered ones at the head itself
+        const int sub = mode[T & 3] == kTileGather ? g : (h0 + g) / gqa - h0 / gqa;
+        const uint32_t v_at = v_lo + ((vslot * C::kUnitBytes + sub * C::kHeadBytes) >> 4);
+        const uint32_t d_tmem = tmem + C::kTmemD + 64 * g;
+        if (issuer) {
+#pragma unroll
+          for (int w4 = 0; w4 < 4; ++w4)  // the 32 tokens of warp w4: 32 rows of 64 bytes
+            umma_i8(d_tmem + 16 * w4 + ((how >> (8 * w4)) & 1) * 8, join64(v_at + ((w4 * 2048) >> 4), v_hi),
+                    join64(p_lo + (((2 * g + (w4 >> 1)) * C::kPlaneBytes) >> 4), p_hi), idesc, (how >> (8 * w4)) & 2);
           umma_commit(bar(C::kBarDFull + g));
           umma_commit(bar(C::kBarVEmpty + vslot));
           if (g == 0 && G < C::kG) mbar_arrive_n(bar(C::kBarVEmpty + vslot), C::kG - G);  // for the heads that are not there
         }
+        __syncwarp();
       }
     }
   }
@@ -961,36 +983,48 @@ __device__ __forceinline__ volatile int* item_state(uint8_t* sm, int g, uint32_t
   return reinterpret_cast<volatile int*>(sm + Cfg::kOffItem) + (g * 2 + (item & 1)) * 16;
 }
 
-// One head's running sums over the tiles of an item.
+// One head's running sums over the tiles of an item, all in the log2 domain and fp32.
+//  - Denominator: l_lane, this lane's tokens, under the warp's reference m_run.  The reference follows the warp's
+//    maximum of z only when that has grown by more than kSlackZ: a weight may reach 2^kSlackZ, which fp32 does not mind.
+//  - Values: the sums of this warp's tokens stay in tensor memory, in integers relative to 2^my_ref, until a weight
+//    would no longer fit.  Then the warp goes over to its other accumulator with a new reference and leaves
+//    the old one to be folded into acc (rank 16*q4 + lane, lanes 0..15, all four warps' tokens, under big_m).
+//    New references leave kSlackY bits of room, so that a few per item are enough: folding every tile cost an
+//    eighth of the kernel's instructions.
 struct HeadSums {
-  float m_run, l_lane;  // softmax denominator of this lane's tokens, under the warp's running maximum of z
-  float big_m, acc;     // value sum of rank 16*q4 + lane (lanes 0..15), all four warps' tokens, under the running
-                        // reference big_m (max y of every (tile, warp) folded in so far)
+  float m_run, l_lane;
+  float my_ref, scale;  // scale: 2^(m_run - my_ref) * kPlaneScale
+  float big_m, acc;
+  uint32_t bufs;        // bit w4: the accumulator warp w4 of the head is using
 };
+constexpr float kSlackZ = 8.f;
+constexpr int kSlackY = 3;
 
-// Fold in the value sums of the head's tile number tp: D[rank][8*w + 0..2] are the three digit-plane sums over
-// the 32 tokens of warp w, whose weights were taken relative to refs[tp & 1][w].
-__device__ __forceinline__ void fold_values(HeadSums& hs, uint32_t d_addr, const float* refs, uint32_t tp) {
-  uint32_t d[4][4];
-#pragma unroll
-  for (int w4 = 0; w4 < 4; ++w4) tmem_ld4(d_addr + 8 * w4 + 3 * (w4 & 1), d[w4]);
+// Fold in one accumulator of warp w4 of the head: D[rank][0..3] are its four digit-plane sums, relative to 2^ref.
+__device__ __forceinline__ void fold_values(HeadSums& hs, uint32_t d_addr, int w4, uint32_t buf, float ref) {
+  uint32_t d[4];
+  tmem_ld4(d_addr + 16 * w4 + 8 * buf + 4 * (w4 & 1), d);
+  tmem_wait_ld(d);
+  const float m_new = fmaxf(hs.big_m, ref);
+  const float v = fmaf((float)(int32_t)d[3], 16777216.f, fmaf((float)(int32_t)d[2], 65536.f, fmaf((float)(int32_t)d[1], 256.f, (float)(int32_t)d[0])));
+  hs.acc = fmaf(v, fast_exp2(ref - m_new) * (1.f / kPlaneScale), hs.acc * fast_exp2(hs.big_m - m_new));
+  hs.big_m = m_new;
+}
+
+// What the head's warps have left behind with tile number tp (see HeadSums).
+__device__ __forceinline__ void fold_left(HeadSums& hs, uint32_t d_addr, const float* refs, uint32_t tp) {
   const float4 rf = *reinterpret_cast<const float4*>(refs + (tp & 1) * 4);
-  const float ref[4] = {rf.x, rf.y, rf.z, rf.w};
-  tmem_wait_ld();
-  float m_new = hs.big_m;
-#pragma unroll
-  for (int w4 = 0; w4 < 4; ++w4) m_new = fmaxf(m_new, ref[w4]);
-  if (m_new > -INFINITY) {
-    hs.acc *= fast_exp2(hs.big_m - m_new);  // big_m = -inf -> factor 0
-#pragma unroll
+  if (fmaxf(fmaxf(rf.x, rf.y), fmaxf(rf.z, rf.w)) > kNone) {
+    const float ref[4] = {rf.x, rf.y, rf.z, rf.w};
+    __syncwarp();
+#pragma unroll 1
     for (int w4 = 0; w4 < 4; ++w4) {
-      if (ref[w4] > -INFINITY) {  // (a warp without tokens in this tile has no MMA and reference -inf)
-        // the two low digit sums are combined as integers (|d| <= 32 * 255 * 128 < 2^21)
-        const float v = fmaf((float)(int32_t)d[w4][2], 65536.f, (float)((int32_t)d[w4][1] * 256 + (int32_t)d[w4][0]));
-        hs.acc = fmaf(v, fast_exp2(ref[w4] - m_new) * (1.f / kPlaneScale), hs.acc);
+      const float r = w4 == 0 ? ref[0] : w4 == 1 ? ref[1] : w4 == 2 ? ref[2] : ref[3];
+      if (r > kNone) {
+        fold_values(hs, d_addr, w4, (hs.bufs >> w4) & 1, r);
+        hs.bufs ^= 1u << w4;
       }
     }
-    hs.big_m = m_new;
   }
 }
 
@@ -1005,15 +1039,16 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + C::kOffTmemSlot);
   const volatile int* st = item_state(sm, g, item);
   const volatile int* mode = reinterpret_cast<const volatile int*>(sm + C::kOffMode);
-  float* refs = reinterpret_cast<float*>(sm + C::kOffRef) + g * 8;  // [tile parity][warp]: max y the warp's planes refer to
+  float* refs = reinterpret_cast<float*>(sm + C::kOffRef) + g * 8;  // [tile parity][warp]: reference left behind, or kNone
   // Digit planes: the two warps of half a tile share one 8-row block (the MMA's B operand has 8
-  // rows): rows 0..2 hold the even warp's digits, rows 3..5 the odd warp's.  Each warp's MMA reads
-  // the whole block, so its columns 3..5 (or 0..2) are the other warp's weights times this warp's
-  // V rows: garbage that nobody reads.  Rows 6 and 7 are never written.
-  const uint32_t my_planes = sbase + C::kOffPlanes + (2 * g + (q4 >> 1)) * C::kPlaneBytes + (lane >> 4) * 128 + (q4 & 1) * 48 + (lane & 15);
-  const uint32_t d_addr = tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 32 * g;
+  // rows): rows 0..3 hold the even warp's digits, rows 4..7 the odd warp's.  Each warp's MMA reads
+  // the whole block, so its columns 4..7 (or 0..3) are the other warp's weights times this warp's
+  // V rows: garbage that nobody reads.
+  const uint32_t my_planes = sbase + C::kOffPlanes + (2 * g + (q4 >> 1)) * C::kPlaneBytes + (lane >> 4) * 128 + (q4 & 1) * 64 + (lane & 15);
+  const uint32_t d_addr = tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 64 * g;
   const int h0 = st[kItHg] * C::kG, G = min(C::kG, p.n_q_heads - h0), npairs = (G + 1) >> 1;
   bool ok = true;
+  uint32_t own_buf = 0;  // this warp's accumulator
   const int hk = (h0 + g) / gqa;
   const int pr = g >> 1, sub = hk - h0 / gqa;  // sub: this head's KV head inside a unit
   const int lo = st[kItLo], hi = st[kItHi], ntiles = st[kItTiles];
@@ -1120,26 +1155,46 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     const float2 dsum = __fadd2_rn(dot0, dot1);
     const float sk = __half2float(__ushort_as_half(sk_raw)), sv = __half2float(__ushort_as_half(sv_raw));
     const float z = valid ? (dsum.x + dsum.y) * sk : -INFINITY;
-    const float y = valid ? z + fast_log2(sv) : -INFINITY;  // log2(0) = -inf: a zero scale drops the token's value
     sk_raw = sk_n;
     sv_raw = sv_n;
 
-    // ---- softmax denominator under this warp's own running max (fp32, by the owner threads)
-    const float mz_w = warp_max_redux(z), my_w = warp_max_redux(y);
-    if (mz_w > -INFINITY) {
-      const float m_new = fmaxf(hs.m_run, mz_w);
-      hs.l_lane = fmaf(hs.l_lane, fast_exp2(hs.m_run - m_new), fast_exp2(z - m_new));  // 2^-inf = 0: hs.m_run = -inf, masked tokens
-      hs.m_run = m_new;
+    // ---- softmax weights under the warp's reference, denominator (fp32, by the owner threads)
+    const float mz_w = warp_max_redux(z);
+    bool renew = mz_w > hs.m_run + kSlackZ;
+    if (renew) {
+      hs.l_lane *= fast_exp2(hs.m_run - mz_w);
+      hs.m_run = mz_w;
+    }
+    const float e = fast_exp2(z - hs.m_run);  // masked tokens: 2^-inf = 0
+    hs.l_lane += e;
+    const float pv = e * sv, pv_w = warp_max_redux(pv);
+    // ---- does every weight fit under the reference of the value sums?  (The accumulators are integers of 32 bits
+    //      per digit: 32 tokens add at most 2^20, so 1024 tiles are well inside.)
+    float left = kNone;
+    uint32_t adds = t > 0 ? 2u : 0u;
+    renew = renew || pv_w * hs.scale > kPlaneScale || (t & 1023) == 1023;
+    if (renew) {
+      left = hs.my_ref;
+      if (left > kNone) {
+        adds = 0u;
+        own_buf ^= 1u;
+      }
+      // 2^k, the power of two that leaves the largest weight kSlackY bits of room (weights 2^-60 below the largest
+      // of the softmax do not show in the result)
+      const int k = min(max((int)((__float_as_uint(pv_w) >> 23) & 0xff) - 126 + kSlackY, -60), 100);
+      if (pv_w == INFINITY) hs.l_lane = __int_as_float(0x7fc00000);  // an infinite V scale: the result is NaN
+      hs.my_ref = hs.m_run + (float)k;
+      hs.scale = kPlaneScale * __uint_as_float((uint32_t)(127 - k) << 23);
     }
 
-    // ---- the previous tile's value sums are in tensor memory by now: fold them in.  This also
-    //      orders this warp's reads of D and of the references (and, through the MMAs' completion,
+    // ---- the previous tile's value MMAs are complete: fold in what the head's warps left behind with it.  This
+    //      also orders this warp's reads of D and of the references (and, through the MMAs' completion,
     //      the MMAs' reads of its digit planes and V rows) before those of this tile are written.
     if (t > 0) {
       ok = mbar_wait(bar(C::kBarDFull + g), (mt - 1) & 1);
       if (!ok) break;
       tc_fence_after();
-      fold_values(hs, d_addr, refs, mt - 1);
+      fold_left(hs, d_addr, refs, mt - 1);
     }
     if (gather) {
       // the copying warp's arrival says that every head's value MMAs on the slot are complete
@@ -1153,17 +1208,20 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
                      : "memory");
     }
 
-    // ---- this token's weight for the value MMA, relative to the warp's largest, as three 8-bit digits
+    // ---- this token's weight for the value MMA, relative to the warp's reference, as four 8-bit digits
     {
-      const float wgt = y > -INFINITY ? fast_exp2(y - my_w) : 0.f;  // <= 1
-      const uint32_t nq = __float2uint_rn(wgt * kPlaneScale);
+      const uint32_t nq = __float2uint_rn(pv * hs.scale);
       asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes), "r"(nq) : "memory");
       asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 16), "r"(nq >> 8) : "memory");
       asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 32), "r"(nq >> 16) : "memory");
+      asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 48), "r"(nq >> 24) : "memory");
     }
     fence_proxy_async();
     tc_fence_before();
-    if (lane == 0) refs[(mt & 1) * 4 + q4] = my_w;
+    if (lane == 0) {
+      refs[(mt & 1) * 4 + q4] = left;
+      reinterpret_cast<volatile uint8_t*>(value_modes(sm, g))[q4] = (uint8_t)(own_buf | adds);
+    }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(C::kBarPlanes + g));
   }
@@ -1215,7 +1273,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
     if (pending) finish_head(ta, sm, g, state(item + 1), seen);  // the item before, while the first score MMAs of this one run
     pending = false;
 
-    HeadSums hs = {-INFINITY, 0.f, -INFINITY, 0.f};
+    HeadSums hs = {kNone, 0.f, kNone, 0.f, kNone, 0.f, 0u};
     if (active && ok) ok = run_tiles(ta, sm, item, hs);
 
     // ---- the item's end.  What the next item needs is requested before the last value sums are waited for.
@@ -1240,35 +1298,47 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
     if (active) {
       const uint32_t last = st[kItMine] + st[kItTiles] - 1;  // count of the head's last tile
       const int b = st[kItB], hg = st[kItHg], h = h0 + g;
+      const uint32_t d_addr = tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 64 * g;
+      float* refs = reinterpret_cast<float*>(sm + C::kOffRef) + g * 8;
       if (ok) {
         ok = warp_wait(bar(C::kBarDFull + g), last & 1);
         if (ok) {
           tc_fence_after();
-          fold_values(hs, tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 32 * g, reinterpret_cast<const float*>(sm + C::kOffRef) + g * 8, last);
-          tc_fence_before();
+          fold_left(hs, d_addr, refs, last);
         }
       }
       if (!ok) atomicMax(&g_status, (unsigned)kTimeoutEpilogue);
 
-      // ---- the head's denominator: the four warps' (max z, sum) pairs under a common maximum
+      // ---- the head's denominator: the four warps' (reference, sum) pairs under a common maximum; with them the
+      //      references of the value accumulators in use
       const float l_w = warp_sum(hs.l_lane);
       float2* sums = reinterpret_cast<float2*>(sm + C::kOffSum) + g * 4;
-      if (lane == 0) sums[q4] = make_float2(hs.m_run, l_w);
+      if (lane == 0) {
+        sums[q4] = make_float2(hs.m_run, l_w);
+        refs[((last + 1) & 1) * 4 + q4] = hs.my_ref;
+      }
       head_sync();
-      float m_all = -INFINITY;
+      if (ok) {
+        const float4 rf = *reinterpret_cast<const float4*>(refs + ((last + 1) & 1) * 4);
+        if (rf.x > kNone) fold_values(hs, d_addr, 0, hs.bufs & 1, rf.x);
+        if (rf.y > kNone) fold_values(hs, d_addr, 1, (hs.bufs >> 1) & 1, rf.y);
+        if (rf.z > kNone) fold_values(hs, d_addr, 2, (hs.bufs >> 2) & 1, rf.z);
+        if (rf.w > kNone) fold_values(hs, d_addr, 3, (hs.bufs >> 3) & 1, rf.w);
+        tc_fence_before();
+      }
+      float m_all = kNone;
 #pragma unroll
       for (int w4 = 0; w4 < 4; ++w4) m_all = fmaxf(m_all, sums[w4].x);
-      float l_tot = 0.f;
+      float l_tot = 0.f;  // (a NaN in any warp's sum stays)
 #pragma unroll
-      for (int w4 = 0; w4 < 4; ++w4)
-        if (sums[w4].x > -INFINITY) l_tot = fmaf(sums[w4].y, fast_exp2(sums[w4].x - m_all), l_tot);
+      for (int w4 = 0; w4 < 4; ++w4) l_tot = fmaf(sums[w4].y, fast_exp2(sums[w4].x - m_all), l_tot);
       const int64_t slot = balanced ? ((int64_t)b * n_hg + hg + blockIdx.x) * C::kG + g
                                     : ((int64_t)b * p.n_q_heads + h) * a.n_splits + blockIdx.x % a.n_splits;
       const int r = 16 * q4 + lane;
       // sum_s 2^z sv Lv / sum_s 2^z  =  acc * 2^(big_m - m_all) / l
       // (after a wait that timed out the item's result is poisoned: NaN here propagates through the
       // merge into the output row, so a time-out cannot pass for a valid result)
-      const float o = !ok ? __int_as_float(0x7fc00000) : hs.big_m > -INFINITY ? hs.acc * fast_exp2(hs.big_m - m_all) / l_tot : 0.f;
+      const float o = !ok ? __int_as_float(0x7fc00000) : (hs.big_m > kNone ? hs.acc * fast_exp2(hs.big_m - m_all) : 0.f) / l_tot;
       if (!fused || n_parts > 1) {
         if (lane < 16 && r < Rv) a.mid_o[slot * Rv + r] = o;
         // natural-log lse, as the merge kernel expects (stage1.py:216)
@@ -1278,9 +1348,9 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
         // memory (the head's plane area: its value MMAs are complete).
         reinterpret_cast<float*>(sm + C::kOffPlanes + 2 * g * C::kPlaneBytes)[r] = o;
       }
+      if (fused && n_parts > 1) __threadfence();
+      head_sync();  // the partial is out, the (max, sum) pairs and the references have been read
       if (fused) {
-        if (n_parts > 1) __threadfence();
-        head_sync();  // the partial is out, the (max, sum) pairs have been read
         // the counter's answer is needed only after the next item's [P;Q] build
         if (n_parts > 1 && row == 0) seen = atomicAdd(ta.arrivals + (int64_t)b * p.n_q_heads + h, 1u);
         pending = true;
