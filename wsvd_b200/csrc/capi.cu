@@ -60,6 +60,23 @@ bool tc_eligible(const WsvdLatentDecodeParams* p) {
   return true;
 }
 
+// The tcgen05 kernel with f16 latents: the balanced mode alone, chosen by WSVD_KERNEL_AUTO.  Ranks are multiples of 8
+// and rows start on 16-byte boundaries (tensor copies, 16-byte row loads).  From one tile of 128 tokens and two heads per
+// SM on: below that most SMs would idle, and the warp-MMA kernel, which cuts the context finer, is as fast
+// (2 sequences of 2048 and 900 tokens with 8 heads: @@SMALL@@).
+bool tc_f16_eligible(const WsvdLatentDecodeParams* p) {
+  if (p->kernel != WSVD_KERNEL_AUTO || p->latent_dtype != WSVD_F16 || p->split_len != 0) return false;
+  if (p->head_dim != 128) return false;
+  if (p->rank_k % 8 != 0 || p->rank_k > 64 || p->rank_v % 8 != 0 || p->rank_v > 64) return false;
+  if (p->pos_offset != nullptr && p->rope_table == nullptr) return false;
+  if (!aligned16(p->latent_k) || !aligned16(p->latent_v)) return false;
+  if (!aligned16(p->q) || p->q_stride_b % 8 || p->q_stride_h % 8) return false;  // 16-byte loads of q
+  if (p->k_stride_t % 8 || p->k_stride_h % 8 || p->v_stride_t % 8 || p->v_stride_h % 8) return false;
+  if (p->rope_table && (!aligned16(p->rope_table) || p->rope_table_rows < ((p->max_len + 127) / 128) * 128)) return false;
+  const int64_t groups = (p->n_q_heads + wsvd::kBalancedGroupF16 - 1) / wsvd::kBalancedGroupF16;
+  return p->batch * groups * ((p->max_len + 127) / 128) >= 148;
+}
+
 // the caller's position table serves the warp-MMA kernel too ([2][rows][64] f16 is its layout for head_dim 128)
 bool mma_caller_table(const WsvdLatentDecodeParams* p) {
   return p->rope_table && p->head_dim == 128 && aligned16(p->rope_table) &&
@@ -146,7 +163,8 @@ void fill_args(const WsvdLatentDecodeParams* p, float* mid_o, float* lse, int sp
 // always runs fixed-length splits).
 int run_stage1(const wsvd::KArgs& a, void* scratch_table, const wsvd::Stage1Work& work, cudaStream_t stream) {
   if (a.p.batch == 0) return WSVD_OK;
-  const bool tc = tc_eligible(&a.p) && a.split_len % 128 == 0 && (a.p.rope_table || scratch_table);
+  const bool f16 = work.n_ctas > 0 && tc_f16_eligible(&a.p);
+  const bool tc = (f16 || (tc_eligible(&a.p) && a.split_len % 128 == 0)) && (a.p.rope_table || scratch_table);
   if (!tc) {
     if (a.p.kernel == WSVD_KERNEL_TC) return WSVD_ERR_UNSUPPORTED;
     if (mma_eligible(&a.p) && (mma_caller_table(&a.p) || scratch_table)) {
@@ -179,7 +197,12 @@ int run_stage1(const wsvd::KArgs& a, void* scratch_table, const wsvd::Stage1Work
 
 // Without a split length from the caller, a problem the tensor-core kernel can run is cut into
 // equal shares of tiles, one per SM, instead of fixed-length splits.
-bool balanced_mode(const WsvdLatentDecodeParams* p) { return p->split_len == 0 && tc_eligible(p); }
+bool balanced_mode(const WsvdLatentDecodeParams* p) {
+  return p->split_len == 0 && (tc_eligible(p) || tc_f16_eligible(p));
+}
+int balanced_group(const WsvdLatentDecodeParams* p) {
+  return p->latent_dtype == WSVD_F16 ? wsvd::kBalancedGroupF16 : wsvd::kBalancedGroup;
+}
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
@@ -197,8 +220,8 @@ struct Layout {
 Layout workspace_layout(const WsvdLatentDecodeParams* p, int n_splits) {
   Layout l = {};
   const bool bal = balanced_mode(p);
-  const size_t n_hg = ((size_t)p->n_q_heads + wsvd::kBalancedGroup - 1) / wsvd::kBalancedGroup;
-  l.slots = bal ? ((size_t)p->batch * n_hg + wsvd::kMaxBalancedCtas) * wsvd::kBalancedGroup
+  const size_t group = balanced_group(p), n_hg = ((size_t)p->n_q_heads + group - 1) / group;
+  l.slots = bal ? ((size_t)p->batch * n_hg + wsvd::kMaxBalancedCtas) * group
                 : (size_t)p->batch * p->n_q_heads * n_splits;
   size_t off = align256(l.slots * ((size_t)p->rank_v + 1) * sizeof(float));
   if (bal) {
@@ -208,7 +231,7 @@ Layout workspace_layout(const WsvdLatentDecodeParams* p, int n_splits) {
     off += align256((size_t)p->batch * p->n_q_heads * sizeof(uint32_t));
   }
   l.table_off = off;
-  if (tc_eligible(p)) {
+  if (tc_eligible(p) || tc_f16_eligible(p)) {
     if (!p->rope_table) l.table_bytes = wsvd::rope_table_bytes(table_rows_for(p->max_len));
   } else if (mma_eligible(p) && !mma_caller_table(p)) {
     l.table_bytes = wsvd::mma_table_bytes(table_rows_for(p->max_len), p->head_dim);
@@ -229,7 +252,7 @@ int balanced_ctas(const WsvdLatentDecodeParams* p, int* n_ctas) {
     if (e != cudaSuccess) return cuda_fail(e);
     if (dev >= 0 && dev < 64) sm_count[dev] = sms;
   }
-  const long n_hg = (p->n_q_heads + wsvd::kBalancedGroup - 1) / wsvd::kBalancedGroup;
+  const long n_hg = (p->n_q_heads + balanced_group(p) - 1) / balanced_group(p);
   const long most = (long)p->batch * n_hg * ((p->max_len + 127) / 128);
   long n = sms < wsvd::kMaxBalancedCtas ? sms : wsvd::kMaxBalancedCtas;
   if (n > most) n = most;
@@ -280,7 +303,15 @@ size_t wsvd_latent_decode_workspace_bytes(const WsvdLatentDecodeParams* p) {
   if (!p || p->max_len < 0 || p->split_len < 0 || p->batch < 0 || p->n_q_heads <= 0 || p->rank_v <= 0) return 0;
   int sl, ns;
   plan(p, &sl, &ns);
-  return workspace_layout(p, ns).total;
+  size_t need = workspace_layout(p, ns).total;
+  if (tc_f16_eligible(p)) {
+    // never less than the split plan that wsvd_latent_decode_plan reports for the same block would take
+    WsvdLatentDecodeParams q = *p;
+    q.kernel = WSVD_KERNEL_MMA;
+    const size_t split = workspace_layout(&q, ns).total;
+    if (split > need) need = split;
+  }
+  return need;
 }
 
 size_t wsvd_rope_table_bytes(int32_t positions, int32_t head_dim) {
@@ -356,7 +387,7 @@ static int decode_impl(const WsvdLatentDecodeParams* p, const WsvdPeerSet* peers
   fill_args(p, mid_o, lse, sl, ns, &a);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   void* scratch_table = l.table_bytes ? ws + l.table_off : nullptr;
-  wsvd::PartialIndex where = {nullptr, 0, ns, sl};
+  wsvd::PartialIndex where = {nullptr, 0, ns, sl, balanced_group(p)};
   wsvd::Stage1Work work = {0, nullptr, nullptr, nullptr};
   wsvd::PeerArgs pa;
   if (balanced_mode(p)) {
@@ -525,7 +556,7 @@ int wsvd_dense_decode_f16(const WsvdDenseDecodeParams* p, void* workspace, size_
   cudaError_t e = wsvd::launch_dense_stage1(a, s);
   if (e != cudaSuccess) return cuda_fail(e);
   e = wsvd::launch_stage2(a.mid_o, a.lse, p->b_seq_len, p->out, p->out_stride_b, p->out_stride_h, p->batch,
-                          p->n_q_heads, wsvd::PartialIndex{nullptr, 0, ns, sl}, p->head_dim, nullptr, 0, 1,
+                          p->n_q_heads, wsvd::PartialIndex{nullptr, 0, ns, sl, wsvd::kBalancedGroup}, p->head_dim, nullptr, 0, 1,
                           p->head_dim, s);
   return e == cudaSuccess ? WSVD_OK : cuda_fail(e);
 }
@@ -542,7 +573,7 @@ int wsvd_decode_stage2(const float* mid_o, const float* lse, const int32_t* b_se
     return WSVD_ERR_BAD_SHAPE;
   if (batch == 0) return WSVD_OK;
   cudaError_t e = wsvd::launch_stage2(mid_o, lse, b_seq_len, out, out_stride_b, out_stride_h, batch, n_q_heads,
-                                      wsvd::PartialIndex{nullptr, 0, n_splits, split_len}, width, wv, wv_stride_r,
+                                      wsvd::PartialIndex{nullptr, 0, n_splits, split_len, wsvd::kBalancedGroup}, width, wv, wv_stride_r,
                                       wv ? n_kv_heads : 1, head_dim, reinterpret_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? WSVD_OK : cuda_fail(e);
 }

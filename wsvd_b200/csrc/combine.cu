@@ -36,15 +36,15 @@ stage2_kernel(const float* __restrict__ mid_o, const float* __restrict__ lse, co
     ns = min(where.n_splits, (n + where.split_len - 1) / where.split_len);
     slot0 = ((int64_t)b * n_q_heads + h) * where.n_splits;
   } else if (n > 0) {
-    const int n_hg = (n_q_heads + kBalancedGroup - 1) / kBalancedGroup, hg = h / kBalancedGroup;
+    const int n_hg = (n_q_heads + where.group - 1) / where.group, hg = h / where.group;
     const int before = where.prefix[b], tiles_b = where.prefix[b + 1] - before;
     const int64_t total = (int64_t)where.prefix[gridDim.y] * n_hg;
     const int shares = where.prefix[gridDim.y + 1];
     const int64_t first = (int64_t)before * n_hg + (int64_t)hg * tiles_b;
     const int c0 = share_owner(first, total, shares), c1 = share_owner(first + tiles_b - 1, total, shares);
     ns = c1 - c0 + 1;
-    slot0 = ((int64_t)b * n_hg + hg + c0) * kBalancedGroup + h % kBalancedGroup;
-    step = kBalancedGroup;
+    slot0 = ((int64_t)b * n_hg + hg + c0) * where.group + h % where.group;
+    step = where.group;
   }
   __shared__ float row[128];
 

@@ -63,11 +63,12 @@ __host__ __device__ __forceinline__ int share_owner(int64_t tile, int64_t total,
   const int64_t x = (tile + 1) * n_ctas - 1;
   return (x >> 32) == 0 && (total >> 32) == 0 ? (int)((uint32_t)x / (uint32_t)total) : (int)(x / total);
 }
-constexpr int kBalancedGroup = 4;  // query heads per work item of the tensor-core kernel
+constexpr int kBalancedGroup = 4;     // query heads per work item of the tensor-core kernel, int8 latents
+constexpr int kBalancedGroupF16 = 2;  // the same, f16 latents
 constexpr int kMaxBalancedCtas = 256;
 
 // Where the merge finds the partials.  Split mode (prefix null): [B, Hq, n_splits] slots, the first
-// ceil(len / split_len) of a row used.  Balanced mode: slot (b * n_hg + hg + c) * 4 + h % 4 for every
+// ceil(len / split_len) of a row used.  Balanced mode: slot (b * n_hg + hg + c) * group + h % group for every
 // CTA c whose share holds tiles of (sequence b, head group hg); prefix[b] = tiles in sequences before
 // b, prefix[batch + 1] = number of shares (both written by stage 1).
 struct PartialIndex {
@@ -75,6 +76,7 @@ struct PartialIndex {
   int32_t n_ctas;         // CTAs of the stage-1 grid (>= the number of shares)
   int32_t n_splits;
   int32_t split_len;
+  int32_t group;          // balanced mode: query heads per work item
 };
 
 // Shared by the entry points that live outside capi.cu: the argument checks of

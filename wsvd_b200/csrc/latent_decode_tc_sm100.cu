@@ -77,36 +77,44 @@ constexpr int kRkMax = 64;
 constexpr uint32_t kAHalfBytes = kTile * 128;       // 128 rows x 64 f16
 constexpr uint32_t kABufBytes = 2 * kAHalfBytes;    // cos half + sin half
 constexpr uint32_t kTmemCols = 512;
-constexpr float kPlaneScale = 4294967040.f;         // 2^32 - 256: a weight of 1 is 0xFFFFFF00
 constexpr float kNone = -3.0e38f;                   // log2-domain reference of something that is still empty
 
-// Shape of the CTA.
+// Shape of the CTA, for int8 latents (four heads) and f16 latents (two heads, whose rows take twice the room).
+template <bool F16>
 struct Cfg {
-  static constexpr int kG = 4;                     // heads per CTA
+  static constexpr bool kF16 = F16;
+  static constexpr int kG = F16 ? 2 : 4;           // heads per CTA
   static constexpr int kEpiWarps = 4 * kG;
   static constexpr int kMmaWarp = kEpiWarps;       // score MMAs
   static constexpr int kLoadWarp = kEpiWarps + 1;  // copies
   static constexpr int kValWarp = kEpiWarps + 2;   // value MMAs: one warp per pair of heads
   static constexpr int kThreads = (kEpiWarps + 2 + kG / 2) * 32;
-  static constexpr int kRowBytes = 64;             // a latent row in shared memory (rank < 64: zero-filled)
-  static constexpr int kKSlots = 1;  // tiles of K: a tile's rows are copied to registers at the top of the tile
+  static constexpr int kRowBytes = F16 ? 128 : 64; // a latent row in shared memory (rank < 64: zero-filled)
+  static constexpr int kKSlots = F16 ? 2 : 1;      // tiles of K: a tile's rows are copied to registers at the top of the tile
   static constexpr int kVSlots = 2;  // tiles of V: the tile whose value MMAs are pending, and the next tile in flight
-  static constexpr int kWBufs = 2;   // W accumulators of 128 columns (one pair of heads each)
-  // Registers per thread after the two groups have re-balanced them.  The pool is the CTA's own: what
-  // the control warpgroup hands back, (96 - 64) * 128, is exactly what the epilogue warpgroups take,
-  // (104 - 96) * 512.  (A request the pool cannot satisfy would block for ever.)
-  static constexpr int kLaunchRegs = 96;  // what 640 threads per CTA leave the compiler
+  static constexpr int kWBufs = F16 ? 3 : 2;       // W accumulators of 128 columns (one pair of heads each)
+  // int8: 640 threads leave the compiler 96 registers a thread, and the two groups of warps re-balance them.
+  // The pool is the CTA's own: what the control warpgroup hands back, (96 - 64) * 128, is exactly what the
+  // epilogue warpgroups take, (104 - 96) * 512.  (A request the pool cannot satisfy would block for ever.)
+  // f16: 352 threads have 184 each, nothing to re-balance.
+  static constexpr int kLaunchRegs = 96;
   static constexpr int kEpiRegs = 104;
   static constexpr int kCtlRegs = 64;
-  static_assert((kLaunchRegs - kCtlRegs) * 4 * 32 >= (kEpiRegs - kLaunchRegs) * kEpiWarps * 32, "register pool");
-  static_assert(kThreads == (kEpiWarps + 4) * 32, "the control warps must form one warpgroup (4 warps) for setmaxnreg");
+  static_assert(F16 || (kLaunchRegs - kCtlRegs) * 4 * 32 >= (kEpiRegs - kLaunchRegs) * kEpiWarps * 32, "register pool");
+  static_assert(F16 || kThreads == (kEpiWarps + 4) * 32, "the control warps must form one warpgroup (4 warps) for setmaxnreg");
 
   static constexpr uint32_t kHeadBytes = kTile * kRowBytes;  // one head's part of a ring slot
   static constexpr uint32_t kUnitBytes = kG * kHeadBytes;    // a ring slot: one tile of K or V for the group's KV heads
   static constexpr uint32_t kBHalfBytes = kG * kRkMax * 128; // rows of 64 f16
-  static constexpr uint32_t kPlaneBytes = 256;               // per pair of warps: 2 chunks of 16 tokens x 8 rows x 16 bytes
+  static constexpr uint32_t kPlaneBytes = F16 ? 512 : 256;   // per pair of warps: 32 tokens x 8 rows of digits
   static constexpr uint32_t kTmemD = kWBufs * 128;           // first column of the value accumulators: 2 x 8 per (head, warp)
   static_assert(kTmemD + kG * 64 <= kTmemCols, "tensor memory");
+  // Weights of the value MMA, relative to the warp's reference 2^my_ref.  int8 V: integers in four digits of 8
+  // bits, a weight of 1 is 2^32 - 256.  f16 V: three f16 terms, each 2^11 below the one before, a weight of 1 is 2^15.
+  static constexpr float kPlaneScale = F16 ? 32768.f : 4294967040.f;
+  // Tiles after which a warp goes over to its other accumulator in any case.  int8: 32 tokens add at most 2^20 to a
+  // digit sum of 31 bits.  f16: so that a sum in tensor memory is never more than 32 additions long.
+  static constexpr int kRenewTiles = F16 ? 16 : 1024;
 
   // shared-memory map (offsets from a 1024-byte aligned base)
   static constexpr uint32_t kOffB = 0;
@@ -137,8 +145,14 @@ struct Cfg {
   static constexpr uint32_t kSmemBytes = kOffTmemSlot + 16;  // the dynamic shared-memory base is 1024-byte aligned
   static_assert(kOffA % 1024 == 0 && kOffV % 1024 == 0 && kOffPlanes % 256 == 0 && kOffBar % 8 == 0, "alignment");
   static_assert(kSmemBytes <= 232448, "shared memory budget");
+
+  // Byte offset, inside one head's part of a ring slot, of 16-byte chunk c of token tok (0..127): rows of 64 bytes
+  // with the 64-byte swizzle, or of 128 bytes with the 128-byte swizzle.
+  static __device__ __forceinline__ uint32_t row_off(int tok, int c) {
+    return F16 ? (uint32_t)(tok * 128 + ((c ^ (tok & 7)) << 4)) : (uint32_t)(tok * 64 + ((c ^ ((tok >> 1) & 3)) << 4));
+  }
 };
-static_assert(Cfg::kG == kBalancedGroup, "the merge kernel indexes balanced partials by groups of kG heads");
+static_assert(Cfg<false>::kG == kBalancedGroup && Cfg<true>::kG == kBalancedGroupF16, "the merge kernel indexes balanced partials by groups of kG heads");
 
 enum Status : unsigned int { kOk = 0, kTimeoutProducer = 1, kTimeoutMma = 2, kTimeoutEpilogue = 3, kBadSmemAlignment = 4 };
 
@@ -302,12 +316,6 @@ __device__ __forceinline__ void cvt4(uint32_t w, float2& lo, float2& hi) {
   hi = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(w, magic, 0x7652)), __uint_as_float(__byte_perm(w, magic, 0x7653))), bias);
 }
 
-// Byte offset, inside one head's part of a ring slot, of 16-byte chunk c of token tok (0..127):
-// rows of 64 bytes with the 64-byte swizzle (chunk index XOR (tok/2)%4).
-__device__ __forceinline__ uint32_t latent_off(int tok, int c) {
-  return (uint32_t)(tok * 64 + ((c ^ ((tok >> 1) & 3)) << 4));
-}
-
 // UMMA shared-memory descriptors (sm_100 descriptor version 1).
 // K-major operand, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
@@ -327,6 +335,16 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw64(uint32_t addr) {
   d |= (uint64_t)(512 >> 4) << 32;              // stride byte offset between groups of 8 K indices
   d |= (uint64_t)1 << 46;
   d |= (uint64_t)4 << 61;                       // SWIZZLE_64B
+  return d;
+}
+// MN-major operand, 128-byte swizzle: 128 bytes along M per K index, 8 K indices per 1024 bytes.
+__device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((addr >> 4) & 0x3FFF);
+  d |= (uint64_t)1 << 16;                       // leading byte offset (one 128-byte atom along M: unused)
+  d |= (uint64_t)(1024 >> 4) << 32;             // stride byte offset between groups of 8 K indices
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;                       // SWIZZLE_128B
   return d;
 }
 // K-major operand without swizzle, 8 rows: 16-byte K chunks 128 bytes apart, rows 16 bytes apart.
@@ -442,8 +460,8 @@ struct Walk {
 };
 
 // ------------------------------------------------------------------ score MMAs (one warp)
+template <class C>
 __device__ __forceinline__ void score_role(const TcArgs& ta, const Share& sh, uint32_t sbase, uint32_t tmem) {
-  using C = Cfg;
   const WsvdLatentDecodeParams& p = ta.k.p;
   const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG;
   auto bar = [&](int i) { return sbase + C::kOffBar + 8u * i; };
@@ -498,8 +516,8 @@ __device__ __forceinline__ void score_role(const TcArgs& ta, const Share& sh, ui
 //  - every aligned group of 16 tokens is a run (pages of 16, 32, 64 slots): lane l copies run l / 4 of KV
 //    head l % 4, 1 KB a copy;
 //  - else the epilogue's threads fetch their own tokens' rows (kTileGather), and this warp asks L2 for them.
+template <class C>
 __device__ __forceinline__ void copy_role(const TcArgs& ta, const Share& sh, uint32_t sbase, uint8_t* sm) {
-  using C = Cfg;
   const WsvdLatentDecodeParams& p = ta.k.p;
   const int lane = threadIdx.x & 31;
   const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG, gqa = p.n_q_heads / p.n_kv_heads;
@@ -601,8 +619,9 @@ __device__ __forceinline__ void copy_role(const TcArgs& ta, const Share& sh, uin
 // ------------------------------------------------------------------ value MMAs (one warp per pair of heads)
 // One byte per warp of head g: bit 0 which of its two value accumulators this tile's sums go to, bit 1 whether
 // they are added to it.  (It sits in the unused last word of the head's first ItemState.)
+template <class C>
 __device__ __forceinline__ volatile uint32_t* value_modes(uint8_t* sm, int g) {
-  return reinterpret_cast<volatile uint32_t*>(sm + Cfg::kOffItem + g * 128 + 60);
+  return reinterpret_cast<volatile uint32_t*>(sm + C::kOffItem + g * 128 + 60);
 }
 
 // The warp serves its two heads in turn: it waits for the digit planes of a head's four warps and issues the
@@ -610,15 +629,15 @@ __device__ __forceinline__ volatile uint32_t* value_modes(uint8_t* sm, int g) {
 // then tell the epilogue warps (D full) and the copying warp (V empty) when the MMAs have completed.  All lanes
 // hold the same operands and flags: the instruction takes them from uniform registers, and when two lanes
 // served a head each, one head's sums were now and then added to, or not, as the other's should have been.
+template <class C>
 __device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, uint32_t sbase, uint8_t* sm,
                                            uint32_t tmem, int pair) {
-  using C = Cfg;
   const WsvdLatentDecodeParams& p = ta.k.p;
   const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG, gqa = p.n_q_heads / p.n_kv_heads;
   auto bar = [&](int i) { return sbase + C::kOffBar + 8u * i; };
-  const uint32_t idesc = instr_desc_i8(64, 8);
+  const uint32_t idesc = C::kF16 ? instr_desc_f16(64, 8) | (1u << 15) : instr_desc_i8(64, 8);
   const volatile int* mode = reinterpret_cast<const volatile int*>(sm + C::kOffMode);
-  const uint64_t vdesc0 = smem_desc_mn_sw64(sbase + C::kOffV), pdesc0 = smem_desc_k_plain(sbase + C::kOffPlanes);
+  const uint64_t vdesc0 = C::kF16 ? smem_desc_mn_sw128(sbase + C::kOffV) : smem_desc_mn_sw64(sbase + C::kOffV), pdesc0 = smem_desc_k_plain(sbase + C::kOffPlanes);
   const uint32_t v_lo = (uint32_t)vdesc0, v_hi = (uint32_t)(vdesc0 >> 32), p_lo = (uint32_t)pdesc0, p_hi = (uint32_t)(pdesc0 >> 32);
   const bool issuer = elect_one();
   Walk w;
@@ -643,16 +662,23 @@ __device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, ui
         if (!ok) break;
         ++mine[j];
         tc_fence_after();
-        const uint32_t how = *value_modes(sm, g);  // a byte per warp: which of its accumulators, added to or started
+        const uint32_t how = *value_modes<C>(sm, g);  // a byte per warp: which of its accumulators, added to or started
         // copied rows sit at the head's KV head, gathered ones at the head itself
         const int sub = mode[T & 3] == kTileGather ? g : (h0 + g) / gqa - h0 / gqa;
         const uint32_t v_at = v_lo + ((vslot * C::kUnitBytes + sub * C::kHeadBytes) >> 4);
         const uint32_t d_tmem = tmem + C::kTmemD + 64 * g;
         if (issuer) {
 #pragma unroll
-          for (int w4 = 0; w4 < 4; ++w4)  // the 32 tokens of warp w4: 32 rows of 64 bytes
-            umma_i8(d_tmem + 16 * w4 + ((how >> (8 * w4)) & 1) * 8, join64(v_at + ((w4 * 2048) >> 4), v_hi),
-                    join64(p_lo + (((2 * g + (w4 >> 1)) * C::kPlaneBytes) >> 4), p_hi), idesc, (how >> (8 * w4)) & 2);
+          for (int w4 = 0; w4 < 4; ++w4) {  // the 32 tokens of warp w4: 32 rows
+            const uint32_t d = d_tmem + 16 * w4 + ((how >> (8 * w4)) & 1) * 8, adds = (how >> (8 * w4)) & 2;
+            const uint32_t va = v_at + ((w4 * 32 * C::kRowBytes) >> 4), pa = p_lo + (((2 * g + (w4 >> 1)) * C::kPlaneBytes) >> 4);
+            if constexpr (C::kF16) {  // 16 tokens an instruction
+              umma_f16(d, join64(va, v_hi), join64(pa, p_hi), idesc, adds);
+              umma_f16(d, join64(va + (2048 >> 4), v_hi), join64(pa + (256 >> 4), p_hi), idesc, 1);
+            } else {
+              umma_i8(d, join64(va, v_hi), join64(pa, p_hi), idesc, adds);
+            }
+          }
           umma_commit(bar(C::kBarDFull + g));
           umma_commit(bar(C::kBarVEmpty + vslot));
           if (g == 0 && G < C::kG) mbar_arrive_n(bar(C::kBarVEmpty + vslot), C::kG - G);  // for the heads that are not there
@@ -674,8 +700,8 @@ __device__ __forceinline__ uint32_t pq_off(int g, int r, int ic) {
 // Asks for what the [P;Q] build of an item needs from memory: the head's slice of wk goes, without passing
 // through registers, to the places in the B operand that the thread which asked for it will overwrite with P
 // and Q; the page entries of the first two tiles go to L1.
+template <class C>
 __device__ __forceinline__ void request_pq(const TcArgs& ta, uint32_t sbase, const Walk& w, int g, bool wk_vec) {
-  using C = Cfg;
   const WsvdLatentDecodeParams& p = ta.k.p;
   const int gqa = p.n_q_heads / p.n_kv_heads, hk = (w.hg * C::kG + g) / gqa;
   const bool il = p.rope_layout == WSVD_ROPE_INTERLEAVED, wk_i8 = p.wk_dtype == WSVD_I8;
@@ -707,8 +733,8 @@ __device__ __forceinline__ void request_pq(const TcArgs& ta, uint32_t sbase, con
 
 // B operand: P (cos coefficients) and Q (sin coefficients) of head g of the group, f16, rows n = g*64 + r, 64
 // frequencies per row, 128-byte swizzle; rows r >= rank_k are zero.
+template <class C>
 __device__ __forceinline__ void build_pq(const TcArgs& ta, uint8_t* sm, int b, int h, int hk, int g, bool wk_vec) {
-  using C = Cfg;
   const KArgs& a = ta.k;
   const WsvdLatentDecodeParams& p = a.p;
   const bool interleaved = p.rope_layout == WSVD_ROPE_INTERLEAVED, wk_i8 = p.wk_dtype == WSVD_I8;
@@ -741,8 +767,8 @@ __device__ __forceinline__ void build_pq(const TcArgs& ta, uint8_t* sm, int b, i
     }
   }
   const int64_t col = (int64_t)hk * 128;
-  if (wk_vec && !wk_i8 && !interleaved) {
-    // Common case (f16 wk, half-split pairing): packed f16 arithmetic.  The operands are
+  if (!C::kF16 && wk_vec && !wk_i8 && !interleaved) {
+    // Common case (int8 latents, f16 wk, half-split pairing): packed f16 arithmetic.  The operands are
     // rounded to f16 for the MMA anyway; forming them with one extra f16 rounding of a
     // product keeps the error of the scores within a few 1e-5.  This thread's chunk of 8
     // frequencies is the same for its four ranks, so q is converted once.
@@ -902,8 +928,8 @@ __device__ __forceinline__ Walk get_item(const volatile int* st) {
 // Merges, projects and writes the output rows of a head whose last partial this CTA has delivered (or that it
 // covered alone: the latent-space row is in shared memory then).  Run by the head's 128 threads.
 // `seen`: for thread 0 of the head, the arrivals before this CTA's.
+template <class C>
 __device__ __forceinline__ void finish_head(const TcArgs& ta, uint8_t* sm, int g, const volatile int* st, unsigned int seen) {
-  using C = Cfg;
   const KArgs& a = ta.k;
   const WsvdLatentDecodeParams& p = a.p;
   const int d = threadIdx.x & 127, Rv = p.rank_v;
@@ -979,8 +1005,9 @@ __device__ __forceinline__ void finish_head(const TcArgs& ta, uint8_t* sm, int g
   }
 }
 
+template <class C>
 __device__ __forceinline__ volatile int* item_state(uint8_t* sm, int g, uint32_t item) {
-  return reinterpret_cast<volatile int*>(sm + Cfg::kOffItem) + (g * 2 + (item & 1)) * 16;
+  return reinterpret_cast<volatile int*>(sm + C::kOffItem) + (g * 2 + (item & 1)) * 16;
 }
 
 // One head's running sums over the tiles of an item, all in the log2 domain and fp32.
@@ -993,7 +1020,7 @@ __device__ __forceinline__ volatile int* item_state(uint8_t* sm, int g, uint32_t
 //    eighth of the kernel's instructions.
 struct HeadSums {
   float m_run, l_lane;
-  float my_ref, scale;  // scale: 2^(m_run - my_ref) * kPlaneScale
+  float my_ref, scale;  // scale: 2^(m_run - my_ref) * kPlaneScale of the Cfg
   float big_m, acc;
   uint32_t bufs;        // bit w4: the accumulator warp w4 of the head is using
 };
@@ -1001,17 +1028,25 @@ constexpr float kSlackZ = 8.f;
 constexpr int kSlackY = 3;
 
 // Fold in one accumulator of warp w4 of the head: D[rank][0..3] are its four digit-plane sums, relative to 2^ref.
+template <class C>
 __device__ __forceinline__ void fold_values(HeadSums& hs, uint32_t d_addr, int w4, uint32_t buf, float ref) {
   uint32_t d[4];
   tmem_ld4(d_addr + 16 * w4 + 8 * buf + 4 * (w4 & 1), d);
   tmem_wait_ld(d);
   const float m_new = fmaxf(hs.big_m, ref);
-  const float v = fmaf((float)(int32_t)d[3], 16777216.f, fmaf((float)(int32_t)d[2], 65536.f, fmaf((float)(int32_t)d[1], 256.f, (float)(int32_t)d[0])));
-  hs.acc = fmaf(v, fast_exp2(ref - m_new) * (1.f / kPlaneScale), hs.acc * fast_exp2(hs.big_m - m_new));
+  float v;
+  if constexpr (C::kF16) {
+    v = fmaf(__uint_as_float(d[2]), 2.384185791015625e-7f, fmaf(__uint_as_float(d[1]), 4.8828125e-4f, __uint_as_float(d[0])));  // 2^-22, 2^-11
+    if (isinf(__uint_as_float(d[0]))) v = __uint_as_float(d[0]);  // an infinite V times a lower term of zero is no NaN
+  } else {
+    v = fmaf((float)(int32_t)d[3], 16777216.f, fmaf((float)(int32_t)d[2], 65536.f, fmaf((float)(int32_t)d[1], 256.f, (float)(int32_t)d[0])));
+  }
+  hs.acc = fmaf(v, fast_exp2(ref - m_new) * (1.f / C::kPlaneScale), hs.acc * fast_exp2(hs.big_m - m_new));
   hs.big_m = m_new;
 }
 
 // What the head's warps have left behind with tile number tp (see HeadSums).
+template <class C>
 __device__ __forceinline__ void fold_left(HeadSums& hs, uint32_t d_addr, const float* refs, uint32_t tp) {
   const float4 rf = *reinterpret_cast<const float4*>(refs + (tp & 1) * 4);
   if (fmaxf(fmaxf(rf.x, rf.y), fmaxf(rf.z, rf.w)) > kNone) {
@@ -1021,7 +1056,7 @@ __device__ __forceinline__ void fold_left(HeadSums& hs, uint32_t d_addr, const f
     for (int w4 = 0; w4 < 4; ++w4) {
       const float r = w4 == 0 ? ref[0] : w4 == 1 ? ref[1] : w4 == 2 ? ref[2] : ref[3];
       if (r > kNone) {
-        fold_values(hs, d_addr, w4, (hs.bufs >> w4) & 1, r);
+        fold_values<C>(hs, d_addr, w4, (hs.bufs >> w4) & 1, r);
         hs.bufs ^= 1u << w4;
       }
     }
@@ -1029,22 +1064,23 @@ __device__ __forceinline__ void fold_left(HeadSums& hs, uint32_t d_addr, const f
 }
 
 // The tiles of an item, for one warp of a head that is there.
+template <class C>
 __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_t item, HeadSums& hs) {
-  using C = Cfg;
   const WsvdLatentDecodeParams& p = ta.k.p;
   const int tid = fresh_tid(), lane = tid & 31, g = tid >> 7, row = tid & 127, q4 = row >> 5;
   const uint32_t sbase = smem_u32(sm);
   auto bar = [&](int i) { return sbase + C::kOffBar + 8u * i; };
   const int gqa = p.n_q_heads / p.n_kv_heads, Rv = p.rank_v;
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + C::kOffTmemSlot);
-  const volatile int* st = item_state(sm, g, item);
+  const volatile int* st = item_state<C>(sm, g, item);
   const volatile int* mode = reinterpret_cast<const volatile int*>(sm + C::kOffMode);
   float* refs = reinterpret_cast<float*>(sm + C::kOffRef) + g * 8;  // [tile parity][warp]: reference left behind, or kNone
   // Digit planes: the two warps of half a tile share one 8-row block (the MMA's B operand has 8
   // rows): rows 0..3 hold the even warp's digits, rows 4..7 the odd warp's.  Each warp's MMA reads
   // the whole block, so its columns 4..7 (or 0..3) are the other warp's weights times this warp's
   // V rows: garbage that nobody reads.
-  const uint32_t my_planes = sbase + C::kOffPlanes + (2 * g + (q4 >> 1)) * C::kPlaneBytes + (lane >> 4) * 128 + (q4 & 1) * 64 + (lane & 15);
+  const uint32_t my_planes = sbase + C::kOffPlanes + (2 * g + (q4 >> 1)) * C::kPlaneBytes + (q4 & 1) * 64 +
+                             (C::kF16 ? (lane >> 3) * 128 + (lane & 7) * 2 : (lane >> 4) * 128 + (lane & 15));
   const uint32_t d_addr = tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 64 * g;
   const int h0 = st[kItHg] * C::kG, G = min(C::kG, p.n_q_heads - h0), npairs = (G + 1) >> 1;
   bool ok = true;
@@ -1052,7 +1088,8 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
   const int hk = (h0 + g) / gqa;
   const int pr = g >> 1, sub = hk - h0 / gqa;  // sub: this head's KV head inside a unit
   const int lo = st[kItLo], hi = st[kItHi], ntiles = st[kItTiles];
-  int slot_c, slot_n;
+  constexpr int kChunks = C::kRowBytes / 16;  // 16-byte chunks of a latent row
+  int slot_c = -1, slot_n = -1;
   unsigned short sk_raw = 0, sv_raw = 0;
   const uint32_t T = st[kItT], ub = st[kItUnits], mine = st[kItMine];
   const int32_t* page = p.req_to_token + (int64_t)st[kItReq] * p.rtt_stride;
@@ -1062,12 +1099,14 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
   // ones, and a pair that holds a single head arrives twice
   const uint32_t k_arrivals = g == 0 ? 1u + (C::kG - G) : 1u;
   const uint32_t w_arrivals = (G - 2 * pr) >= 2 ? 1u : 2u;
-  // this lane's first token and its next one (the lines were asked for with the item's other loads)
-  slot_c = lo + row < hi ? page[lo + row] : -1;
-  slot_n = lo + kTile + row < hi ? page[lo + kTile + row] : -1;
-  if (slot_c >= 0) {
-    sk_raw = reinterpret_cast<const unsigned short*>(ksc)[(int64_t)slot_c * p.ks_stride_t];
-    sv_raw = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_c * p.vs_stride_t];
+  if constexpr (!C::kF16) {
+    // this lane's first token and its next one (the lines were asked for with the item's other loads)
+    slot_c = lo + row < hi ? page[lo + row] : -1;
+    slot_n = lo + kTile + row < hi ? page[lo + kTile + row] : -1;
+    if (slot_c >= 0) {
+      sk_raw = reinterpret_cast<const unsigned short*>(ksc)[(int64_t)slot_c * p.ks_stride_t];
+      sv_raw = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_c * p.vs_stride_t];
+    }
   }
   for (int t = 0; t < ntiles && ok; ++t) {
     const int s = lo + t * kTile + row;
@@ -1080,13 +1119,15 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       sk_n = reinterpret_cast<const unsigned short*>(ksc)[(int64_t)slot_n * p.ks_stride_t];
       sv_n = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_n * p.vs_stride_t];
     }
-    const int slot_t = slot_c;
-    slot_c = slot_n;
-    slot_n = -1;
-    if (s + 2 * kTile < hi) slot_n = page[s + 2 * kTile];
+    int slot_t = slot_c;
+    if constexpr (!C::kF16) {
+      slot_c = slot_n;
+      slot_n = -1;
+      if (s + 2 * kTile < hi) slot_n = page[s + 2 * kTile];
+    }
     // ---- this warp's 32 K rows (lane = token) go from the ring slot to registers at once and
     //      the slot is handed back: its refill has the whole tile to arrive
-    uint4 kreg[4];
+    uint4 kreg[kChunks];
     const uint32_t kslot = Tt % C::kKSlots;
     ok = mbar_wait(bar(C::kBarKFull + kslot), (Tt / C::kKSlots) & 1);
     if (!ok) break;
@@ -1094,16 +1135,18 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     if (!gather) {
       const uint32_t krows = sbase + C::kOffK + kslot * C::kUnitBytes + sub * C::kHeadBytes;
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
+      for (int c = 0; c < kChunks; ++c)
         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                      : "=r"(kreg[c].x), "=r"(kreg[c].y), "=r"(kreg[c].z), "=r"(kreg[c].w)
-                     : "r"(krows + latent_off(row, c)));
+                     : "r"(krows + C::row_off(row, c)));
     } else {
-      const uint8_t* src = reinterpret_cast<const uint8_t*>(p.latent_k) + (int64_t)slot_t * p.k_stride_t + (int64_t)hk * p.k_stride_h;
+      if constexpr (C::kF16) slot_t = valid ? page[s] : -1;
+      const uint8_t* src = reinterpret_cast<const uint8_t*>(p.latent_k) +
+                           (C::kRowBytes / 64) * ((int64_t)slot_t * p.k_stride_t + (int64_t)hk * p.k_stride_h);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < kChunks; ++c) {
         kreg[c] = make_uint4(0u, 0u, 0u, 0u);
-        if (valid && c * 16 < p.rank_k) kreg[c] = __ldg(reinterpret_cast<const uint4*>(src) + c);
+        if (valid && c * 16 < p.rank_k * (C::kRowBytes / 64)) kreg[c] = __ldg(reinterpret_cast<const uint4*>(src) + c);
       }
     }
     __syncwarp();
@@ -1112,17 +1155,24 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     if (!ok) break;
     tc_fence_after();
 
-    // ---- score: dot of this token's int8 K row with its row of W, 16 ranks at a time
+    // ---- score: dot of this token's K row with its row of W, 16 ranks at a time
     const uint32_t taddr = tmem + ((uint32_t)(q4 * 32) << 16) + wb * 128 + (g & 1) * kRkMax;
     float2 dot0 = make_float2(0.f, 0.f), dot1 = make_float2(0.f, 0.f);
     // two 16-column loads in flight alternately: the next chunk of W travels while this one is used
     uint32_t wa[16], wb16[16];
-    auto mac16 = [&](const uint32_t (&wv)[16], const uint4 kq) {
-      const uint32_t kws[4] = {kq.x ^ 0x80808080u, kq.y ^ 0x80808080u, kq.z ^ 0x80808080u, kq.w ^ 0x80808080u};
+    auto mac16 = [&](const uint32_t (&wv)[16], int c) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         float2 x01, x23;
-        cvt4(kws[j], x01, x23);
+        if constexpr (C::kF16) {
+          const uint4 kq = kreg[(2 * c + (j >> 1)) % kChunks];
+          const uint32_t h01 = j & 1 ? kq.z : kq.x, h23 = j & 1 ? kq.w : kq.y;
+          x01 = __half22float2(*reinterpret_cast<const __half2*>(&h01));
+          x23 = __half22float2(*reinterpret_cast<const __half2*>(&h23));
+        } else {
+          const uint4 kq = kreg[c % kChunks];
+          cvt4((j == 0 ? kq.x : j == 1 ? kq.y : j == 2 ? kq.z : kq.w) ^ 0x80808080u, x01, x23);
+        }
         dot0 = __ffma2_rn(x01, make_float2(__uint_as_float(wv[4 * j]), __uint_as_float(wv[4 * j + 1])), dot0);
         dot1 = __ffma2_rn(x23, make_float2(__uint_as_float(wv[4 * j + 2]), __uint_as_float(wv[4 * j + 3])), dot1);
       }
@@ -1130,31 +1180,32 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     tmem_ld16(taddr, wa);
     tmem_wait_ld();
     tmem_ld16(taddr + 16, wb16);
-    mac16(wa, kreg[0]);
+    mac16(wa, 0);
     tmem_wait_ld();
     tmem_ld16(taddr + 32, wa);
-    mac16(wb16, kreg[1]);
+    mac16(wb16, 1);
     tmem_wait_ld();
     tmem_ld16(taddr + 48, wb16);
-    mac16(wa, kreg[2]);
+    mac16(wa, 2);
     tmem_wait_ld();
-    mac16(wb16, kreg[3]);
+    mac16(wb16, 3);
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive_n(bar(C::kBarWEmpty + wb), w_arrivals);  // this warp has read its rows of W
     if (gather) {  // the V row of this token: requested now, stored once the slot is known to be free
 #pragma unroll
-      for (int c = 0; c < 4; ++c) kreg[c] = make_uint4(0u, 0u, 0u, 0u);
+      for (int c = 0; c < kChunks; ++c) kreg[c] = make_uint4(0u, 0u, 0u, 0u);
       if (valid) {
-        const uint8_t* src = reinterpret_cast<const uint8_t*>(p.latent_v) + (int64_t)slot_t * p.v_stride_t + (int64_t)hk * p.v_stride_h;
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(p.latent_v) +
+                             (C::kRowBytes / 64) * ((int64_t)slot_t * p.v_stride_t + (int64_t)hk * p.v_stride_h);
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (c * 16 < Rv) kreg[c] = __ldg(reinterpret_cast<const uint4*>(src) + c);
+        for (int c = 0; c < kChunks; ++c)
+          if (c * 16 < Rv * (C::kRowBytes / 64)) kreg[c] = __ldg(reinterpret_cast<const uint4*>(src) + c);
       }
     }
     const float2 dsum = __fadd2_rn(dot0, dot1);
     const float sk = __half2float(__ushort_as_half(sk_raw)), sv = __half2float(__ushort_as_half(sv_raw));
-    const float z = valid ? (dsum.x + dsum.y) * sk : -INFINITY;
+    const float z = valid ? (C::kF16 ? dsum.x + dsum.y : (dsum.x + dsum.y) * sk) : -INFINITY;
     sk_raw = sk_n;
     sv_raw = sv_n;
 
@@ -1167,12 +1218,11 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     }
     const float e = fast_exp2(z - hs.m_run);  // masked tokens: 2^-inf = 0
     hs.l_lane += e;
-    const float pv = e * sv, pv_w = warp_max_redux(pv);
-    // ---- does every weight fit under the reference of the value sums?  (The accumulators are integers of 32 bits
-    //      per digit: 32 tokens add at most 2^20, so 1024 tiles are well inside.)
+    const float pv = C::kF16 ? e : e * sv, pv_w = warp_max_redux(pv);
+    // ---- does every weight fit under the reference of the value sums?
     float left = kNone;
     uint32_t adds = t > 0 ? 2u : 0u;
-    renew = renew || pv_w * hs.scale > kPlaneScale || (t & 1023) == 1023;
+    renew = renew || pv_w * hs.scale > C::kPlaneScale || (t & (C::kRenewTiles - 1)) == C::kRenewTiles - 1;
     if (renew) {
       left = hs.my_ref;
       if (left > kNone) {
@@ -1184,7 +1234,7 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       const int k = min(max((int)((__float_as_uint(pv_w) >> 23) & 0xff) - 126 + kSlackY, -60), 100);
       if (pv_w == INFINITY) hs.l_lane = __int_as_float(0x7fc00000);  // an infinite V scale: the result is NaN
       hs.my_ref = hs.m_run + (float)k;
-      hs.scale = kPlaneScale * __uint_as_float((uint32_t)(127 - k) << 23);
+      hs.scale = C::kPlaneScale * __uint_as_float((uint32_t)(127 - k) << 23);
     }
 
     // ---- the previous tile's value MMAs are complete: fold in what the head's warps left behind with it.  This
@@ -1194,7 +1244,7 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       ok = mbar_wait(bar(C::kBarDFull + g), (mt - 1) & 1);
       if (!ok) break;
       tc_fence_after();
-      fold_left(hs, d_addr, refs, mt - 1);
+      fold_left<C>(hs, d_addr, refs, mt - 1);
     }
     if (gather) {
       // the copying warp's arrival says that every head's value MMAs on the slot are complete
@@ -1202,14 +1252,35 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       if (!ok) break;
       const uint32_t vrow = sbase + C::kOffV + (Tt % C::kVSlots) * C::kUnitBytes + g * C::kHeadBytes;
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(vrow + latent_off(row, c)), "r"(kreg[c].x),
+      for (int c = 0; c < kChunks; ++c)
+        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(vrow + C::row_off(row, c)), "r"(kreg[c].x),
                      "r"(kreg[c].y), "r"(kreg[c].z), "r"(kreg[c].w)
                      : "memory");
+    } else if (C::kF16 && lo + (t + 1) * kTile > hi) {
+      // the end of the sequence: what was copied behind it may be anything, and in f16 a NaN times a weight of
+      // zero is a NaN
+      ok = mbar_wait(bar(C::kBarVFull + Tt % C::kVSlots), (Tt / C::kVSlots) & 1);
+      if (!ok) break;
+      const uint32_t vrow = sbase + C::kOffV + (Tt % C::kVSlots) * C::kUnitBytes + sub * C::kHeadBytes;
+      if (!valid) {
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c)
+          asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(vrow + C::row_off(row, c)), "r"(0) : "memory");
+      }
     }
 
-    // ---- this token's weight for the value MMA, relative to the warp's reference, as four 8-bit digits
-    {
+    // ---- this token's weight for the value MMA, relative to the warp's reference: four 8-bit digits, or three f16
+    //      terms (11 bits each, every remainder is exact: nothing that fp32 holds of the weight is lost)
+    if constexpr (C::kF16) {
+      const float wgt = pv * hs.scale;
+      const __half t0 = __float2half_rn(wgt);
+      const float r1 = (wgt - __half2float(t0)) * 2048.f;
+      const __half t1 = __float2half_rn(r1);
+      const __half t2 = __float2half_rn((r1 - __half2float(t1)) * 2048.f);
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(my_planes), "h"(__half_as_ushort(t0)) : "memory");
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(my_planes + 16), "h"(__half_as_ushort(t1)) : "memory");
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(my_planes + 32), "h"(__half_as_ushort(t2)) : "memory");
+    } else {
       const uint32_t nq = __float2uint_rn(pv * hs.scale);
       asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes), "r"(nq) : "memory");
       asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 16), "r"(nq >> 8) : "memory");
@@ -1220,7 +1291,7 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     tc_fence_before();
     if (lane == 0) {
       refs[(mt & 1) * 4 + q4] = left;
-      reinterpret_cast<volatile uint8_t*>(value_modes(sm, g))[q4] = (uint8_t)(own_buf | adds);
+      reinterpret_cast<volatile uint8_t*>(value_modes<C>(sm, g))[q4] = (uint8_t)(own_buf | adds);
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(C::kBarPlanes + g));
@@ -1228,8 +1299,8 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
   return ok;
 }
 
+template <class C>
 __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh, uint8_t* sm, uint32_t sbase, uint32_t tmem) {
-  using C = Cfg;
   const KArgs& a = ta.k;
   const WsvdLatentDecodeParams& p = a.p;
   const int n_hg = (p.n_q_heads + C::kG - 1) / C::kG, gqa = p.n_q_heads / p.n_kv_heads;
@@ -1245,14 +1316,14 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
   const bool wk_vec = (p.wk_stride_r & 7) == 0 &&
                       (wk_i8 ? (reinterpret_cast<uintptr_t>(p.wk) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.wk_scale) & 15) == 0
                              : (reinterpret_cast<uintptr_t>(p.wk) & 15) == 0);
-  auto state = [&](uint32_t i) { return item_state(sm, g, i); };
+  auto state = [&](uint32_t i) { return item_state<C>(sm, g, i); };
   bool ok = true;  // after a wait that timed out: tiles are skipped, results are NaN
   bool pending = false;  // the item before is still to be finished
   unsigned int seen = 0;
   {
     Walk w;
     if (!w.start(ta, sh, n_hg)) return;
-    if (g < p.n_q_heads - w.hg * C::kG) request_pq(ta, sbase, w, g, wk_vec);
+    if (g < p.n_q_heads - w.hg * C::kG) request_pq<C>(ta, sbase, w, g, wk_vec);
     put_item(state(0), w, 0, 0, 0);
   }
   for (uint32_t item = 0;; ++item) {
@@ -1263,18 +1334,18 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
       const int hk = (h0 + g) / gqa;
       // The rows of this head in the B operand are free: this warp has seen W of the head's last tile, and
       // with it the completion of every score MMA that read them.
-      build_pq(ta, sm, st[kItB], h0 + g, hk, g, wk_vec);
+      build_pq<C>(ta, sm, st[kItB], h0 + g, hk, g, wk_vec);
       fence_proxy_async();
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(C::kBarPq));
     // a warp whose head is not there must not arrive for the next item before this one's phase is over
     if (!active && ok) ok = warp_wait(bar(C::kBarPq), item & 1);
-    if (pending) finish_head(ta, sm, g, state(item + 1), seen);  // the item before, while the first score MMAs of this one run
+    if (pending) finish_head<C>(ta, sm, g, state(item + 1), seen);  // the item before, while the first score MMAs of this one run
     pending = false;
 
     HeadSums hs = {kNone, 0.f, kNone, 0.f, kNone, 0.f, 0u};
-    if (active && ok) ok = run_tiles(ta, sm, item, hs);
+    if (active && ok) ok = run_tiles<C>(ta, sm, item, hs);
 
     // ---- the item's end.  What the next item needs is requested before the last value sums are waited for.
     bool more;
@@ -1291,7 +1362,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
       }
       more = w.next(p, n_hg);
       if (more) {
-        if (g < p.n_q_heads - w.hg * C::kG) request_pq(ta, sbase, w, g, wk_vec);
+        if (g < p.n_q_heads - w.hg * C::kG) request_pq<C>(ta, sbase, w, g, wk_vec);
         put_item(state(item + 1), w, T, units, mine);
       }
     }
@@ -1304,7 +1375,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
         ok = warp_wait(bar(C::kBarDFull + g), last & 1);
         if (ok) {
           tc_fence_after();
-          fold_left(hs, d_addr, refs, last);
+          fold_left<C>(hs, d_addr, refs, last);
         }
       }
       if (!ok) atomicMax(&g_status, (unsigned)kTimeoutEpilogue);
@@ -1320,10 +1391,10 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
       head_sync();
       if (ok) {
         const float4 rf = *reinterpret_cast<const float4*>(refs + ((last + 1) & 1) * 4);
-        if (rf.x > kNone) fold_values(hs, d_addr, 0, hs.bufs & 1, rf.x);
-        if (rf.y > kNone) fold_values(hs, d_addr, 1, (hs.bufs >> 1) & 1, rf.y);
-        if (rf.z > kNone) fold_values(hs, d_addr, 2, (hs.bufs >> 2) & 1, rf.z);
-        if (rf.w > kNone) fold_values(hs, d_addr, 3, (hs.bufs >> 3) & 1, rf.w);
+        if (rf.x > kNone) fold_values<C>(hs, d_addr, 0, hs.bufs & 1, rf.x);
+        if (rf.y > kNone) fold_values<C>(hs, d_addr, 1, (hs.bufs >> 1) & 1, rf.y);
+        if (rf.z > kNone) fold_values<C>(hs, d_addr, 2, (hs.bufs >> 2) & 1, rf.z);
+        if (rf.w > kNone) fold_values<C>(hs, d_addr, 3, (hs.bufs >> 3) & 1, rf.w);
         tc_fence_before();
       }
       float m_all = kNone;
@@ -1357,15 +1428,15 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
       }
     }
     if (!more) {
-      if (pending) finish_head(ta, sm, g, st, seen);
+      if (pending) finish_head<C>(ta, sm, g, st, seen);
       break;
     }
   }
 }
 
 // ------------------------------------------------------------------ the kernel
-__global__ void __launch_bounds__(Cfg::kThreads, 1) stage1_tc_kernel(const __grid_constant__ TcArgs ta) {
-  using C = Cfg;
+template <class C>
+__global__ void __launch_bounds__(C::kThreads, 1) stage1_tc_kernel(const __grid_constant__ TcArgs ta) {
   const KArgs& a = ta.k;
   const WsvdLatentDecodeParams& p = a.p;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1497,17 +1568,17 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) stage1_tc_kernel(const __gri
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  // ---- register budgets.  The launch gives every thread 96 registers (640 threads); the tile loop of
+  // ---- register budgets.  With int8 latents the launch gives every thread 96 registers (640 threads); the tile loop of
   //      the epilogue needs more and the control warps far fewer, so the control warpgroup hands
   //      registers back to the pool and the four epilogue warpgroups take them.
   if (warp < C::kEpiWarps) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kEpiRegs));
-    epilogue_role(ta, sh, sm, sbase, tmem);
+    if constexpr (!C::kF16) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kEpiRegs));
+    epilogue_role<C>(ta, sh, sm, sbase, tmem);
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kCtlRegs));
-    if (warp == C::kMmaWarp) score_role(ta, sh, sbase, tmem);
-    else if (warp == C::kLoadWarp) copy_role(ta, sh, sbase, sm);
-    else value_role(ta, sh, sbase, sm, tmem, warp - C::kValWarp);
+    if constexpr (!C::kF16) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kCtlRegs));
+    if (warp == C::kMmaWarp) score_role<C>(ta, sh, sbase, tmem);
+    else if (warp == C::kLoadWarp) copy_role<C>(ta, sh, sbase, sm);
+    else value_role<C>(ta, sh, sbase, sm, tmem, warp - C::kValWarp);
   }
 
   // ---- common exit
@@ -1551,20 +1622,22 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// One latent tensor [T, Hkv, R] int8 with byte strides (st, sh) as a 3-D tensor map [Hkv][T][R], whatever the
-// order of the strides; box = 64 bytes x `slots` token slots x `heads` KV heads, so that a head's rows sit
+// One latent tensor [T, Hkv, R] with element strides (st, sh) as a 3-D tensor map [Hkv][T][R], whatever the
+// order of the strides; box = 64 ranks x `slots` token slots x `heads` KV heads, so that a head's rows sit
 // together in shared memory.  The box is wider than the tensor when the rank is below 64, and may reach past
-// the last head: the missing bytes arrive as zeros.
-bool encode_latent(CUtensorMap* map, const void* base, int64_t st, int64_t sh, int64_t T, int Hkv, int R, int heads,
-                   int slots) {
+// the last head: the missing elements arrive as zeros.
+bool encode_latent(CUtensorMap* map, const void* base, bool f16, int64_t st, int64_t sh, int64_t T, int Hkv, int R,
+                   int heads, int slots) {
   EncodeTiledFn fn = encode_fn();
   if (!fn || T <= 0 || T > 0xffffffffll || st < 0 || sh < 0) return false;
+  const int64_t size = f16 ? 2 : 1;
   cuuint64_t dims[3] = {(cuuint64_t)R, (cuuint64_t)T, (cuuint64_t)Hkv};
-  cuuint64_t strides[2] = {(cuuint64_t)st, (cuuint64_t)sh};
+  cuuint64_t strides[2] = {(cuuint64_t)(st * size), (cuuint64_t)(sh * size)};
   cuuint32_t box[3] = {64, (cuuint32_t)slots, (cuuint32_t)heads};
   cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+  const CUresult r = fn(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
+                        const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        f16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
@@ -1595,10 +1668,9 @@ cudaError_t launch_rope_table(void* table, int rows, const KArgs& a, cudaStream_
   return cudaGetLastError();
 }
 
-cudaError_t launch_stage1_tc(const KArgs& a, const void* table, int table_rows, const Stage1Work& work,
-                             cudaStream_t stream) {
-  using C = tc::Cfg;
-  cudaError_t e = cudaFuncSetAttribute(tc::stage1_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+template <class C>
+static cudaError_t launch_tc(const KArgs& a, const void* table, int table_rows, const Stage1Work& work, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(tc::stage1_tc_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)C::kSmemBytes);
   if (e != cudaSuccess) return e;
   tc::TcArgs ta;
@@ -1609,11 +1681,11 @@ cudaError_t launch_stage1_tc(const KArgs& a, const void* table, int table_rows, 
   for (CUtensorMap* m : {&ta.tmap_k, &ta.tmap_v, &ta.tmap_k16, &ta.tmap_v16}) memset(m, 0, sizeof(CUtensorMap));
   if (!tc::encode_table(&ta.tmap_table, table, table_rows)) return cudaErrorInvalidValue;
   if (a.p.n_token_slots > 0) {
-    // KV heads one group of query heads can touch (its first head is a multiple of the group's size, 4)
+    // KV heads one group of query heads can touch (its first head is a multiple of the group's size)
     const int gqa = a.p.n_q_heads / a.p.n_kv_heads;
-    const int heads = gqa == 1 ? 4 : gqa == 2 ? 2 : gqa % 4 == 0 ? 1 : 2;
+    const int heads = gqa == 1 ? C::kG : gqa == 2 ? C::kG / 2 : gqa % C::kG == 0 ? 1 : 2;
     auto encode = [&](CUtensorMap* m, bool is_k, int heads_in_box, int slots) {
-      return tc::encode_latent(m, is_k ? a.p.latent_k : a.p.latent_v, is_k ? a.p.k_stride_t : a.p.v_stride_t,
+      return tc::encode_latent(m, is_k ? a.p.latent_k : a.p.latent_v, C::kF16, is_k ? a.p.k_stride_t : a.p.v_stride_t,
                                is_k ? a.p.k_stride_h : a.p.v_stride_h, a.p.n_token_slots, a.p.n_kv_heads,
                                is_k ? a.p.rank_k : a.p.rank_v, heads_in_box, slots);
     };
@@ -1634,8 +1706,14 @@ cudaError_t launch_stage1_tc(const KArgs& a, const void* table, int table_rows, 
     e = cudaMemsetAsync(work.arrivals, 0, sizeof(unsigned int) * (size_t)a.p.batch * a.p.n_q_heads, stream);
     if (e != cudaSuccess) return e;
   }
-  tc::stage1_tc_kernel<<<grid, C::kThreads, C::kSmemBytes, stream>>>(ta);
+  tc::stage1_tc_kernel<C><<<grid, C::kThreads, C::kSmemBytes, stream>>>(ta);
   return cudaGetLastError();
+}
+
+cudaError_t launch_stage1_tc(const KArgs& a, const void* table, int table_rows, const Stage1Work& work,
+                             cudaStream_t stream) {
+  return a.p.latent_dtype == WSVD_F16 ? launch_tc<tc::Cfg<true>>(a, table, table_rows, work, stream)
+                                      : launch_tc<tc::Cfg<false>>(a, table, table_rows, work, stream);
 }
 
 cudaError_t read_tc_status(unsigned int* out) {

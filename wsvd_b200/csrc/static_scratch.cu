@@ -48,7 +48,15 @@ extern "C" int wsvd_latent_decode_static(const WsvdLatentDecodeParams* p, void* 
   const int st = wsvd::validate_decode_params(p);
   if (st != WSVD_OK) return st;
   if (p->batch == 0) return WSVD_OK;
-  const size_t need = wsvd_latent_decode_workspace_bytes(p);
+  size_t need = wsvd_latent_decode_workspace_bytes(p);
+  WsvdLatentDecodeParams split;
+  if (need > (size_t)WSVD_STATIC_SCRATCH_BYTES && p->kernel == WSVD_KERNEL_AUTO && p->latent_dtype == WSVD_F16) {
+    // f16 latents: the warp-MMA kernel's fixed splits may fit where the balanced shares do not
+    split = *p;
+    split.kernel = WSVD_KERNEL_MMA;
+    const size_t less = wsvd_latent_decode_workspace_bytes(&split);
+    if (less < need) p = &split, need = less;
+  }
   if (need > (size_t)WSVD_STATIC_SCRATCH_BYTES) return WSVD_ERR_TOO_LARGE;
   void* scratch = nullptr;
   const cudaError_t e = scratch_for_current_device(&scratch);
