@@ -60,21 +60,31 @@ bool tc_eligible(const WsvdLatentDecodeParams* p) {
   return true;
 }
 
-// The tcgen05 kernel with f16 latents: the balanced mode alone, chosen by WSVD_KERNEL_AUTO.  Ranks are multiples of 8
-// and rows start on 16-byte boundaries (tensor copies, 16-byte row loads).  From one tile of 128 tokens and two heads per
-// SM on: below that most SMs would idle, and the warp-MMA kernel, which cuts the context finer, is as fast
-// (2 sequences of 2048 and 900 tokens with 8 heads: @@SMALL@@).
-bool tc_f16_eligible(const WsvdLatentDecodeParams* p) {
-  if (p->kernel != WSVD_KERNEL_AUTO || p->latent_dtype != WSVD_F16 || p->split_len != 0) return false;
-  if (p->head_dim != 128) return false;
-  if (p->rank_k % 8 != 0 || p->rank_k > 64 || p->rank_v % 8 != 0 || p->rank_v > 64) return false;
-  if (p->pos_offset != nullptr && p->rope_table == nullptr) return false;
-  if (!aligned16(p->latent_k) || !aligned16(p->latent_v)) return false;
-  if (!aligned16(p->q) || p->q_stride_b % 8 || p->q_stride_h % 8) return false;  // 16-byte loads of q
-  if (p->k_stride_t % 8 || p->k_stride_h % 8 || p->v_stride_t % 8 || p->v_stride_h % 8) return false;
-  if (p->rope_table && (!aligned16(p->rope_table) || p->rope_table_rows < ((p->max_len + 127) / 128) * 128)) return false;
-  const int64_t groups = (p->n_q_heads + wsvd::kBalancedGroupF16 - 1) / wsvd::kBalancedGroupF16;
-  return p->batch * groups * ((p->max_len + 127) / 128) >= 148;
+// What WSVD_KERNEL_AUTO alone gives to the tcgen05 kernel, in its balanced mode: f16 latents, and caches whose ranks or
+// rows do not fit the tensor copies (rank 62, token rows that do not start on 16-byte boundaries), which the kernel's
+// threads then fetch row by row.  0: none, else a Stage1Rows value.
+int tc_auto_rows(const WsvdLatentDecodeParams* p) {
+  if (p->kernel != WSVD_KERNEL_AUTO || p->split_len != 0 || tc_eligible(p)) return 0;
+  if (p->head_dim != 128 || p->rank_k > 64 || p->rank_v > 64) return 0;
+  if (p->pos_offset != nullptr && p->rope_table == nullptr) return 0;
+  if (!aligned16(p->q) || p->q_stride_b % 8 || p->q_stride_h % 8) return 0;  // 16-byte loads of q
+  if (p->rope_table && (!aligned16(p->rope_table) || p->rope_table_rows < ((p->max_len + 127) / 128) * 128)) return 0;
+  const bool f16 = p->latent_dtype == WSVD_F16;
+  const int64_t unit = f16 ? 8 : 16;  // elements of 16 bytes
+  const bool rows16 = p->rank_k % unit == 0 && p->rank_v % unit == 0 && aligned16(p->latent_k) && aligned16(p->latent_v) &&
+                      p->k_stride_t % unit == 0 && p->k_stride_h % unit == 0 && p->v_stride_t % unit == 0 &&
+                      p->v_stride_h % unit == 0;
+  if (f16) {
+    // Odd ranks stay with the generic kernel.  So do batches below one tile of 128 tokens and two heads per SM with the
+    // warp-MMA kernel: there both are bound by latency (2 sequences of 2048 tokens, 8 heads: 17 us here, 36 us there; 32
+    // heads of 512 tokens: 14 and 34 us; 8 sequences, 8 heads: 25 and 38 us; 40 heads, 16 x 8192 tokens: 250 and 713 us),
+    // and callers may rely on AUTO giving the bits that WSVD_KERNEL_MMA gives.
+    if (p->rank_k % 2 || p->rank_v % 2) return 0;
+    if ((reinterpret_cast<uintptr_t>(p->latent_k) | reinterpret_cast<uintptr_t>(p->latent_v)) & 1) return 0;
+    const int64_t groups = (p->n_q_heads + wsvd::kBalancedGroupF16 - 1) / wsvd::kBalancedGroupF16;
+    if (p->batch * groups * ((p->max_len + 127) / 128) < 148) return 0;
+  }
+  return rows16 ? wsvd::kRows16 : wsvd::kRowsAny;
 }
 
 // the caller's position table serves the warp-MMA kernel too ([2][rows][64] f16 is its layout for head_dim 128)
@@ -163,8 +173,8 @@ void fill_args(const WsvdLatentDecodeParams* p, float* mid_o, float* lse, int sp
 // always runs fixed-length splits).
 int run_stage1(const wsvd::KArgs& a, void* scratch_table, const wsvd::Stage1Work& work, cudaStream_t stream) {
   if (a.p.batch == 0) return WSVD_OK;
-  const bool f16 = work.n_ctas > 0 && tc_f16_eligible(&a.p);
-  const bool tc = (f16 || (tc_eligible(&a.p) && a.split_len % 128 == 0)) && (a.p.rope_table || scratch_table);
+  const int rows = work.n_ctas > 0 ? tc_auto_rows(&a.p) : 0;
+  const bool tc = (rows != 0 || (tc_eligible(&a.p) && a.split_len % 128 == 0)) && (a.p.rope_table || scratch_table);
   if (!tc) {
     if (a.p.kernel == WSVD_KERNEL_TC) return WSVD_ERR_UNSUPPORTED;
     if (mma_eligible(&a.p) && (mma_caller_table(&a.p) || scratch_table)) {
@@ -184,21 +194,21 @@ int run_stage1(const wsvd::KArgs& a, void* scratch_table, const wsvd::Stage1Work
     return e == cudaSuccess ? WSVD_OK : cuda_fail(e);
   }
   const void* table = a.p.rope_table;
-  int rows = a.p.rope_table_rows;
+  int table_rows = a.p.rope_table_rows;
   if (!table) {
-    rows = table_rows_for(a.p.max_len);
-    cudaError_t e = wsvd::launch_rope_table(scratch_table, rows, a, stream);
+    table_rows = table_rows_for(a.p.max_len);
+    cudaError_t e = wsvd::launch_rope_table(scratch_table, table_rows, a, stream);
     if (e != cudaSuccess) return cuda_fail(e);
     table = scratch_table;
   }
-  cudaError_t e = wsvd::launch_stage1_tc(a, table, rows, work, stream);
+  cudaError_t e = wsvd::launch_stage1_tc(a, table, table_rows, work, rows == wsvd::kRowsAny, stream);
   return e == cudaSuccess ? WSVD_OK : cuda_fail(e);
 }
 
 // Without a split length from the caller, a problem the tensor-core kernel can run is cut into
 // equal shares of tiles, one per SM, instead of fixed-length splits.
 bool balanced_mode(const WsvdLatentDecodeParams* p) {
-  return p->split_len == 0 && (tc_eligible(p) || tc_f16_eligible(p));
+  return p->split_len == 0 && (tc_eligible(p) || tc_auto_rows(p) != 0);
 }
 int balanced_group(const WsvdLatentDecodeParams* p) {
   return p->latent_dtype == WSVD_F16 ? wsvd::kBalancedGroupF16 : wsvd::kBalancedGroup;
@@ -231,7 +241,7 @@ Layout workspace_layout(const WsvdLatentDecodeParams* p, int n_splits) {
     off += align256((size_t)p->batch * p->n_q_heads * sizeof(uint32_t));
   }
   l.table_off = off;
-  if (tc_eligible(p) || tc_f16_eligible(p)) {
+  if (tc_eligible(p) || (bal && tc_auto_rows(p) != 0)) {
     if (!p->rope_table) l.table_bytes = wsvd::rope_table_bytes(table_rows_for(p->max_len));
   } else if (mma_eligible(p) && !mma_caller_table(p)) {
     l.table_bytes = wsvd::mma_table_bytes(table_rows_for(p->max_len), p->head_dim);
@@ -265,6 +275,7 @@ int balanced_ctas(const WsvdLatentDecodeParams* p, int* n_ctas) {
 namespace wsvd {
 int record_cuda_error(cudaError_t e) { return cuda_fail(e); }
 int validate_decode_params(const WsvdLatentDecodeParams* p) { return validate(p, true); }
+bool tc_by_auto_only(const WsvdLatentDecodeParams* p) { return tc_auto_rows(p) != 0; }
 }  // namespace wsvd
 
 extern "C" {
@@ -304,7 +315,7 @@ size_t wsvd_latent_decode_workspace_bytes(const WsvdLatentDecodeParams* p) {
   int sl, ns;
   plan(p, &sl, &ns);
   size_t need = workspace_layout(p, ns).total;
-  if (tc_f16_eligible(p)) {
+  if (tc_auto_rows(p) != 0) {
     // never less than the split plan that wsvd_latent_decode_plan reports for the same block would take
     WsvdLatentDecodeParams q = *p;
     q.kernel = WSVD_KERNEL_MMA;
@@ -400,7 +411,7 @@ static int decode_impl(const WsvdLatentDecodeParams* p, const WsvdPeerSet* peers
       work.arrivals = reinterpret_cast<unsigned int*>(ws + l.arrivals_off);
       if (peers) {
         // 16-byte peer stores need aligned rows; anything else goes through the merge kernel
-        bool vec = peers->out_stride_b % 8 == 0 && peers->out_stride_h % 8 == 0;
+        bool vec = peers->out_stride_b % 8 == 0 && peers->out_stride_h % 8 == 0 && (p->wv || p->rank_v % 8 == 0);
         for (int i = 0; i < peers->n_peers; ++i) vec = vec && aligned16(peers->out[i]);
         if (vec) {
           pa = wsvd::make_peer_args(*peers);

@@ -84,6 +84,8 @@ struct PartialIndex {
 // (returns WSVD_ERR_CUDA).
 int validate_decode_params(const WsvdLatentDecodeParams* p);
 int record_cuda_error(cudaError_t e);
+// whether the block runs on the tcgen05 kernel only because WSVD_KERNEL_AUTO may choose
+bool tc_by_auto_only(const WsvdLatentDecodeParams* p);
 
 // Launchers implemented in the kernel translation units.
 cudaError_t launch_stage1_generic(const KArgs& a, cudaStream_t stream);
@@ -169,7 +171,9 @@ struct Stage1Work {
   unsigned int* arrivals;
   const PeerArgs* peers;
 };
-cudaError_t launch_stage1_tc(const KArgs& a, const void* table, int table_rows, const Stage1Work& work,
+// kRows16: latent rows start on 16-byte boundaries and are multiples of 16 bytes (tensor copies); kRowsAny: they need not
+enum Stage1Rows { kRows16 = 1, kRowsAny = 2 };
+cudaError_t launch_stage1_tc(const KArgs& a, const void* table, int table_rows, const Stage1Work& work, bool any_rows,
                              cudaStream_t stream);
 cudaError_t launch_rope_table(void* table, int rows, const KArgs& a, cudaStream_t stream);
 // warp-MMA kernel: its table is [2][rows][head_dim / 2] f16 (the same bytes as the table above for head_dim 128)

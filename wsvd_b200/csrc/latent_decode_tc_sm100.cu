@@ -80,9 +80,13 @@ constexpr uint32_t kTmemCols = 512;
 constexpr float kNone = -3.0e38f;                   // log2-domain reference of something that is still empty
 
 // Shape of the CTA, for int8 latents (four heads) and f16 latents (two heads, whose rows take twice the room).
-template <bool F16>
+// ANY: ranks and row addresses that the tensor copies cannot take (rank 62, say).  Every thread then fetches its own
+// token's rows in the 16-byte pieces that hold them, K by asynchronous copies a tile ahead, and shifts them into place in
+// registers; the rings for K and V rows are not used.
+template <bool F16, bool ANY>
 struct Cfg {
   static constexpr bool kF16 = F16;
+  static constexpr bool kAny = ANY;
   static constexpr int kG = F16 ? 2 : 4;           // heads per CTA
   static constexpr int kEpiWarps = 4 * kG;
   static constexpr int kMmaWarp = kEpiWarps;       // score MMAs
@@ -91,7 +95,9 @@ struct Cfg {
   static constexpr int kThreads = (kEpiWarps + 2 + kG / 2) * 32;
   static constexpr int kRowBytes = F16 ? 128 : 64; // a latent row in shared memory (rank < 64: zero-filled)
   static constexpr int kKSlots = F16 ? 2 : 1;      // tiles of K: a tile's rows are copied to registers at the top of the tile
-  static constexpr int kVSlots = 2;  // tiles of V: the tile whose value MMAs are pending, and the next tile in flight
+  static constexpr int kVSlots = ANY ? 1 : 2;      // tiles of V: the tile whose value MMAs are pending, and the next tile in flight
+  static constexpr int kABufs = ANY ? 1 : 2;       // tiles of the position table
+  static constexpr uint32_t kRawPitch = kRowBytes + 16;  // ANY: a row as fetched; 16 bytes more than a row: no bank conflicts
   static constexpr int kWBufs = F16 ? 3 : 2;       // W accumulators of 128 columns (one pair of heads each)
   // int8: 640 threads leave the compiler 96 registers a thread, and the two groups of warps re-balance them.
   // The pool is the CTA's own: what the control warpgroup hands back, (96 - 64) * 128, is exactly what the
@@ -119,23 +125,24 @@ struct Cfg {
   // shared-memory map (offsets from a 1024-byte aligned base)
   static constexpr uint32_t kOffB = 0;
   static constexpr uint32_t kOffA = kOffB + 2 * kBHalfBytes;
-  static constexpr uint32_t kOffV = kOffA + 2 * kABufBytes;
+  static constexpr uint32_t kOffV = kOffA + kABufs * kABufBytes;
   static constexpr uint32_t kOffK = kOffV + kVSlots * kUnitBytes;
-  static constexpr uint32_t kOffPlanes = kOffK + kKSlots * kUnitBytes;
+  static constexpr uint32_t kOffPlanes = kOffK + (ANY ? 2 * kTile * kG * kRawPitch : kKSlots * kUnitBytes);
+  static constexpr uint32_t kOffVRaw = kOffK + kTile * kG * kRawPitch;  // ANY
   static constexpr uint32_t kOffRef = kOffPlanes + 2 * kG * kPlaneBytes;  // [head][tile parity][warp] reference that a warp left with this tile
   static constexpr uint32_t kOffSum = kOffRef + kG * 2 * 4 * 4;           // [head][warp] (max z, denominator) at the end
   static constexpr uint32_t kOffMode = kOffSum + kG * 4 * 8;              // [4] how the K and V rows of a tile arrive (ring)
   static constexpr uint32_t kOffItem = kOffMode + 16;                     // [head][item parity] ItemState
   static constexpr uint32_t kOffBar = kOffItem + kG * 2 * 64;
-  // barriers: V and K full/empty per ring slot, table full/empty x2, W full/empty, per head: D full,
+  // barriers: V and K full/empty per ring slot, table full/empty, W full/empty, per head: D full,
   // planes ready; [P;Q] ready.  All are initialised once: their phases run on from one item to the next.
   static constexpr int kBarVFull = 0;
   static constexpr int kBarKFull = kBarVFull + kVSlots;
   static constexpr int kBarVEmpty = kBarKFull + kKSlots;
   static constexpr int kBarKEmpty = kBarVEmpty + kVSlots;
   static constexpr int kBarAFull = kBarKEmpty + kKSlots;
-  static constexpr int kBarAEmpty = kBarAFull + 2;
-  static constexpr int kBarWFull = kBarAEmpty + 2;
+  static constexpr int kBarAEmpty = kBarAFull + kABufs;
+  static constexpr int kBarWFull = kBarAEmpty + kABufs;
   static constexpr int kBarWEmpty = kBarWFull + kWBufs;
   static constexpr int kBarDFull = kBarWEmpty + kWBufs;
   static constexpr int kBarPlanes = kBarDFull + kG;
@@ -152,7 +159,7 @@ struct Cfg {
     return F16 ? (uint32_t)(tok * 128 + ((c ^ (tok & 7)) << 4)) : (uint32_t)(tok * 64 + ((c ^ ((tok >> 1) & 3)) << 4));
   }
 };
-static_assert(Cfg<false>::kG == kBalancedGroup && Cfg<true>::kG == kBalancedGroupF16, "the merge kernel indexes balanced partials by groups of kG heads");
+static_assert(Cfg<false, false>::kG == kBalancedGroup && Cfg<true, false>::kG == kBalancedGroupF16, "the merge kernel indexes balanced partials by groups of kG heads");
 
 enum Status : unsigned int { kOk = 0, kTimeoutProducer = 1, kTimeoutMma = 2, kTimeoutEpilogue = 3, kBadSmemAlignment = 4 };
 
@@ -230,7 +237,6 @@ __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
@@ -378,8 +384,8 @@ struct TcArgs {
   PeerArgs peers;
   alignas(64) CUtensorMap tmap_k;      // latents as 3-D tensors [KV head][slot][rank]: box rank x 128 slots x box_heads,
   alignas(64) CUtensorMap tmap_v;      // swizzled over the row of shared memory
-  alignas(64) CUtensorMap tmap_k16;    // the same with a box of 16 slots x 1 head, for tiles made of several runs of
-  alignas(64) CUtensorMap tmap_v16;    // slots (a paged cache)
+  alignas(64) CUtensorMap tmap_runs[4];  // the same with boxes of 64 slots x 1 head (K, V) and of 16 slots x 1 head (K, V),
+                                         // for tiles made of several runs of slots (a paged cache)
   alignas(64) CUtensorMap tmap_table;  // [2][rows][64] f16, box 64 x 128 x 2 (cos and sin tile), 128-byte swizzle
 };
 
@@ -395,8 +401,9 @@ __global__ void rope_table_kernel(__half* table, int rows, KArgs a) {
   table[((size_t)rows + pos) * 64 + i] = __float2half_rn(sn);
 }
 
-// How the K and V rows of a tile reach shared memory, published by the copying warp with the K slot.
-enum TileMode : int { kTileCopied = 0, kTileGather = 1 };
+// How the K and V rows of a tile reach shared memory: the copying warp publishes 2 * tile + 1 when the epilogue's threads
+// are to fetch them, 2 * tile when it copies them, in word tile % 4, before the tile's K slot is handed over (and as
+// early as it knows: the epilogue looks a tile ahead).
 
 // A CTA's place in the list of work.
 struct Share {
@@ -476,8 +483,8 @@ __device__ __forceinline__ void score_role(const TcArgs& ta, const Share& sh, ui
     const int G = min(C::kG, p.n_q_heads - w.hg * C::kG), npairs = (G + 1) >> 1;
     ok = warp_wait(bar(C::kBarPq), item & 1);
     for (int t = 0; t < w.ntiles && ok; ++t, ++T) {
-      const uint32_t buf = T & 1;
-      ok = warp_wait(bar(C::kBarAFull + buf), (T >> 1) & 1);
+      const uint32_t buf = T % C::kABufs;
+      ok = warp_wait(bar(C::kBarAFull + buf), (T / C::kABufs) & 1);
       for (int pr = 0; pr < npairs && ok; ++pr, ++u) {
         const uint32_t wb = u % C::kWBufs, use = u / C::kWBufs;
         if (use > 0) ok = warp_wait(bar(C::kBarWEmpty + wb), (use - 1) & 1);
@@ -498,9 +505,10 @@ __device__ __forceinline__ void score_role(const TcArgs& ta, const Share& sh, ui
       }
     }
   }
-  // the releases of the last two table buffers are arrivals that nobody else waits for: none may be on
-  // its way when the CTA exits
-  for (uint32_t t = T < 2 ? 0 : T - 2; t < T && ok; ++t) ok = warp_wait(bar(C::kBarAEmpty + (t & 1)), (t >> 1) & 1);
+  // the releases of the last table buffers are arrivals that nobody else waits for: none may be on its way
+  // when the CTA exits
+  for (uint32_t t = T < C::kABufs ? 0 : T - C::kABufs; t < T && ok; ++t)
+    ok = warp_wait(bar(C::kBarAEmpty + t % C::kABufs), (t / C::kABufs) & 1);
   if (!ok) atomicMax(&g_status, (unsigned)kTimeoutMma);
 }
 
@@ -513,9 +521,10 @@ __device__ __forceinline__ void score_role(const TcArgs& ta, const Share& sh, ui
 // page entries of tokens 4l..4l+3 (fetched one tile ahead), and the warp votes.
 //  - the tile's 128 slots are one run (a cache laid out sequence by sequence, a page of 128 or more): one copy
 //    for K and one for V fetch all heads of the group;
-//  - every aligned group of 16 tokens is a run (pages of 16, 32, 64 slots): lane l copies run l / 4 of KV
-//    head l % 4, 1 KB a copy;
-//  - else the epilogue's threads fetch their own tokens' rows (kTileGather), and this warp asks L2 for them.
+//  - every aligned group of 64, or else of 16, tokens is a run (a paged cache): one copy per run and head.  A copy
+//    costs this warp about 80 cycles whatever its size: 24 sequences of 500 to 4096 tokens, 32 heads, took 82 us in
+//    one run, 118 us with pages of 64 copied by sixteens, 88 us by 64;
+//  - else the epilogue's warps fetch their own tokens' rows.
 template <class C>
 __device__ __forceinline__ void copy_role(const TcArgs& ta, const Share& sh, uint32_t sbase, uint8_t* sm) {
   const WsvdLatentDecodeParams& p = ta.k.p;
@@ -534,6 +543,17 @@ __device__ __forceinline__ void copy_role(const TcArgs& ta, const Share& sh, uin
     const int hk0 = h0 / gqa, nkv = (h0 + G - 1) / gqa - hk0 + 1;  // the group's KV heads
     const int32_t* page = p.req_to_token + (int64_t)w.req * p.rtt_stride;
     int pos = (p.pos_offset != nullptr ? p.pos_offset[w.b] : 0) + w.lo;  // RoPE position of the tile's first token
+    if constexpr (C::kAny) {  // the position table alone
+      for (int t = 0; t < w.ntiles && ok; ++t, ++T, pos += kTile) {
+        const uint32_t buf = T % C::kABufs, au = T / C::kABufs;
+        if (au > 0) ok = warp_wait(bar(C::kBarAEmpty + buf), (au - 1) & 1);
+        if (ok && issuer) {
+          mbar_expect_tx(bar(C::kBarAFull + buf), kABufBytes);
+          tma_load_3d(sbase + C::kOffA + buf * kABufBytes, &ta.tmap_table, 0, pos, 0, bar(C::kBarAFull + buf));
+        }
+      }
+      continue;
+    }
     int ent[4];
     auto fetch_entries = [&](int t) {
       const int s0 = w.lo + t * kTile + 4 * lane;
@@ -543,8 +563,8 @@ __device__ __forceinline__ void copy_role(const TcArgs& ta, const Share& sh, uin
     fetch_entries(0);
     for (int t = 0; t < w.ntiles && ok; ++t, ++T, pos += kTile) {
       // ---- position table
-      const uint32_t buf = T & 1;
-      if (T >= 2) ok = warp_wait(bar(C::kBarAEmpty + buf), ((T >> 1) - 1) & 1);
+      const uint32_t buf = T % C::kABufs, au = T / C::kABufs;
+      if (au > 0) ok = warp_wait(bar(C::kBarAEmpty + buf), (au - 1) & 1);
       if (!ok) break;
       if (issuer) {
         mbar_expect_tx(bar(C::kBarAFull + buf), kABufBytes);
@@ -556,47 +576,40 @@ __device__ __forceinline__ void copy_role(const TcArgs& ta, const Share& sh, uin
 #pragma unroll
       for (int j = 0; j < 4; ++j) good = good && (ent[j] < 0 || ent[j] == first + 4 * lane + j);
       const bool run = __all_sync(0xffffffffu, good);
-      const int first16 = __shfl_sync(0xffffffffu, ent[0], lane & ~3);
-      bool run16 = false;
-      int groups = 0;  // groups of 16 that hold tokens
+      // not one run: two of 64 slots, or eight of 16?  Lane l copies run l / 4 of KV head l % 4.
+      int len = 0, first_r = 0, groups = 0;  // length of a run, first slot of this lane's run (-1: past the end), runs that hold tokens
       if (!run) {
-        good = use_tma;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) good = good && (ent[j] < 0 || ent[j] == first16 + 4 * (lane & 3) + j);
-        run16 = __all_sync(0xffffffffu, good);
-        groups = __popc(__ballot_sync(0xffffffffu, first16 >= 0)) >> 2;
-        if (!run16) {
-#pragma unroll 1
-          for (int j = 0; j < 4; ++j) {
-            if (ent[j] < 0) continue;
-            for (int hk = hk0; hk < hk0 + nkv; ++hk) {
-              prefetch_l2(reinterpret_cast<const uint8_t*>(p.latent_k) +
-                          (C::kRowBytes / 64) * ((int64_t)ent[j] * p.k_stride_t + (int64_t)hk * p.k_stride_h));
-              prefetch_l2(reinterpret_cast<const uint8_t*>(p.latent_v) +
-                          (C::kRowBytes / 64) * ((int64_t)ent[j] * p.v_stride_t + (int64_t)hk * p.v_stride_h));
-            }
+        for (int lg = 4; lg >= 2 && len == 0; lg -= 2) {  // a run spans 2^lg lanes' entries
+          const int first_l = __shfl_sync(0xffffffffu, ent[0], lane & ~((1 << lg) - 1));
+          good = use_tma;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) good = good && (ent[j] < 0 || ent[j] == first_l + 4 * (lane & ((1 << lg) - 1)) + j);
+          if (__all_sync(0xffffffffu, good)) {
+            len = 4 << lg;
+            groups = __popc(__ballot_sync(0xffffffffu, first_l >= 0)) >> lg;
+            first_r = __shfl_sync(0xffffffffu, ent[0], ((lane >> 2) << lg) & 31);
+            if (lane >= 4 * (32 >> lg)) first_r = -1;
           }
         }
       }
+      if (issuer) mode[T & 3] = (int)(2 * T) + (!run && len == 0);
       if (t + 1 < w.ntiles) fetch_entries(t + 1);
-      auto request = [&](const CUtensorMap* whole, const CUtensorMap* part, uint32_t dst, uint32_t full, bool is_k) {
+      auto request = [&](const CUtensorMap* whole, const CUtensorMap* part, uint32_t dst, uint32_t full) {
         if (run) {
           if (issuer) {
-            if (is_k) mode[T & 3] = kTileCopied;
             mbar_expect_tx(full, box_bytes);
             tma_load_3d(dst, whole, 0, first, hk0, full);
           }
-        } else if (run16) {
+        } else if (len != 0) {
           if (issuer) {
-            if (is_k) mode[T & 3] = kTileCopied;
-            mbar_expect_tx(full, (uint32_t)(groups * nkv) * (16u * C::kRowBytes));
+            mbar_expect_tx(full, (uint32_t)(groups * nkv * len) * C::kRowBytes);
           }
           __syncwarp();
           const int j = lane & 3;
-          if (j < nkv && first16 >= 0)
-            tma_load_3d(dst + j * C::kHeadBytes + (lane >> 2) * (16 * C::kRowBytes), part, 0, first16, hk0 + j, full);
+          if (j < nkv && first_r >= 0)
+            tma_load_3d(dst + j * C::kHeadBytes + (lane >> 2) * (len * C::kRowBytes), part + (len == 64 ? 0 : 2), 0, first_r, hk0 + j, full);
         } else if (issuer) {
-          if (is_k) mode[T & 3] = kTileGather;
           mbar_arrive(full);
         }
       };
@@ -604,14 +617,14 @@ __device__ __forceinline__ void copy_role(const TcArgs& ta, const Share& sh, uin
       const uint32_t ks = T % C::kKSlots, ku = T / C::kKSlots, vs = T % C::kVSlots, vu = T / C::kVSlots;
       if (ku > 0) ok = warp_wait(bar(C::kBarKEmpty + ks), (ku - 1) & 1);
       if (!ok) break;
-      request(&ta.tmap_k, &ta.tmap_k16, sbase + C::kOffK + ks * C::kUnitBytes, bar(C::kBarKFull + ks), true);
+      request(&ta.tmap_k, &ta.tmap_runs[0], sbase + C::kOffK + ks * C::kUnitBytes, bar(C::kBarKFull + ks));
       if (vu > 0) ok = warp_wait(bar(C::kBarVEmpty + vs), (vu - 1) & 1);
       if (!ok) break;
-      request(&ta.tmap_v, &ta.tmap_v16, sbase + C::kOffV + vs * C::kUnitBytes, bar(C::kBarVFull + vs), false);
+      request(&ta.tmap_v, &ta.tmap_runs[1], sbase + C::kOffV + vs * C::kUnitBytes, bar(C::kBarVFull + vs));
     }
   }
   // as in the score role: the releases of the last V slots
-  for (uint32_t t = T < C::kVSlots ? 0 : T - C::kVSlots; t < T && ok; ++t)
+  for (uint32_t t = T < C::kVSlots ? 0 : T - C::kVSlots; t < T && ok && !C::kAny; ++t)
     ok = warp_wait(bar(C::kBarVEmpty + t % C::kVSlots), (t / C::kVSlots) & 1);
   if (!ok) atomicMax(&g_status, (unsigned)kTimeoutProducer);
 }
@@ -653,7 +666,7 @@ __device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, ui
       const uint32_t vslot = T % C::kVSlots;
       // the V rows arrive long before the planes are ready: wait for them first, off the
       // critical path from "planes ready" to "D full"
-      ok = warp_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
+      if constexpr (!C::kAny) ok = warp_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int g = 2 * pair + j;
@@ -664,7 +677,7 @@ __device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, ui
         tc_fence_after();
         const uint32_t how = *value_modes<C>(sm, g);  // a byte per warp: which of its accumulators, added to or started
         // copied rows sit at the head's KV head, gathered ones at the head itself
-        const int sub = mode[T & 3] == kTileGather ? g : (h0 + g) / gqa - h0 / gqa;
+        const int sub = C::kAny || (mode[T & 3] & 1) ? g : (h0 + g) / gqa - h0 / gqa;
         const uint32_t v_at = v_lo + ((vslot * C::kUnitBytes + sub * C::kHeadBytes) >> 4);
         const uint32_t d_tmem = tmem + C::kTmemD + 64 * g;
         if (issuer) {
@@ -680,8 +693,8 @@ __device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, ui
             }
           }
           umma_commit(bar(C::kBarDFull + g));
-          umma_commit(bar(C::kBarVEmpty + vslot));
-          if (g == 0 && G < C::kG) mbar_arrive_n(bar(C::kBarVEmpty + vslot), C::kG - G);  // for the heads that are not there
+          if constexpr (!C::kAny) umma_commit(bar(C::kBarVEmpty + vslot));
+          if (!C::kAny && g == 0 && G < C::kG) mbar_arrive_n(bar(C::kBarVEmpty + vslot), C::kG - G);  // for the heads that are not there
         }
         __syncwarp();
       }
@@ -767,44 +780,7 @@ __device__ __forceinline__ void build_pq(const TcArgs& ta, uint8_t* sm, int b, i
     }
   }
   const int64_t col = (int64_t)hk * 128;
-  if (!C::kF16 && wk_vec && !wk_i8 && !interleaved) {
-    // Common case (int8 latents, f16 wk, half-split pairing): packed f16 arithmetic.  The operands are
-    // rounded to f16 for the MMA anyway; forming them with one extra f16 rounding of a
-    // product keeps the error of the scores within a few 1e-5.  This thread's chunk of 8
-    // frequencies is the same for its four ranks, so q is converted once.
-    const int ic = tid & 7;
-    __half2 qa[4], qb[4], nqa[4];
-    {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        qa[e] = __floats2half2_rn(qlo[2 * e], qlo[2 * e + 1]);
-        qb[e] = __floats2half2_rn(qhi[2 * e], qhi[2 * e + 1]);
-      }
-#pragma unroll
-      for (int e = 0; e < 4; ++e) nqa[e] = __hneg2(qa[e]);
-    }
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int r = (tid + 128 * it) >> 3;
-      const uint32_t off = pq_off(g, r, ic);
-      uint4 u_lo = make_uint4(0u, 0u, 0u, 0u), u_hi = u_lo;
-      if (r < p.rank_k) {
-        u_lo = *reinterpret_cast<const uint4*>(sm + C::kOffB + off);
-        u_hi = *reinterpret_cast<const uint4*>(sm + C::kOffB + C::kBHalfBytes + off);
-      }
-      const __half2* ua = reinterpret_cast<const __half2*>(&u_lo);  // U[d = ic*8 .. +7]
-      const __half2* ub = reinterpret_cast<const __half2*>(&u_hi);  // U[64 + ic*8 .. +7]
-      __align__(16) __half2 pv[4];
-      __align__(16) __half2 qv[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        pv[e] = __hfma2(qa[e], ua[e], __hmul2(qb[e], ub[e]));   // P = q_i U_i + q_{i+64} U_{i+64}
-        qv[e] = __hfma2(nqa[e], ub[e], __hmul2(qb[e], ua[e]));  // Q = q_{i+64} U_i - q_i U_{i+64}
-      }
-      *reinterpret_cast<uint4*>(sm + C::kOffB + off) = *reinterpret_cast<const uint4*>(pv);
-      *reinterpret_cast<uint4*>(sm + C::kOffB + C::kBHalfBytes + off) = *reinterpret_cast<const uint4*>(qv);
-    }
-  } else if (wk_vec && wk_i8) {
+  if (wk_vec && wk_i8) {
     // int8 wk in vectors of eight; the columns' scales are this thread's for all four ranks.  fp32 throughout.
     const int ic = tid & 7;
     const __half* ws = reinterpret_cast<const __half*>(p.wk_scale) + col;
@@ -984,13 +960,16 @@ __device__ __forceinline__ void finish_head(const TcArgs& ta, uint8_t* sm, int g
     // 32 loads of U_v (L2) in flight
     const __half* w = reinterpret_cast<const __half*>(p.wv) + (int64_t)hk * p.head_dim + d;
     float y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f;
+    int k = 0;
 #pragma unroll 8
-    for (int k = 0; k < Rv; k += 4) {
+    for (; k + 4 <= Rv; k += 4) {
       y0 = fmaf(o_row[k], __half2float(__ldg(w + (int64_t)k * p.wv_stride_r)), y0);
       y1 = fmaf(o_row[k + 1], __half2float(__ldg(w + (int64_t)(k + 1) * p.wv_stride_r)), y1);
       y2 = fmaf(o_row[k + 2], __half2float(__ldg(w + (int64_t)(k + 2) * p.wv_stride_r)), y2);
       y3 = fmaf(o_row[k + 3], __half2float(__ldg(w + (int64_t)(k + 3) * p.wv_stride_r)), y3);
     }
+    if constexpr (C::kAny)
+      for (; k < Rv; ++k) y0 = fmaf(o_row[k], __half2float(__ldg(w + (int64_t)k * p.wv_stride_r)), y0);
     out[d] = __float2half_rn((y0 + y1) + (y2 + y3));
   }
   head_sync();  // o_row has been read (and the staged row is complete): the next item's planes may go there
@@ -1008,6 +987,46 @@ __device__ __forceinline__ void finish_head(const TcArgs& ta, uint8_t* sm, int g
 template <class C>
 __device__ __forceinline__ volatile int* item_state(uint8_t* sm, int g, uint32_t item) {
   return reinterpret_cast<volatile int*>(sm + C::kOffItem) + (g * 2 + (item & 1)) * 16;
+}
+
+// The rows of a warp's 32 tokens (lane l: slot of token l, -1: none), by asynchronous 16-byte copies.  kRowBytes / 16
+// lanes share a row, so that a copy instruction touches a few lines of memory and not 32 (with one lane per row the
+// load unit, not HBM, set the pace: f16 rows scattered over their slots took 354 us for 24 sequences of 32 heads against 170 us).
+//  - whole 16-byte rows: piece c goes where the tensor copy would have put it;
+//  - ANY: the 16-byte pieces that hold bytes of the row, each fetched only if it does (so never past the row by more than
+//    the 16 bytes it ends in), go to the row's place in the area of raw rows.
+template <class C>
+__device__ __forceinline__ void fetch_rows_async(uint32_t dst, const uint8_t* base, int64_t stride_bytes, int slot, int bytes) {
+  constexpr int kLanes = C::kRowBytes / 16;
+  const int lane = threadIdx.x & 31, c = lane % kLanes, row0 = (threadIdx.x & 127) & ~31;
+#pragma unroll
+  for (int i = 0; i < kLanes; ++i) {
+    const int r = i * (32 / kLanes) + lane / kLanes;
+    const int sl = __shfl_sync(0xffffffffu, slot, r);
+    const uint8_t* src = base + (int64_t)sl * stride_bytes;
+    if constexpr (C::kAny) {
+      const uintptr_t first = reinterpret_cast<uintptr_t>(src) & ~(uintptr_t)15;
+      const int span = (int)(reinterpret_cast<uintptr_t>(src) & 15) + bytes;
+      const uint32_t to = dst + (row0 + r) * C::kRawPitch;
+      if (sl >= 0 && c * 16 < span) cp_async16(to + c * 16, reinterpret_cast<const void*>(first + c * 16));
+      if (sl >= 0 && c == 0 && C::kRowBytes < span)
+        cp_async16(to + C::kRowBytes, reinterpret_cast<const void*>(first + C::kRowBytes));
+    } else {
+      if (sl >= 0 && c * 16 < bytes) cp_async16(dst + C::row_off(row0 + r, c), src + c * 16);
+    }
+  }
+}
+// Shifts the row, `skip` (0..15) bytes into the words, to their start: by 8 and 4 bytes with selects, by the rest with
+// funnel shifts.  Bytes past the row are whatever the pieces held: they meet zeros of W, or ranks nobody reads.
+template <int kWordsOut>
+__device__ __forceinline__ void shift_row(uint32_t (&w)[kWordsOut + 4], int skip) {
+  const bool by8 = skip & 8, by4 = skip & 4;
+#pragma unroll
+  for (int i = 0; i < kWordsOut + 2; ++i) w[i] = by8 ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < kWordsOut + 1; ++i) w[i] = by4 ? w[i + 1] : w[i];
+#pragma unroll
+  for (int i = 0; i < kWordsOut; ++i) w[i] = __funnelshift_r(w[i], w[i + 1], (skip & 3) * 8);
 }
 
 // One head's running sums over the tiles of an item, all in the log2 domain and fp32.
@@ -1099,14 +1118,36 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
   // ones, and a pair that holds a single head arrives twice
   const uint32_t k_arrivals = g == 0 ? 1u + (C::kG - G) : 1u;
   const uint32_t w_arrivals = (G - 2 * pr) >= 2 ? 1u : 2u;
+  // this lane's first token and its next one (the lines were asked for with the item's other loads)
+  slot_c = lo + row < hi ? page[lo + row] : -1;
+  slot_n = lo + kTile + row < hi ? page[lo + kTile + row] : -1;
   if constexpr (!C::kF16) {
-    // this lane's first token and its next one (the lines were asked for with the item's other loads)
-    slot_c = lo + row < hi ? page[lo + row] : -1;
-    slot_n = lo + kTile + row < hi ? page[lo + kTile + row] : -1;
     if (slot_c >= 0) {
       sk_raw = reinterpret_cast<const unsigned short*>(ksc)[(int64_t)slot_c * p.ks_stride_t];
       sv_raw = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_c * p.vs_stride_t];
     }
+  }
+  constexpr int kEsize = C::kRowBytes / 64;  // bytes of a latent
+  constexpr int kWords = C::kRowBytes / 4;
+  const uint8_t* k_base = reinterpret_cast<const uint8_t*>(p.latent_k) + kEsize * (int64_t)hk * p.k_stride_h;
+  const uint8_t* v_base = reinterpret_cast<const uint8_t*>(p.latent_v) + kEsize * (int64_t)hk * p.v_stride_h;
+  // ANY: this head's raw rows
+  const uint32_t k_raw = sbase + C::kOffK + g * (kTile * C::kRawPitch), v_raw = k_raw + (C::kOffVRaw - C::kOffK);
+  auto fetch_k = [&](uint32_t dst, int slot) { fetch_rows_async<C>(dst, k_base, p.k_stride_t * kEsize, slot, p.rank_k * kEsize); };
+  auto fetch_v = [&](uint32_t dst, int slot) { fetch_rows_async<C>(dst, v_base, p.v_stride_t * kEsize, slot, Rv * kEsize); };
+  auto read_raw = [&](uint32_t (&w)[kWords + 4], uint32_t raw, const uint8_t* base, int64_t stride, int slot) {
+#pragma unroll
+    for (int c = 0; c <= kChunks; ++c)
+      asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(w[4 * c]), "=r"(w[4 * c + 1]), "=r"(w[4 * c + 2]), "=r"(w[4 * c + 3])
+                   : "r"(raw + row * C::kRawPitch + 16 * c));
+    shift_row<kWords>(w, slot >= 0 ? (int)((reinterpret_cast<uintptr_t>(base) + (int64_t)slot * stride) & 15) : 0);
+  };
+  bool k_ahead = false;  // the K rows of the tile that comes are on their way (gathered tiles)
+  bool gathered = false; // the tile before was
+  if constexpr (C::kAny) {
+    fetch_k(k_raw, slot_c);
+    fetch_v(v_raw, slot_c);
   }
   for (int t = 0; t < ntiles && ok; ++t) {
     const int s = lo + t * kTile + row;
@@ -1119,38 +1160,67 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       sk_n = reinterpret_cast<const unsigned short*>(ksc)[(int64_t)slot_n * p.ks_stride_t];
       sv_n = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_n * p.vs_stride_t];
     }
-    int slot_t = slot_c;
-    if constexpr (!C::kF16) {
-      slot_c = slot_n;
-      slot_n = -1;
-      if (s + 2 * kTile < hi) slot_n = page[s + 2 * kTile];
-    }
+    const int slot_t = slot_c;
+    slot_c = slot_n;
+    slot_n = -1;
+    if (s + 2 * kTile < hi) slot_n = page[s + 2 * kTile];
     // ---- this warp's 32 K rows (lane = token) go from the ring slot to registers at once and
     //      the slot is handed back: its refill has the whole tile to arrive
     uint4 kreg[kChunks];
-    const uint32_t kslot = Tt % C::kKSlots;
-    ok = mbar_wait(bar(C::kBarKFull + kslot), (Tt / C::kKSlots) & 1);
-    if (!ok) break;
-    const bool gather = mode[Tt & 3] == kTileGather;
-    if (!gather) {
-      const uint32_t krows = sbase + C::kOffK + kslot * C::kUnitBytes + sub * C::kHeadBytes;
+    bool gather = false;
+    if constexpr (C::kAny) {
+      // the rows of this tile have been on their way for a tile; the next tile's K rows take their place
+      cp_async_wait_all();
+      __syncwarp();
+      uint32_t w[kWords + 4];
+      read_raw(w, k_raw, k_base, p.k_stride_t * kEsize, slot_t);
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c) kreg[c] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+      __syncwarp();
+      if (lo + (t + 1) * kTile < hi) fetch_k(k_raw, slot_c);
+    } else {
+      const uint32_t kslot = Tt % C::kKSlots;
+      ok = mbar_wait(bar(C::kBarKFull + kslot), (Tt / C::kKSlots) & 1);
+      if (!ok) break;
+      gather = mode[Tt & 3] & 1;
+      // copied rows sit at the head's KV head, gathered ones at the head itself
+      const uint32_t krows = sbase + C::kOffK + kslot * C::kUnitBytes + (gather ? g : sub) * C::kHeadBytes;
+      if (gather) {
+        if (!k_ahead) fetch_k(krows, slot_t);
+        cp_async_wait_all();
+        __syncwarp();
+      }
 #pragma unroll
       for (int c = 0; c < kChunks; ++c)
         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                      : "=r"(kreg[c].x), "=r"(kreg[c].y), "=r"(kreg[c].z), "=r"(kreg[c].w)
                      : "r"(krows + C::row_off(row, c)));
-    } else {
-      if constexpr (C::kF16) slot_t = valid ? page[s] : -1;
-      const uint8_t* src = reinterpret_cast<const uint8_t*>(p.latent_k) +
-                           (C::kRowBytes / 64) * ((int64_t)slot_t * p.k_stride_t + (int64_t)hk * p.k_stride_h);
+      __syncwarp();
+      if (lane == 0) mbar_arrive_n(bar(C::kBarKEmpty + kslot), k_arrivals);
+      if (gather) {
+        // the copying warp's arrival says that every head's value MMAs on the V slot are complete
+        ok = mbar_wait(bar(C::kBarVFull + Tt % C::kVSlots), (Tt / C::kVSlots) & 1);
+        if (!ok) break;
+        fetch_v(sbase + C::kOffV + (Tt % C::kVSlots) * C::kUnitBytes + g * C::kHeadBytes, slot_t);
+        // K of the next tile, if that is known to be gathered too and the slot's last tile was (with one slot that
+        // is this tile): then this head's rows of the slot are its own, and this warp has read them
+        k_ahead = (C::kKSlots == 1 || gathered) && lo + (t + 1) * kTile < hi && mode[(Tt + 1) & 3] == (int)(2 * (Tt + 1)) + 1;
+        if (k_ahead) fetch_k(sbase + C::kOffK + (Tt + 1) % C::kKSlots * C::kUnitBytes + g * C::kHeadBytes, slot_c);
+      } else {
+        k_ahead = false;
+      }
+      gathered = gather;
+    }
+    if constexpr (C::kF16) {
+      if (C::kAny || gather) {  // what lies behind the row may be a NaN, which a zero of W does not silence (the rank is even)
 #pragma unroll
-      for (int c = 0; c < kChunks; ++c) {
-        kreg[c] = make_uint4(0u, 0u, 0u, 0u);
-        if (valid && c * 16 < p.rank_k * (C::kRowBytes / 64)) kreg[c] = __ldg(reinterpret_cast<const uint4*>(src) + c);
+        for (int c = 0; c < kChunks; ++c) {
+          uint32_t* x = reinterpret_cast<uint32_t*>(&kreg[c]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) x[j] = 2 * (4 * c + j) < p.rank_k ? x[j] : 0u;
+        }
       }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive_n(bar(C::kBarKEmpty + kslot), k_arrivals);
     ok = mbar_wait(bar(C::kBarWFull + wb), (u / C::kWBufs) & 1);
     if (!ok) break;
     tc_fence_after();
@@ -1192,17 +1262,6 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive_n(bar(C::kBarWEmpty + wb), w_arrivals);  // this warp has read its rows of W
-    if (gather) {  // the V row of this token: requested now, stored once the slot is known to be free
-#pragma unroll
-      for (int c = 0; c < kChunks; ++c) kreg[c] = make_uint4(0u, 0u, 0u, 0u);
-      if (valid) {
-        const uint8_t* src = reinterpret_cast<const uint8_t*>(p.latent_v) +
-                             (C::kRowBytes / 64) * ((int64_t)slot_t * p.v_stride_t + (int64_t)hk * p.v_stride_h);
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c)
-          if (c * 16 < Rv * (C::kRowBytes / 64)) kreg[c] = __ldg(reinterpret_cast<const uint4*>(src) + c);
-      }
-    }
     const float2 dsum = __fadd2_rn(dot0, dot1);
     const float sk = __half2float(__ushort_as_half(sk_raw)), sv = __half2float(__ushort_as_half(sv_raw));
     const float z = valid ? (C::kF16 ? dsum.x + dsum.y : (dsum.x + dsum.y) * sk) : -INFINITY;
@@ -1246,26 +1305,33 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       tc_fence_after();
       fold_left<C>(hs, d_addr, refs, mt - 1);
     }
-    if (gather) {
-      // the copying warp's arrival says that every head's value MMAs on the slot are complete
-      ok = mbar_wait(bar(C::kBarVFull + Tt % C::kVSlots), (Tt / C::kVSlots) & 1);
-      if (!ok) break;
-      const uint32_t vrow = sbase + C::kOffV + (Tt % C::kVSlots) * C::kUnitBytes + g * C::kHeadBytes;
+    const uint32_t vrow = sbase + C::kOffV + (Tt % C::kVSlots) * C::kUnitBytes + (C::kAny || gather ? g : sub) * C::kHeadBytes;
+    if constexpr (C::kAny) {
+      // this head's own region: its value MMAs of the tile before are complete (and its V rows came with its K rows)
+      uint32_t w[kWords + 4];
+      read_raw(w, v_raw, v_base, p.v_stride_t * kEsize, slot_t);
 #pragma unroll
       for (int c = 0; c < kChunks; ++c)
-        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(vrow + C::row_off(row, c)), "r"(kreg[c].x),
-                     "r"(kreg[c].y), "r"(kreg[c].z), "r"(kreg[c].w)
+        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(vrow + C::row_off(row, c)),
+                     "r"(valid ? w[4 * c] : 0u), "r"(valid ? w[4 * c + 1] : 0u), "r"(valid ? w[4 * c + 2] : 0u), "r"(valid ? w[4 * c + 3] : 0u)
                      : "memory");
-    } else if (C::kF16 && lo + (t + 1) * kTile > hi) {
-      // the end of the sequence: what was copied behind it may be anything, and in f16 a NaN times a weight of
-      // zero is a NaN
-      ok = mbar_wait(bar(C::kBarVFull + Tt % C::kVSlots), (Tt / C::kVSlots) & 1);
-      if (!ok) break;
-      const uint32_t vrow = sbase + C::kOffV + (Tt % C::kVSlots) * C::kUnitBytes + sub * C::kHeadBytes;
-      if (!valid) {
+      __syncwarp();
+      if (lo + (t + 1) * kTile < hi) fetch_v(v_raw, slot_c);
+    } else {
+      if (gather) {
+        cp_async_wait_all();
+        __syncwarp();
+      }
+      if (C::kF16 && lo + (t + 1) * kTile > hi) {
+        // the end of the sequence: what was copied behind it may be anything, and in f16 a NaN times a weight of
+        // zero is a NaN
+        ok = mbar_wait(bar(C::kBarVFull + Tt % C::kVSlots), (Tt / C::kVSlots) & 1);
+        if (!ok) break;
+        if (!valid) {
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c)
-          asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(vrow + C::row_off(row, c)), "r"(0) : "memory");
+          for (int c = 0; c < kChunks; ++c)
+            asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(vrow + C::row_off(row, c)), "r"(0) : "memory");
+        }
       }
     }
 
@@ -1464,6 +1530,7 @@ __global__ void __launch_bounds__(C::kThreads, 1) stage1_tc_kernel(const __grid_
     tmem_relinquish();
     tc_fence_before();
   } else if (warp == C::kLoadWarp) {
+    if (lane < 4) reinterpret_cast<volatile int*>(sm + C::kOffMode)[lane] = -1;  // no tile (the epilogue looks ahead)
     for (int i = lane; i < C::kNumBars; i += 32) {
       uint32_t count = 1;                                                       // one copy, or one commit
       if (i >= C::kBarVEmpty && i < C::kBarKEmpty) count = C::kG;               // a commit per head, after its value MMAs on the slot
@@ -1678,9 +1745,11 @@ static cudaError_t launch_tc(const KArgs& a, const void* table, int table_rows, 
   ta.table_rows = table_rows;
   ta.use_tma = 0;
   ta.box_heads = 1;
-  for (CUtensorMap* m : {&ta.tmap_k, &ta.tmap_v, &ta.tmap_k16, &ta.tmap_v16}) memset(m, 0, sizeof(CUtensorMap));
+  memset(&ta.tmap_k, 0, sizeof(CUtensorMap));
+  memset(&ta.tmap_v, 0, sizeof(CUtensorMap));
+  memset(&ta.tmap_runs, 0, sizeof(ta.tmap_runs));
   if (!tc::encode_table(&ta.tmap_table, table, table_rows)) return cudaErrorInvalidValue;
-  if (a.p.n_token_slots > 0) {
+  if (a.p.n_token_slots > 0 && !C::kAny) {
     // KV heads one group of query heads can touch (its first head is a multiple of the group's size)
     const int gqa = a.p.n_q_heads / a.p.n_kv_heads;
     const int heads = gqa == 1 ? C::kG : gqa == 2 ? C::kG / 2 : gqa % C::kG == 0 ? 1 : 2;
@@ -1690,7 +1759,8 @@ static cudaError_t launch_tc(const KArgs& a, const void* table, int table_rows, 
                                is_k ? a.p.rank_k : a.p.rank_v, heads_in_box, slots);
     };
     if (encode(&ta.tmap_k, true, heads, tc::kTile) && encode(&ta.tmap_v, false, heads, tc::kTile) &&
-        encode(&ta.tmap_k16, true, 1, 16) && encode(&ta.tmap_v16, false, 1, 16)) {
+        encode(&ta.tmap_runs[0], true, 1, 64) && encode(&ta.tmap_runs[1], false, 1, 64) &&
+        encode(&ta.tmap_runs[2], true, 1, 16) && encode(&ta.tmap_runs[3], false, 1, 16)) {
       ta.use_tma = 1;
       ta.box_heads = heads;
     }
@@ -1710,10 +1780,13 @@ static cudaError_t launch_tc(const KArgs& a, const void* table, int table_rows, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_stage1_tc(const KArgs& a, const void* table, int table_rows, const Stage1Work& work,
+cudaError_t launch_stage1_tc(const KArgs& a, const void* table, int table_rows, const Stage1Work& work, bool any_rows,
                              cudaStream_t stream) {
-  return a.p.latent_dtype == WSVD_F16 ? launch_tc<tc::Cfg<true>>(a, table, table_rows, work, stream)
-                                      : launch_tc<tc::Cfg<false>>(a, table, table_rows, work, stream);
+  if (a.p.latent_dtype == WSVD_F16)
+    return any_rows ? launch_tc<tc::Cfg<true, true>>(a, table, table_rows, work, stream)
+                    : launch_tc<tc::Cfg<true, false>>(a, table, table_rows, work, stream);
+  return any_rows ? launch_tc<tc::Cfg<false, true>>(a, table, table_rows, work, stream)
+                  : launch_tc<tc::Cfg<false, false>>(a, table, table_rows, work, stream);
 }
 
 cudaError_t read_tc_status(unsigned int* out) {

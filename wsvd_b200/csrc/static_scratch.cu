@@ -50,8 +50,8 @@ extern "C" int wsvd_latent_decode_static(const WsvdLatentDecodeParams* p, void* 
   if (p->batch == 0) return WSVD_OK;
   size_t need = wsvd_latent_decode_workspace_bytes(p);
   WsvdLatentDecodeParams split;
-  if (need > (size_t)WSVD_STATIC_SCRATCH_BYTES && p->kernel == WSVD_KERNEL_AUTO && p->latent_dtype == WSVD_F16) {
-    // f16 latents: the warp-MMA kernel's fixed splits may fit where the balanced shares do not
+  if (need > (size_t)WSVD_STATIC_SCRATCH_BYTES && wsvd::tc_by_auto_only(p)) {
+    // the fixed splits of the kernels that such a block would run on otherwise may fit where the balanced shares do not
     split = *p;
     split.kernel = WSVD_KERNEL_MMA;
     const size_t less = wsvd_latent_decode_workspace_bytes(&split);
