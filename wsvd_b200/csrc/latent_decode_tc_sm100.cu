@@ -98,7 +98,7 @@ struct Cfg {
   static constexpr int kVSlots = ANY ? 1 : 2;      // tiles of V: the tile whose value MMAs are pending, and the next tile in flight
   static constexpr int kABufs = ANY ? 1 : 2;       // tiles of the position table
   static constexpr uint32_t kRawPitch = kRowBytes + 16;  // ANY: a row as fetched; 16 bytes more than a row: no bank conflicts
-  static constexpr int kWBufs = F16 ? 3 : 2;       // W accumulators of 128 columns (one pair of heads each)
+  static constexpr int kWBufs = 3;                 // W accumulators of 128 columns (one pair of heads each)
   // int8: 640 threads leave the compiler 96 registers a thread, and the two groups of warps re-balance them.
   // The pool is the CTA's own: what the control warpgroup hands back, (96 - 64) * 128, is exactly what the
   // epilogue warpgroups take, (104 - 96) * 512.  (A request the pool cannot satisfy would block for ever.)
@@ -113,14 +113,16 @@ struct Cfg {
   static constexpr uint32_t kUnitBytes = kG * kHeadBytes;    // a ring slot: one tile of K or V for the group's KV heads
   static constexpr uint32_t kBHalfBytes = kG * kRkMax * 128; // rows of 64 f16
   static constexpr uint32_t kPlaneBytes = F16 ? 512 : 256;   // per pair of warps: 32 tokens x 8 rows of digits
-  static constexpr uint32_t kTmemD = kWBufs * 128;           // first column of the value accumulators: 2 x 8 per (head, warp)
-  static_assert(kTmemD + kG * 64 <= kTmemCols, "tensor memory");
-  // Weights of the value MMA, relative to the warp's reference 2^my_ref.  int8 V: integers in four digits of 8
-  // bits, a weight of 1 is 2^32 - 256.  f16 V: three f16 terms, each 2^11 below the one before, a weight of 1 is 2^15.
-  static constexpr float kPlaneScale = F16 ? 32768.f : 4294967040.f;
-  // Tiles after which a warp goes over to its other accumulator in any case.  int8: 32 tokens add at most 2^20 to a
-  // digit sum of 31 bits.  f16: so that a sum in tensor memory is never more than 32 additions long.
-  static constexpr int kRenewTiles = F16 ? 16 : 1024;
+  static constexpr uint32_t kTmemD = kWBufs * 128;           // first column of the value accumulators
+  static constexpr uint32_t kDCols = F16 ? 16 : 8;           // per (head, warp): f16 has two of 8 columns
+  static_assert(kTmemD + kG * 4 * kDCols <= kTmemCols, "tensor memory");
+  // Weights of the value MMA.  int8 V: integers in three digits of 8 bits, relative to the largest of the warp's 32 tokens
+  // (a weight of 1 is 2^24 - 256), summed per tile.  f16 V: three f16 terms, each 2^11 below the one before, relative to the
+  // warp's reference 2^my_ref (a weight of 1 is 2^15), summed over tiles in tensor memory.
+  static constexpr float kPlaneScale = F16 ? 32768.f : 16776960.f;
+  // f16: tiles after which a warp goes over to its other accumulator in any case, so that a sum in tensor memory is never
+  // more than 32 additions long
+  static constexpr int kRenewTiles = 16;
 
   // shared-memory map (offsets from a 1024-byte aligned base)
   static constexpr uint32_t kOffB = 0;
@@ -129,7 +131,7 @@ struct Cfg {
   static constexpr uint32_t kOffK = kOffV + kVSlots * kUnitBytes;
   static constexpr uint32_t kOffPlanes = kOffK + (ANY ? 2 * kTile * kG * kRawPitch : kKSlots * kUnitBytes);
   static constexpr uint32_t kOffVRaw = kOffK + kTile * kG * kRawPitch;  // ANY
-  static constexpr uint32_t kOffRef = kOffPlanes + 2 * kG * kPlaneBytes;  // [head][tile parity][warp] reference that a warp left with this tile
+  static constexpr uint32_t kOffRef = kOffPlanes + 2 * kG * kPlaneBytes;  // [head][tile parity][warp] int8: reference of the tile's planes; f16: reference that a warp left with this tile
   static constexpr uint32_t kOffSum = kOffRef + kG * 2 * 4 * 4;           // [head][warp] (max z, denominator) at the end
   static constexpr uint32_t kOffMode = kOffSum + kG * 4 * 8;              // [4] how the K and V rows of a tile arrive (ring)
   static constexpr uint32_t kOffItem = kOffMode + 16;                     // [head][item parity] ItemState
@@ -236,6 +238,8 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
   asm volatile(
@@ -675,21 +679,21 @@ __device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, ui
         if (!ok) break;
         ++mine[j];
         tc_fence_after();
-        const uint32_t how = *value_modes<C>(sm, g);  // a byte per warp: which of its accumulators, added to or started
+        const uint32_t how = C::kF16 ? *value_modes<C>(sm, g) : 0u;  // a byte per warp: which of its accumulators, added to or started
         // copied rows sit at the head's KV head, gathered ones at the head itself
         const int sub = C::kAny || (mode[T & 3] & 1) ? g : (h0 + g) / gqa - h0 / gqa;
         const uint32_t v_at = v_lo + ((vslot * C::kUnitBytes + sub * C::kHeadBytes) >> 4);
-        const uint32_t d_tmem = tmem + C::kTmemD + 64 * g;
+        const uint32_t d_tmem = tmem + C::kTmemD + 4 * C::kDCols * g;
         if (issuer) {
 #pragma unroll
           for (int w4 = 0; w4 < 4; ++w4) {  // the 32 tokens of warp w4: 32 rows
-            const uint32_t d = d_tmem + 16 * w4 + ((how >> (8 * w4)) & 1) * 8, adds = (how >> (8 * w4)) & 2;
+            const uint32_t d = d_tmem + C::kDCols * w4 + ((how >> (8 * w4)) & 1) * 8;
             const uint32_t va = v_at + ((w4 * 32 * C::kRowBytes) >> 4), pa = p_lo + (((2 * g + (w4 >> 1)) * C::kPlaneBytes) >> 4);
             if constexpr (C::kF16) {  // 16 tokens an instruction
-              umma_f16(d, join64(va, v_hi), join64(pa, p_hi), idesc, adds);
+              umma_f16(d, join64(va, v_hi), join64(pa, p_hi), idesc, (how >> (8 * w4)) & 2);
               umma_f16(d, join64(va + (2048 >> 4), v_hi), join64(pa + (256 >> 4), p_hi), idesc, 1);
             } else {
-              umma_i8(d, join64(va, v_hi), join64(pa, p_hi), idesc, adds);
+              umma_i8(d, join64(va, v_hi), join64(pa, p_hi), idesc, 0);
             }
           }
           umma_commit(bar(C::kBarDFull + g));
@@ -780,7 +784,44 @@ __device__ __forceinline__ void build_pq(const TcArgs& ta, uint8_t* sm, int b, i
     }
   }
   const int64_t col = (int64_t)hk * 128;
-  if (wk_vec && wk_i8) {
+  if (!C::kF16 && !C::kAny && wk_vec && !wk_i8 && !interleaved) {
+    // Common case (int8 latents in whole 16-byte rows, f16 wk, half-split pairing): packed f16 arithmetic.  The operands are
+    // rounded to f16 for the MMA anyway; forming them with one extra f16 rounding of a
+    // product keeps the error of the scores within a few 1e-5.  This thread's chunk of 8
+    // frequencies is the same for its four ranks, so q is converted once.
+    const int ic = tid & 7;
+    __half2 qa[4], qb[4], nqa[4];
+    {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        qa[e] = __floats2half2_rn(qlo[2 * e], qlo[2 * e + 1]);
+        qb[e] = __floats2half2_rn(qhi[2 * e], qhi[2 * e + 1]);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) nqa[e] = __hneg2(qa[e]);
+    }
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int r = (tid + 128 * it) >> 3;
+      const uint32_t off = pq_off(g, r, ic);
+      uint4 u_lo = make_uint4(0u, 0u, 0u, 0u), u_hi = u_lo;
+      if (r < p.rank_k) {
+        u_lo = *reinterpret_cast<const uint4*>(sm + C::kOffB + off);
+        u_hi = *reinterpret_cast<const uint4*>(sm + C::kOffB + C::kBHalfBytes + off);
+      }
+      const __half2* ua = reinterpret_cast<const __half2*>(&u_lo);  // U[d = ic*8 .. +7]
+      const __half2* ub = reinterpret_cast<const __half2*>(&u_hi);  // U[64 + ic*8 .. +7]
+      __align__(16) __half2 pv[4];
+      __align__(16) __half2 qv[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        pv[e] = __hfma2(qa[e], ua[e], __hmul2(qb[e], ub[e]));   // P = q_i U_i + q_{i+64} U_{i+64}
+        qv[e] = __hfma2(nqa[e], ub[e], __hmul2(qb[e], ua[e]));  // Q = q_{i+64} U_i - q_i U_{i+64}
+      }
+      *reinterpret_cast<uint4*>(sm + C::kOffB + off) = *reinterpret_cast<const uint4*>(pv);
+      *reinterpret_cast<uint4*>(sm + C::kOffB + C::kBHalfBytes + off) = *reinterpret_cast<const uint4*>(qv);
+    }
+  } else if (wk_vec && wk_i8) {
     // int8 wk in vectors of eight; the columns' scales are this thread's for all four ranks.  fp32 throughout.
     const int ic = tid & 7;
     const __half* ws = reinterpret_cast<const __half*>(p.wk_scale) + col;
@@ -788,7 +829,7 @@ __device__ __forceinline__ void build_pq(const TcArgs& ta, uint8_t* sm, int b, i
     const uint4 s1v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 + 8 : 64 + ic * 8));
     const __half* s0h = reinterpret_cast<const __half*>(&s0v);
     const __half* s1h = reinterpret_cast<const __half*>(&s1v);
-#pragma unroll 1
+#pragma unroll 2
     for (int it = 0; it < 4; ++it) {
       const int r = (tid + 128 * it) >> 3;
       const uint32_t off = pq_off(g, r, ic);
@@ -826,7 +867,7 @@ __device__ __forceinline__ void build_pq(const TcArgs& ta, uint8_t* sm, int b, i
       *reinterpret_cast<uint4*>(sm + C::kOffB + C::kBHalfBytes + off) = *reinterpret_cast<const uint4*>(qv);
     }
   } else
-#pragma unroll 1
+#pragma unroll 2
   for (int it = 0; it < 4; ++it) {
     const int task = tid + 128 * it;
     const int r = task >> 3, ic = task & 7;  // rank, chunk of 8 frequencies
@@ -924,26 +965,31 @@ __device__ __forceinline__ void finish_head(const TcArgs& ta, uint8_t* sm, int g
     head_sync();
     if (verdict[0] == 0) return;
     const int64_t slot0 = ((int64_t)f.b * n_hg + f.hg + f.c_first) * C::kG + g;
-    // the first four partials (a head is rarely shared by more CTAs) are requested at once
-    float ls[4], mo[4];
+    // Eight partials at a time, their loads all in flight at once, each batch under a running maximum.  (A loop of one
+    // partial after another cost a round trip to L2 each: with 16 CTAs on a head, half of the smallest call's time.)
+    float m = -INFINITY, wsum = 0.f, osum = 0.f;
+    for (int i0 = 0; i0 < f.n_parts; i0 += 8) {
+      float ls[8], mo[8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      ls[i] = i < f.n_parts ? __ldcg(a.lse + slot0 + (int64_t)i * C::kG) : -INFINITY;
-      mo[i] = i < f.n_parts && d < Rv ? __ldcg(a.mid_o + (slot0 + (int64_t)i * C::kG) * Rv + d) : 0.f;
-    }
-    float m = fmaxf(fmaxf(ls[0], ls[1]), fmaxf(ls[2], ls[3]));
-    for (int i = 4; i < f.n_parts; ++i) m = fmaxf(m, __ldcg(a.lse + slot0 + (int64_t)i * C::kG));
-    float wsum = 0.f, osum = 0.f;
+      for (int i = 0; i < 8; ++i) {
+        const bool on = i0 + i < f.n_parts;
+        ls[i] = on ? __ldcg(a.lse + slot0 + (int64_t)(i0 + i) * C::kG) : -INFINITY;
+        mo[i] = on && d < Rv ? __ldcg(a.mid_o + (slot0 + (int64_t)(i0 + i) * C::kG) * Rv + d) : 0.f;
+      }
+      float m_new = m;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float w = ls[i] > -INFINITY ? __expf(ls[i] - m) : 0.f;
-      wsum += w;
-      osum = fmaf(w, mo[i], osum);
-    }
-    for (int i = 4; i < f.n_parts; ++i) {
-      const float w = __expf(__ldcg(a.lse + slot0 + (int64_t)i * C::kG) - m);
-      wsum += w;
-      if (d < Rv) osum = fmaf(w, __ldcg(a.mid_o + (slot0 + (int64_t)i * C::kG) * Rv + d), osum);
+      for (int i = 0; i < 8; ++i) m_new = fmaxf(m_new, ls[i]);
+      const float keep = m > -INFINITY ? __expf(m - m_new) : 0.f;
+      wsum *= keep;
+      osum *= keep;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (i0 + i >= f.n_parts) continue;
+        const float w = __expf(ls[i] - m_new);  // (a NaN stays one)
+        wsum += w;
+        osum = fmaf(w, mo[i], osum);
+      }
+      m = m_new;
     }
     if (d < Rv) o_row[d] = osum / wsum;
   }
@@ -1030,41 +1076,63 @@ __device__ __forceinline__ void shift_row(uint32_t (&w)[kWordsOut + 4], int skip
 }
 
 // One head's running sums over the tiles of an item, all in the log2 domain and fp32.
-//  - Denominator: l_lane, this lane's tokens, under the warp's reference m_run.  The reference follows the warp's
-//    maximum of z only when that has grown by more than kSlackZ: a weight may reach 2^kSlackZ, which fp32 does not mind.
-//  - Values: the sums of this warp's tokens stay in tensor memory, in integers relative to 2^my_ref, until a weight
-//    would no longer fit.  Then the warp goes over to its other accumulator with a new reference and leaves
-//    the old one to be folded into acc (rank 16*q4 + lane, lanes 0..15, all four warps' tokens, under big_m).
-//    New references leave kSlackY bits of room, so that a few per item are enough: folding every tile cost an
-//    eighth of the kernel's instructions.
+//  - Denominator: l_lane, this lane's tokens, under the warp's reference m_run: the warp's maximum of z (int8), or a value
+//    that follows it only when it has grown by more than kSlackZ (f16: a weight may reach 2^kSlackZ, which fp32 does not mind).
+//  - Values: acc, rank 16*q4 + lane (lanes 0..15), all four warps' tokens, under big_m.  int8: every tile's sums are folded
+//    in.  f16: the sums of a warp's tokens stay in tensor memory, relative to 2^my_ref, until a weight would no longer fit.
+//    Then the warp goes over to its other accumulator with a new reference and leaves the old one to be folded into
+//    acc.  New references leave kSlackY bits of room, so that a few per item are enough.
 struct HeadSums {
   float m_run, l_lane;
-  float my_ref, scale;  // scale: 2^(m_run - my_ref) * kPlaneScale of the Cfg
   float big_m, acc;
-  uint32_t bufs;        // bit w4: the accumulator warp w4 of the head is using
+  float my_ref, scale;  // f16: scale = 2^(m_run - my_ref) * kPlaneScale
+  uint32_t bufs;        // f16, bit w4: the accumulator warp w4 of the head is using
 };
 constexpr float kSlackZ = 8.f;
 constexpr int kSlackY = 3;
 
-// Fold in one accumulator of warp w4 of the head: D[rank][0..3] are its four digit-plane sums, relative to 2^ref.
+// int8: fold in the value sums of the head's tile number tp: D[rank][8*w + 0..2] are the three digit-plane sums over
+// the 32 tokens of warp w, whose weights were taken relative to refs[tp & 1][w].
+template <class C>
+__device__ __forceinline__ void fold_tile(HeadSums& hs, uint32_t d_addr, const float* refs, uint32_t tp) {
+  uint32_t d[4][4];
+#pragma unroll
+  for (int w4 = 0; w4 < 4; ++w4) tmem_ld4(d_addr + 8 * w4 + 3 * (w4 & 1), d[w4]);
+  const float4 rf = *reinterpret_cast<const float4*>(refs + (tp & 1) * 4);
+  const float ref[4] = {rf.x, rf.y, rf.z, rf.w};
+#pragma unroll
+  for (int w4 = 0; w4 < 4; ++w4) tmem_wait_ld(d[w4]);
+  float m_new = hs.big_m;
+#pragma unroll
+  for (int w4 = 0; w4 < 4; ++w4) m_new = fmaxf(m_new, ref[w4]);
+  if (m_new > -INFINITY) {
+    hs.acc *= fast_exp2(hs.big_m - m_new);  // big_m = -inf -> factor 0
+#pragma unroll
+    for (int w4 = 0; w4 < 4; ++w4) {
+      if (ref[w4] > -INFINITY) {  // (a warp without tokens in this tile has reference -inf)
+        // the two low digit sums are combined as integers (|d| <= 32 * 255 * 128 < 2^21)
+        const float v = fmaf((float)(int32_t)d[w4][2], 65536.f, (float)((int32_t)d[w4][1] * 256 + (int32_t)d[w4][0]));
+        hs.acc = fmaf(v, fast_exp2(ref[w4] - m_new) * (1.f / C::kPlaneScale), hs.acc);
+      }
+    }
+    hs.big_m = m_new;
+  }
+}
+
+// f16: fold in one accumulator of warp w4 of the head: D[rank][0..2] are its three sums, relative to 2^ref.
 template <class C>
 __device__ __forceinline__ void fold_values(HeadSums& hs, uint32_t d_addr, int w4, uint32_t buf, float ref) {
   uint32_t d[4];
   tmem_ld4(d_addr + 16 * w4 + 8 * buf + 4 * (w4 & 1), d);
   tmem_wait_ld(d);
   const float m_new = fmaxf(hs.big_m, ref);
-  float v;
-  if constexpr (C::kF16) {
-    v = fmaf(__uint_as_float(d[2]), 2.384185791015625e-7f, fmaf(__uint_as_float(d[1]), 4.8828125e-4f, __uint_as_float(d[0])));  // 2^-22, 2^-11
-    if (isinf(__uint_as_float(d[0]))) v = __uint_as_float(d[0]);  // an infinite V times a lower term of zero is no NaN
-  } else {
-    v = fmaf((float)(int32_t)d[3], 16777216.f, fmaf((float)(int32_t)d[2], 65536.f, fmaf((float)(int32_t)d[1], 256.f, (float)(int32_t)d[0])));
-  }
+  float v = fmaf(__uint_as_float(d[2]), 2.384185791015625e-7f, fmaf(__uint_as_float(d[1]), 4.8828125e-4f, __uint_as_float(d[0])));  // 2^-22, 2^-11
+  if (isinf(__uint_as_float(d[0]))) v = __uint_as_float(d[0]);  // an infinite V times a lower term of zero is no NaN
   hs.acc = fmaf(v, fast_exp2(ref - m_new) * (1.f / C::kPlaneScale), hs.acc * fast_exp2(hs.big_m - m_new));
   hs.big_m = m_new;
 }
 
-// What the head's warps have left behind with tile number tp (see HeadSums).
+// f16: what the head's warps have left behind with tile number tp (see HeadSums).
 template <class C>
 __device__ __forceinline__ void fold_left(HeadSums& hs, uint32_t d_addr, const float* refs, uint32_t tp) {
   const float4 rf = *reinterpret_cast<const float4*>(refs + (tp & 1) * 4);
@@ -1093,14 +1161,14 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + C::kOffTmemSlot);
   const volatile int* st = item_state<C>(sm, g, item);
   const volatile int* mode = reinterpret_cast<const volatile int*>(sm + C::kOffMode);
-  float* refs = reinterpret_cast<float*>(sm + C::kOffRef) + g * 8;  // [tile parity][warp]: reference left behind, or kNone
+  float* refs = reinterpret_cast<float*>(sm + C::kOffRef) + g * 8;  // [tile parity][warp], see Cfg
   // Digit planes: the two warps of half a tile share one 8-row block (the MMA's B operand has 8
-  // rows): rows 0..3 hold the even warp's digits, rows 4..7 the odd warp's.  Each warp's MMA reads
-  // the whole block, so its columns 4..7 (or 0..3) are the other warp's weights times this warp's
-  // V rows: garbage that nobody reads.
-  const uint32_t my_planes = sbase + C::kOffPlanes + (2 * g + (q4 >> 1)) * C::kPlaneBytes + (q4 & 1) * 64 +
+  // rows): rows 0..2 hold the even warp's digits, rows 3..5 (f16: 4..6) the odd warp's.  Each warp's MMA
+  // reads the whole block, so its other columns are the other warp's weights times this warp's V rows:
+  // garbage that nobody reads.  The remaining rows are never written.
+  const uint32_t my_planes = sbase + C::kOffPlanes + (2 * g + (q4 >> 1)) * C::kPlaneBytes + (q4 & 1) * (C::kF16 ? 64 : 48) +
                              (C::kF16 ? (lane >> 3) * 128 + (lane & 7) * 2 : (lane >> 4) * 128 + (lane & 15));
-  const uint32_t d_addr = tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 64 * g;
+  const uint32_t d_addr = tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 4 * C::kDCols * g;
   const int h0 = st[kItHg] * C::kG, G = min(C::kG, p.n_q_heads - h0), npairs = (G + 1) >> 1;
   bool ok = true;
   uint32_t own_buf = 0;  // this warp's accumulator
@@ -1147,7 +1215,9 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
   bool gathered = false; // the tile before was
   if constexpr (C::kAny) {
     fetch_k(k_raw, slot_c);
+    cp_async_commit();
     fetch_v(v_raw, slot_c);
+    cp_async_commit();
   }
   for (int t = 0; t < ntiles && ok; ++t) {
     const int s = lo + t * kTile + row;
@@ -1169,8 +1239,9 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     uint4 kreg[kChunks];
     bool gather = false;
     if constexpr (C::kAny) {
-      // the rows of this tile have been on their way for a tile; the next tile's K rows take their place
-      cp_async_wait_all();
+      // the K rows of this tile have been on their way for a tile (its V rows may still be); those of the next tile
+      // take their place
+      cp_async_wait_but_one();
       __syncwarp();
       uint32_t w[kWords + 4];
       read_raw(w, k_raw, k_base, p.k_stride_t * kEsize, slot_t);
@@ -1178,6 +1249,7 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       for (int c = 0; c < kChunks; ++c) kreg[c] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
       __syncwarp();
       if (lo + (t + 1) * kTile < hi) fetch_k(k_raw, slot_c);
+      cp_async_commit();
     } else {
       const uint32_t kslot = Tt % C::kKSlots;
       ok = mbar_wait(bar(C::kBarKFull + kslot), (Tt / C::kKSlots) & 1);
@@ -1270,44 +1342,61 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
 
     // ---- softmax weights under the warp's reference, denominator (fp32, by the owner threads)
     const float mz_w = warp_max_redux(z);
-    bool renew = mz_w > hs.m_run + kSlackZ;
-    if (renew) {
-      hs.l_lane *= fast_exp2(hs.m_run - mz_w);
-      hs.m_run = mz_w;
-    }
-    const float e = fast_exp2(z - hs.m_run);  // masked tokens: 2^-inf = 0
-    hs.l_lane += e;
-    const float pv = C::kF16 ? e : e * sv, pv_w = warp_max_redux(pv);
-    // ---- does every weight fit under the reference of the value sums?
-    float left = kNone;
-    uint32_t adds = t > 0 ? 2u : 0u;
-    renew = renew || pv_w * hs.scale > C::kPlaneScale || (t & (C::kRenewTiles - 1)) == C::kRenewTiles - 1;
-    if (renew) {
-      left = hs.my_ref;
-      if (left > kNone) {
-        adds = 0u;
-        own_buf ^= 1u;
+    float wgt, left;        // what the value MMA's operand is made of; what goes to refs
+    uint32_t how = 0;       // f16: accumulator and whether to add to it
+    if constexpr (C::kF16) {
+      bool renew = mz_w > hs.m_run + kSlackZ;
+      if (renew) {
+        hs.l_lane *= fast_exp2(hs.m_run - mz_w);
+        hs.m_run = mz_w;
       }
-      // 2^k, the power of two that leaves the largest weight kSlackY bits of room (weights 2^-60 below the largest
-      // of the softmax do not show in the result)
-      const int k = min(max((int)((__float_as_uint(pv_w) >> 23) & 0xff) - 126 + kSlackY, -60), 100);
-      if (pv_w == INFINITY) hs.l_lane = __int_as_float(0x7fc00000);  // an infinite V scale: the result is NaN
-      hs.my_ref = hs.m_run + (float)k;
-      hs.scale = C::kPlaneScale * __uint_as_float((uint32_t)(127 - k) << 23);
+      const float e = fast_exp2(z - hs.m_run);  // masked tokens: 2^-inf = 0
+      hs.l_lane += e;
+      const float e_w = warp_max_redux(e);
+      // does every weight fit under the reference of the value sums?
+      left = kNone;
+      how = t > 0 ? 2u : 0u;
+      renew = renew || e_w * hs.scale > C::kPlaneScale || (t & (C::kRenewTiles - 1)) == C::kRenewTiles - 1;
+      if (renew) {
+        left = hs.my_ref;
+        if (left > kNone) {
+          how = 0u;
+          own_buf ^= 1u;
+        }
+        // 2^k, the power of two that leaves the largest weight kSlackY bits of room (weights 2^-60 below the largest
+        // of the softmax do not show in the result)
+        const int k = max((int)((__float_as_uint(e_w) >> 23) & 0xff) - 126 + kSlackY, -60);
+        hs.my_ref = hs.m_run + (float)k;
+        hs.scale = C::kPlaneScale * __uint_as_float((uint32_t)(127 - k) << 23);
+      }
+      how |= own_buf;
+      wgt = e * hs.scale;
+    } else {
+      const float y = valid ? z + fast_log2(sv) : -INFINITY;  // log2(0) = -inf: a zero scale drops the token's value
+      left = warp_max_redux(y);
+      if (mz_w > -INFINITY) {
+        const float m_new = fmaxf(hs.m_run, mz_w);
+        hs.l_lane = fmaf(hs.l_lane, fast_exp2(hs.m_run - m_new), fast_exp2(z - m_new));  // 2^-inf = 0: m_run = -inf, masked tokens
+        hs.m_run = m_new;
+      }
+      wgt = (y > -INFINITY ? fast_exp2(y - left) : 0.f) * C::kPlaneScale;  // <= kPlaneScale
     }
 
-    // ---- the previous tile's value MMAs are complete: fold in what the head's warps left behind with it.  This
+    // ---- the previous tile's value MMAs are complete: fold in its sums, or what the head's warps left behind.  This
     //      also orders this warp's reads of D and of the references (and, through the MMAs' completion,
     //      the MMAs' reads of its digit planes and V rows) before those of this tile are written.
     if (t > 0) {
       ok = mbar_wait(bar(C::kBarDFull + g), (mt - 1) & 1);
       if (!ok) break;
       tc_fence_after();
-      fold_left<C>(hs, d_addr, refs, mt - 1);
+      if constexpr (C::kF16) fold_left<C>(hs, d_addr, refs, mt - 1);
+      else fold_tile<C>(hs, d_addr, refs, mt - 1);
     }
     const uint32_t vrow = sbase + C::kOffV + (Tt % C::kVSlots) * C::kUnitBytes + (C::kAny || gather ? g : sub) * C::kHeadBytes;
     if constexpr (C::kAny) {
-      // this head's own region: its value MMAs of the tile before are complete (and its V rows came with its K rows)
+      // this head's own region: its value MMAs of the tile before are complete
+      cp_async_wait_but_one();  // all but the next tile's K rows
+      __syncwarp();
       uint32_t w[kWords + 4];
       read_raw(w, v_raw, v_base, p.v_stride_t * kEsize, slot_t);
 #pragma unroll
@@ -1317,6 +1406,7 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
                      : "memory");
       __syncwarp();
       if (lo + (t + 1) * kTile < hi) fetch_v(v_raw, slot_c);
+      cp_async_commit();
     } else {
       if (gather) {
         cp_async_wait_all();
@@ -1335,10 +1425,9 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       }
     }
 
-    // ---- this token's weight for the value MMA, relative to the warp's reference: four 8-bit digits, or three f16
-    //      terms (11 bits each, every remainder is exact: nothing that fp32 holds of the weight is lost)
+    // ---- this token's weight for the value MMA: three 8-bit digits, or three f16 terms (11 bits each, every remainder
+    //      is exact: nothing that fp32 holds of the weight is lost)
     if constexpr (C::kF16) {
-      const float wgt = pv * hs.scale;
       const __half t0 = __float2half_rn(wgt);
       const float r1 = (wgt - __half2float(t0)) * 2048.f;
       const __half t1 = __float2half_rn(r1);
@@ -1347,17 +1436,16 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       asm volatile("st.shared.u16 [%0], %1;" ::"r"(my_planes + 16), "h"(__half_as_ushort(t1)) : "memory");
       asm volatile("st.shared.u16 [%0], %1;" ::"r"(my_planes + 32), "h"(__half_as_ushort(t2)) : "memory");
     } else {
-      const uint32_t nq = __float2uint_rn(pv * hs.scale);
+      const uint32_t nq = __float2uint_rn(wgt);
       asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes), "r"(nq) : "memory");
       asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 16), "r"(nq >> 8) : "memory");
       asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 32), "r"(nq >> 16) : "memory");
-      asm volatile("st.shared.u8 [%0], %1;" ::"r"(my_planes + 48), "r"(nq >> 24) : "memory");
     }
     fence_proxy_async();
     tc_fence_before();
     if (lane == 0) {
       refs[(mt & 1) * 4 + q4] = left;
-      reinterpret_cast<volatile uint8_t*>(value_modes<C>(sm, g))[q4] = (uint8_t)(own_buf | adds);
+      if constexpr (C::kF16) reinterpret_cast<volatile uint8_t*>(value_modes<C>(sm, g))[q4] = (uint8_t)how;
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(C::kBarPlanes + g));
@@ -1410,7 +1498,8 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
     if (pending) finish_head<C>(ta, sm, g, state(item + 1), seen);  // the item before, while the first score MMAs of this one run
     pending = false;
 
-    HeadSums hs = {kNone, 0.f, kNone, 0.f, kNone, 0.f, 0u};
+    const float none = C::kF16 ? kNone : -INFINITY;
+    HeadSums hs = {none, 0.f, none, 0.f, kNone, 0.f, 0u};
     if (active && ok) ok = run_tiles<C>(ta, sm, item, hs);
 
     // ---- the item's end.  What the next item needs is requested before the last value sums are waited for.
@@ -1435,27 +1524,32 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
     if (active) {
       const uint32_t last = st[kItMine] + st[kItTiles] - 1;  // count of the head's last tile
       const int b = st[kItB], hg = st[kItHg], h = h0 + g;
-      const uint32_t d_addr = tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 64 * g;
+      const uint32_t d_addr = tmem + ((uint32_t)(q4 * 32) << 16) + C::kTmemD + 4 * C::kDCols * g;
       float* refs = reinterpret_cast<float*>(sm + C::kOffRef) + g * 8;
       if (ok) {
         ok = warp_wait(bar(C::kBarDFull + g), last & 1);
         if (ok) {
           tc_fence_after();
-          fold_left<C>(hs, d_addr, refs, last);
+          if constexpr (C::kF16) {
+            fold_left<C>(hs, d_addr, refs, last);
+          } else {
+            fold_tile<C>(hs, d_addr, refs, last);
+            tc_fence_before();
+          }
         }
       }
       if (!ok) atomicMax(&g_status, (unsigned)kTimeoutEpilogue);
 
-      // ---- the head's denominator: the four warps' (reference, sum) pairs under a common maximum; with them the
+      // ---- the head's denominator: the four warps' (reference, sum) pairs under a common maximum; with them, f16, the
       //      references of the value accumulators in use
       const float l_w = warp_sum(hs.l_lane);
       float2* sums = reinterpret_cast<float2*>(sm + C::kOffSum) + g * 4;
       if (lane == 0) {
         sums[q4] = make_float2(hs.m_run, l_w);
-        refs[((last + 1) & 1) * 4 + q4] = hs.my_ref;
+        if constexpr (C::kF16) refs[((last + 1) & 1) * 4 + q4] = hs.my_ref;
       }
       head_sync();
-      if (ok) {
+      if (C::kF16 && ok) {
         const float4 rf = *reinterpret_cast<const float4*>(refs + ((last + 1) & 1) * 4);
         if (rf.x > kNone) fold_values<C>(hs, d_addr, 0, hs.bufs & 1, rf.x);
         if (rf.y > kNone) fold_values<C>(hs, d_addr, 1, (hs.bufs >> 1) & 1, rf.y);
@@ -1463,19 +1557,21 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
         if (rf.w > kNone) fold_values<C>(hs, d_addr, 3, (hs.bufs >> 3) & 1, rf.w);
         tc_fence_before();
       }
-      float m_all = kNone;
+      float m_all = none;
 #pragma unroll
       for (int w4 = 0; w4 < 4; ++w4) m_all = fmaxf(m_all, sums[w4].x);
-      float l_tot = 0.f;  // (a NaN in any warp's sum stays)
+      float l_tot = 0.f;  // (f16: a NaN in any warp's sum stays)
 #pragma unroll
-      for (int w4 = 0; w4 < 4; ++w4) l_tot = fmaf(sums[w4].y, fast_exp2(sums[w4].x - m_all), l_tot);
+      for (int w4 = 0; w4 < 4; ++w4)
+        if (C::kF16 || sums[w4].x > -INFINITY) l_tot = fmaf(sums[w4].y, fast_exp2(sums[w4].x - m_all), l_tot);
       const int64_t slot = balanced ? ((int64_t)b * n_hg + hg + blockIdx.x) * C::kG + g
                                     : ((int64_t)b * p.n_q_heads + h) * a.n_splits + blockIdx.x % a.n_splits;
       const int r = 16 * q4 + lane;
       // sum_s 2^z sv Lv / sum_s 2^z  =  acc * 2^(big_m - m_all) / l
       // (after a wait that timed out the item's result is poisoned: NaN here propagates through the
       // merge into the output row, so a time-out cannot pass for a valid result)
-      const float o = !ok ? __int_as_float(0x7fc00000) : (hs.big_m > kNone ? hs.acc * fast_exp2(hs.big_m - m_all) : 0.f) / l_tot;
+      const float sum = hs.big_m > none ? hs.acc * fast_exp2(hs.big_m - m_all) : 0.f;
+      const float o = !ok ? __int_as_float(0x7fc00000) : C::kF16 || hs.big_m > none ? sum / l_tot : 0.f;
       if (!fused || n_parts > 1) {
         if (lane < 16 && r < Rv) a.mid_o[slot * Rv + r] = o;
         // natural-log lse, as the merge kernel expects (stage1.py:216)
@@ -1519,9 +1615,18 @@ __global__ void __launch_bounds__(C::kThreads, 1) stage1_tc_kernel(const __grid_
     const int n = i < p.batch ? p.b_seq_len[i] : 0;
     return n > 0 ? (n + kTile - 1) / kTile : 0;
   };
-  int mine = 0;  // balanced mode: tiles of the sequences this thread counts (requested before the set-up below)
-  if (balanced)
+  // Balanced mode.  Up to 128 sequences: every warp works the shares out for itself, lane l from the lengths of sequences
+  // 4l..4l+3 (requested here, before the set-up below).  More: block-wide sums.
+  const bool by_warp = balanced && p.batch <= 128;
+  int len4[4] = {0, 0, 0, 0};
+  int mine = 0;
+  if (by_warp) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) len4[j] = 4 * lane + j < p.batch ? p.b_seq_len[4 * lane + j] : 0;
+    if (4 * lane < p.batch) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.b_req_idx + 4 * lane));
+  } else if (balanced) {
     for (int i = threadIdx.x; i < p.batch; i += C::kThreads) mine += tiles_of(i);
+  }
 
   // ---- once per CTA: tensor memory, barriers, descriptor prefetch
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + C::kOffTmemSlot);
@@ -1550,7 +1655,51 @@ __global__ void __launch_bounds__(C::kThreads, 1) stage1_tc_kernel(const __grid_
   }
 
   Share sh = {};
-  if (balanced) {
+  if (by_warp) {
+    int tiles[4], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      tiles[j] = len4[j] > 0 ? (len4[j] + kTile - 1) / kTile : 0;
+      sum += tiles[j];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    const int all_tiles = __shfl_sync(0xffffffffu, incl, 31);
+    sh.total = (int64_t)all_tiles * n_hg;
+    sh.shares = (int)min((int64_t)gridDim.x, sh.total);
+    if ((int)blockIdx.x < sh.shares) {
+      const int64_t begin = share_begin(blockIdx.x, sh.total, sh.shares);
+      sh.tiles_left = (int)(share_begin(blockIdx.x + 1, sh.total, sh.shares) - begin);
+      // the sequence that holds tile begin / n_hg of the batch (a sequence takes n_hg entries per tile)
+      const int at = (begin >> 32) == 0 ? (int)((uint32_t)begin / (uint32_t)n_hg) : (int)(begin / n_hg);
+      int excl = incl - sum, found = -1, before = 0, tiles_b = 1;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (at >= excl && at < excl + tiles[j]) found = 4 * lane + j, before = excl, tiles_b = tiles[j];
+        excl += tiles[j];
+      }
+      const int src = __ffs(__ballot_sync(0xffffffffu, found >= 0)) - 1;
+      sh.b = __shfl_sync(0xffffffffu, found, src);
+      sh.before_b = __shfl_sync(0xffffffffu, before, src);
+      tiles_b = __shfl_sync(0xffffffffu, tiles_b, src);
+      const int rem = (int)(begin - (int64_t)sh.before_b * n_hg);
+      sh.hg = rem / tiles_b;
+      sh.t_first = rem % tiles_b;
+    }
+    if (blockIdx.x == 0 && warp == 0 && ta.prefix_out != nullptr) {
+      int excl = incl - sum;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (4 * lane + j < p.batch) ta.prefix_out[4 * lane + j] = excl;
+        excl += tiles[j];
+      }
+      if (lane == 0) ta.prefix_out[p.batch] = all_tiles, ta.prefix_out[p.batch + 1] = sh.shares;
+    }
+  } else if (balanced) {
     // Tiles per sequence -> block-wide sums -> this CTA's share [begin, end) of the tile list and the
     // (sequence, head group, tile) it starts at.  Scratch: the reference/sum area, unused until the
     // first tile.
@@ -1611,23 +1760,23 @@ __global__ void __launch_bounds__(C::kThreads, 1) stage1_tc_kernel(const __grid_
         sh.t_first = rem % tiles_b;
       }
     }
-    // sequences without tokens belong to no share: their output rows are zeros
-    if (fused) {
-      const int n_out = p.wv != nullptr ? p.head_dim : p.rank_v;
-      for (int bb = blockIdx.x; bb < p.batch; bb += gridDim.x) {
-        if (p.b_seq_len[bb] > 0) continue;
-        if (ta.has_peers) {
-          for (int i = threadIdx.x; i < p.n_q_heads * n_out * ta.peers.n_peers; i += C::kThreads) {
-            const int peer = i / (p.n_q_heads * n_out), j = i % (p.n_q_heads * n_out);
-            ta.peers.out[peer][(int64_t)bb * ta.peers.out_stride_b +
-                               (int64_t)(j / n_out + ta.peers.head_offset) * ta.peers.out_stride_h + j % n_out] =
-                __float2half_rn(0.f);
-          }
-        } else {
-          __half* orow = reinterpret_cast<__half*>(p.out) + (int64_t)bb * p.out_stride_b;
-          for (int i = threadIdx.x; i < p.n_q_heads * n_out; i += C::kThreads)
-            orow[(int64_t)(i / n_out) * p.out_stride_h + i % n_out] = __float2half_rn(0.f);
+  }
+  // sequences without tokens belong to no share: their output rows are zeros
+  if (fused) {
+    const int n_out = p.wv != nullptr ? p.head_dim : p.rank_v;
+    for (int bb = blockIdx.x; bb < p.batch; bb += gridDim.x) {
+      if (p.b_seq_len[bb] > 0) continue;
+      if (ta.has_peers) {
+        for (int i = threadIdx.x; i < p.n_q_heads * n_out * ta.peers.n_peers; i += C::kThreads) {
+          const int peer = i / (p.n_q_heads * n_out), j = i % (p.n_q_heads * n_out);
+          ta.peers.out[peer][(int64_t)bb * ta.peers.out_stride_b +
+                             (int64_t)(j / n_out + ta.peers.head_offset) * ta.peers.out_stride_h + j % n_out] =
+              __float2half_rn(0.f);
         }
+      } else {
+        __half* orow = reinterpret_cast<__half*>(p.out) + (int64_t)bb * p.out_stride_b;
+        for (int i = threadIdx.x; i < p.n_q_heads * n_out; i += C::kThreads)
+          orow[(int64_t)(i / n_out) * p.out_stride_h + i % n_out] = __float2half_rn(0.f);
       }
     }
   }
