@@ -156,9 +156,11 @@ void plan(const WsvdLatentDecodeParams* p, int* split_len, int* n_splits) {
 }
 
 void fill_args(const WsvdLatentDecodeParams* p, float* mid_o, float* lse, int split_len, int n_splits,
-               wsvd::KArgs* a) {
+               wsvd::KArgs* a, bool with_freq = true) {
   a->p = *p;
-  const int h2 = p->head_dim / 2;
+  // The frequencies, for the kernels that read them (table builders, generic kernel): sixty-four pow() are a
+  // third of a small call's time on the host, and a decode step with the caller's table needs none of them.
+  const int h2 = with_freq ? p->head_dim / 2 : 0;
   for (int i = 0; i < wsvd::kMaxHalfDim; ++i)
     a->inv_freq[i] = i < h2 ? (float)(1.0 / pow((double)p->theta, (2.0 * i) / (double)p->head_dim)) : 0.f;
   a->mid_o = mid_o;
@@ -395,7 +397,7 @@ static int decode_impl(const WsvdLatentDecodeParams* p, const WsvdPeerSet* peers
   float* mid_o = reinterpret_cast<float*>(ws);
   float* lse = mid_o + l.slots * p->rank_v;
   wsvd::KArgs a;
-  fill_args(p, mid_o, lse, sl, ns, &a);
+  fill_args(p, mid_o, lse, sl, ns, &a, !(balanced_mode(p) && p->rope_table));
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   void* scratch_table = l.table_bytes ? ws + l.table_off : nullptr;
   wsvd::PartialIndex where = {nullptr, 0, ns, sl, balanced_group(p)};

@@ -67,6 +67,8 @@
 #include <cuda.h>
 #include <string.h>
 
+#include <atomic>
+
 #include "common.cuh"
 
 namespace wsvd {
@@ -1876,6 +1878,22 @@ bool encode_table(CUtensorMap* map, const void* table, int rows) {
 
 }  // namespace tc
 
+namespace tc {
+// The kernel's shared-memory size is an attribute of the function on a device: set once per device and process.  (Two
+// threads that come first may both set it; a device past the array sets it on every call.)
+template <class C>
+cudaError_t allow_smem() {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 64 && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+  e = cudaFuncSetAttribute(stage1_tc_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
+  if (e == cudaSuccess && dev < 64) done[dev].store(true, std::memory_order_release);
+  return e;
+}
+}  // namespace tc
+
 size_t rope_table_bytes(int rows) { return (size_t)rows * 256; }
 
 cudaError_t launch_rope_table(void* table, int rows, const KArgs& a, cudaStream_t stream) {
@@ -1886,8 +1904,7 @@ cudaError_t launch_rope_table(void* table, int rows, const KArgs& a, cudaStream_
 
 template <class C>
 static cudaError_t launch_tc(const KArgs& a, const void* table, int table_rows, const Stage1Work& work, cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(tc::stage1_tc_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)C::kSmemBytes);
+  cudaError_t e = tc::allow_smem<C>();
   if (e != cudaSuccess) return e;
   tc::TcArgs ta;
   ta.k = a;

@@ -6,6 +6,7 @@ wrappers assert (efficiency/kernel/flash_int8_latent_per_head_decoding_rope_stag
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from typing import Callable, Optional, Tuple
 
@@ -29,14 +30,29 @@ def _need(cond: bool, msg: str, exc=ValueError):
 
 
 def _cuda_tensor(name, t, dtypes, ndim, inner_contiguous=True):
-    _need(isinstance(t, torch.Tensor), f"{name} must be a torch.Tensor", TypeError)
-    _need(t.is_cuda, f"{name} must be a CUDA tensor (no CPU path exists)")
-    _need(t.dtype in dtypes, f"{name} has dtype {t.dtype}, expected one of {dtypes}", TypeError)
-    _need(t.dim() == ndim, f"{name} must have {ndim} dims, got {tuple(t.shape)}")
-    _need(not inner_contiguous or t.numel() == 0 or t.stride(-1) == 1,
-          f"{name}: innermost dimension must be contiguous")
+    # (the messages are formatted only when they are needed: formatting them was most of a small call's host time)
+    if not isinstance(t, torch.Tensor):
+        raise TypeError(f"{name} must be a torch.Tensor")
+    if not t.is_cuda:
+        raise ValueError(f"{name} must be a CUDA tensor (no CPU path exists)")
+    if t.dtype not in dtypes:
+        raise TypeError(f"{name} has dtype {t.dtype}, expected one of {dtypes}")
+    if t.dim() != ndim:
+        raise ValueError(f"{name} must have {ndim} dims, got {tuple(t.shape)}")
+    if inner_contiguous and t.stride(-1) != 1 and t.numel() != 0:
+        raise ValueError(f"{name}: innermost dimension must be contiguous")
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def _on_device(device):
+    """Context in which `device` is the current one; entered only where it is not already."""
+    index = device.index
+    return _HERE if index is None or index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+_HERE = contextlib.nullcontext()
 _TABLES = {}
 _RETIRED_TABLES = []  # superseded tables stay allocated: cached argument blocks and captured graphs may point at them
 _CALLS = {}
@@ -55,7 +71,7 @@ def rope_table(device, positions: int, head_dim: int = 128, theta: float = 10000
     can order itself behind it.  A table that is replaced by a larger one is never freed:
     argument blocks handed out earlier, and CUDA graphs captured with them, keep pointing
     at memory that still holds a valid (shorter) table."""
-    dev = torch.device(device)
+    dev = device if isinstance(device, torch.device) else torch.device(device)
     key = (dev.index if dev.index is not None else torch.cuda.current_device(), float(theta), int(head_dim))
     have = _TABLES.get(key)
     if have is not None and have[1] >= positions:
@@ -208,8 +224,11 @@ def workspace_bytes(p: LatentDecodeParams) -> int:
 
 
 def _stream(stream) -> ctypes.c_void_p:
-    s = torch.cuda.current_stream() if stream is None else stream
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
+    if _raw_stream is not None:  # the handle without building a Stream object around it
+        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def _cached_params(tag, q3, infer_state, latent_k, k_scale, latent_v, v_scale, wk, wk_scale, wv, pos_offset, theta,
@@ -249,7 +268,6 @@ def _cached_params(tag, q3, infer_state, latent_k, k_scale, latent_v, v_scale, w
     return p, need
 
 
-@torch.no_grad()
 def latent_decode(
     q, infer_state, latent_k, k_scale, latent_v, v_scale, wk, wk_scale=None, *, wv=None, out=None,
     workspace: Optional[torch.Tensor] = None, alloc_tensor_func: Callable = torch.empty, pos_offset=None,
@@ -267,14 +285,15 @@ def latent_decode(
         out = alloc_tensor_func((B, p.n_q_heads, out_w), dtype=q.dtype, device=q.device)
     else:
         _cuda_tensor("out", out, (torch.float16,), 3)
-        _need(tuple(out.shape) == (B, p.n_q_heads, out_w), f"out must be {(B, p.n_q_heads, out_w)}")
+        if tuple(out.shape) != (B, p.n_q_heads, out_w):
+            raise ValueError(f"out must be {(B, p.n_q_heads, out_w)}")
     p.out, p.out_stride_b, p.out_stride_h = out.data_ptr(), out.stride(0), out.stride(1)
     if workspace is None:
         workspace = alloc_tensor_func(((need + 3) // 4,), dtype=torch.float32, device=q.device)
     else:
         _need(workspace.is_cuda and workspace.is_contiguous(), "workspace must be a contiguous CUDA tensor")
     have = workspace.numel() * workspace.element_size()
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         check(_lib.lib().wsvd_latent_decode(ctypes.byref(p), _ptr(workspace), have, _stream(stream)),
               "wsvd_latent_decode")
     return out
@@ -295,7 +314,7 @@ def latent_decode_gather(q, infer_state, latent_k, k_scale, latent_v, v_scale, w
     if workspace is None:
         workspace = torch.empty(((need + 3) // 4,), dtype=torch.float32, device=q.device)
     have = workspace.numel() * workspace.element_size()
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         check(_lib.lib().wsvd_latent_decode_gather(ctypes.byref(p), ctypes.byref(peers), _ptr(workspace), have,
                                                    _stream(stream)), "wsvd_latent_decode_gather")
 
@@ -344,7 +363,6 @@ def decode_stage2(mid_out, mid_out_lse, b_seq_len, out, block_seq, *, wv=None, n
             B, Hq, ns, W, int(block_seq), _ptr(wv), wv_stride, hkv, head_dim, _stream(stream)), "wsvd_decode_stage2")
 
 
-@torch.no_grad()
 def dense_decode(q, infer_state, cache_k, cache_v, out=None, alloc_tensor_func: Callable = torch.empty,
                  workspace=None, split_len=0, stream=None):
     """Dense f16 flash-decoding baseline: q [B,Hq,D], caches [T,Hkv,D] f16 -> [B,Hq,D] f16."""
@@ -357,7 +375,8 @@ def dense_decode(q, infer_state, cache_k, cache_v, out=None, alloc_tensor_func: 
     Hkv = cache_k.shape[1]
     _need(cache_k.shape[2] == D and cache_v.shape[2] == D, "q and K/V disagree on head_dim")
     _need(cache_v.shape[1] == Hkv and Hq % Hkv == 0, "bad head counts")
-    _need(D in (16, 32, 64, 128), f"head_dim {D} not in {{16, 32, 64, 128}}")
+    if D not in (16, 32, 64, 128):
+        raise ValueError(f"head_dim {D} not in {{16, 32, 64, 128}}")
     rtt = infer_state.req_manager.req_to_token_indexs
     _cuda_tensor("b_seq_len", infer_state.b_seq_len, (torch.int32,), 1)
     _cuda_tensor("b_req_idx", infer_state.b_req_idx, (torch.int32,), 1)
@@ -378,7 +397,7 @@ def dense_decode(q, infer_state, cache_k, cache_v, out=None, alloc_tensor_func: 
     if workspace is None:
         workspace = alloc_tensor_func(((need + 3) // 4,), dtype=torch.float32, device=q.device)
     have = workspace.numel() * workspace.element_size()
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         check(_lib.lib().wsvd_dense_decode_f16(ctypes.byref(p), _ptr(workspace), have, _stream(stream)),
               "wsvd_dense_decode_f16")
     return out
@@ -428,7 +447,7 @@ def latent_quant_append(x_k, x_v, infer_state, cache_latent_k, cache_latent_k_sc
     p.batch, p.n_kv_heads, p.rank_k, p.rank_v = B, Hkv, Rk, Rv
     p.max_len = rtt.shape[1]
     p.x_dtype = 1 if x_k.dtype == torch.float16 else 2
-    with torch.cuda.device(x_k.device):
+    with _on_device(x_k.device):
         check(_lib.lib().wsvd_latent_quant_append_i8(ctypes.byref(p), _stream(stream)), "wsvd_latent_quant_append_i8")
 
 
