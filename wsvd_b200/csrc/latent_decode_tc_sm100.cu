@@ -765,6 +765,13 @@ __device__ __forceinline__ void build_pq(const TcArgs& ta, uint8_t* sm, int b, i
     qv0 = *reinterpret_cast<const uint4*>(qp + (interleaved ? ic * 16 : ic * 8));
     qv1 = *reinterpret_cast<const uint4*>(qp + (interleaved ? ic * 16 + 8 : 64 + ic * 8));
   }
+  uint4 s0v = make_uint4(0u, 0u, 0u, 0u), s1v = s0v;  // int8 wk: the scales of the chunk's two sets of dimensions
+  if (wk_vec && wk_i8) {
+    const int ic = tid & 7;
+    const __half* ws = reinterpret_cast<const __half*>(p.wk_scale) + (int64_t)hk * 128;
+    s0v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 : ic * 8));
+    s1v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 + 8 : 64 + ic * 8));
+  }
   cp_async_wait_all();  // this thread's own pieces of wk
   // q * sm_scale * log2(e) (scores come out in the log2 domain): qlo[e] pairs with dimension
   // d0 and qhi[e] with its rotation partner d1 of frequency ic*8 + e
@@ -826,9 +833,6 @@ __device__ __forceinline__ void build_pq(const TcArgs& ta, uint8_t* sm, int b, i
   } else if (wk_vec && wk_i8) {
     // int8 wk in vectors of eight; the columns' scales are this thread's for all four ranks.  fp32 throughout.
     const int ic = tid & 7;
-    const __half* ws = reinterpret_cast<const __half*>(p.wk_scale) + col;
-    const uint4 s0v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 : ic * 8));
-    const uint4 s1v = *reinterpret_cast<const uint4*>(ws + (interleaved ? ic * 16 + 8 : 64 + ic * 8));
     const __half* s0h = reinterpret_cast<const __half*>(&s0v);
     const __half* s1h = reinterpret_cast<const __half*>(&s1v);
 #pragma unroll 2
@@ -1583,11 +1587,14 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
         // memory (the head's plane area: its value MMAs are complete).
         reinterpret_cast<float*>(sm + C::kOffPlanes + 2 * g * C::kPlaneBytes)[r] = o;
       }
-      if (fused && n_parts > 1) __threadfence();
       head_sync();  // the partial is out, the (max, sum) pairs and the references have been read
       if (fused) {
         // the counter's answer is needed only after the next item's [P;Q] build
-        if (n_parts > 1 && row == 0) seen = atomicAdd(ta.arrivals + (int64_t)b * p.n_q_heads + h, 1u);
+        // (the fence is this thread's alone: it covers what the barrier above has shown it of the others' stores)
+        if (n_parts > 1 && row == 0) {
+          __threadfence();
+          seen = atomicAdd(ta.arrivals + (int64_t)b * p.n_q_heads + h, 1u);
+        }
         pending = true;
       }
     }
