@@ -755,7 +755,8 @@ def dense_baseline(m, spec, ms_step, k):
 
 def f16_latents_leg(m, spec, peak, k):
     """The same shape with an f16 latent cache (the reference's f16 op, 2*(rank_k+rank_v) bytes per
-    token-head, no scales): the warp-MMA kernel with fixed-length splits, then the merge kernel."""
+    token-head, no scales) on the tcgen05 kernel; `split_len` and `n_splits` are the plan that an explicit
+    split length, or the warp-MMA kernel, would run."""
     import ctypes as ct
 
     from wsvd_b200 import _lib, inputs, ops
@@ -789,7 +790,7 @@ def f16_latents_leg(m, spec, peak, k):
     generic()
     ms_generic = m.timed(generic, 3) / 3
     nbytes = sum(m.lens) * m.H * 2 * (spec.rank_k + spec.rank_v)
-    return {"kernel": "warp-MMA (mma.sync m16n8k16), fixed-length splits", "split_len": split_len, "n_splits": n_splits,
+    return {"kernel": "tcgen05, balanced shares", "split_len": split_len, "n_splits": n_splits,
             "bytes_per_token_head": 2 * (spec.rank_k + spec.rank_v), "us_per_layer": ms_full * 1e3,
             "us_stage1": ms_s1 * 1e3, "GB/s": nbytes / (ms_full * 1e-3) / 1e9,
             "stage1_frac": nbytes / (ms_s1 * 1e-3) / 1e9 / peak, "us_per_layer_generic_kernel": ms_generic * 1e3}

@@ -125,7 +125,7 @@ int wsvd_kernel_status_reset(void);
  * BLOCK_SEQ constant that the reference hard-codes on the host (flash_decoding.py:18,31-36)
  * while its kernel autotunes it.  It is what runs when p->split_len > 0 and on the generic
  * kernel.  With p->split_len == 0 and a problem the tensor-core kernel accepts (head_dim 128,
- * int8 latents, ranks multiples of 16 up to 64, 16-byte aligned rows), wsvd_latent_decode does
+ * ranks up to 64; f16 latents: even ranks and at least 148 tiles), wsvd_latent_decode does
  * not use fixed-length splits at all: one kernel, one persistent CTA per SM, cuts the batch's
  * tiles of 128 positions into equal shares from the sequence lengths on the device (ragged
  * batches load every SM alike), and the CTA that completes a head's last partial merges the

@@ -41,9 +41,9 @@ int validate(const WsvdLatentDecodeParams* p, bool need_out) {
 
 bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; }
 
-// The tcgen05 kernel covers the decode shapes of the 7B/13B models with an int8 cache; the
-// warp-MMA kernel takes f16 latents, other head dimensions and any even rank; the rest runs on the
-// generic kernel.
+// What any selector but the others' sends to the tcgen05 kernel: int8 latents in whole 16-byte rows, with the balanced
+// shares or fixed splits.  (tc_auto_rows below adds what AUTO alone may send there.)  The warp-MMA kernel takes other
+// head dimensions and any even rank; the rest runs on the generic kernel.
 bool tc_eligible(const WsvdLatentDecodeParams* p) {
   if (p->kernel == WSVD_KERNEL_GENERIC || p->kernel == WSVD_KERNEL_MMA) return false;
   if (p->head_dim != 128) return false;

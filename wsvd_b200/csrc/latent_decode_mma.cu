@@ -1,4 +1,5 @@
-// Split-KV stage 1 of the latent decode attention for the shapes the tcgen05 kernel does not take:
+// Split-KV stage 1 of the latent decode attention for the shapes the tcgen05 kernel does not take (other head
+// dimensions, ranks above 64, f16 batches below one tile per SM, f16 with fixed splits):
 // f16 or int8 latents, head_dim 16..128, any even rank up to 128, fixed-length splits.  Same
 // algebra as the tcgen05 kernel, on warp-level tensor-core instructions (mma.sync m16n8k16) and
 // plain or cp.async loads; its only waits are block barriers:

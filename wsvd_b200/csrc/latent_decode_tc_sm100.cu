@@ -1,66 +1,69 @@
-// The latent decode attention on the Blackwell tensor cores (tcgen05.mma with accumulators in
-// tensor memory), for head_dim 128, int8 latents, rank_k and rank_v in {16,32,48,64}: split-KV
-// stage 1 and, in the balanced mode, also the merge, the U_v projection and the head all-gather.
+// The latent decode attention on the Blackwell tensor cores (tcgen05.mma with accumulators in tensor memory), for
+// head_dim 128, int8 or f16 latents and ranks up to 64: split-KV stage 1 and, in the balanced mode, also the merge, the
+// U_v projection and the head all-gather.
 //
 // Scores.  For one head, query q and position s
 //   z_s = c * sk_s * sum_r Lk[s,r] * W[s,r],
 //   W[s,r] = sum_i cos(s f_i) P[r,i] + sin(s f_i) Q[r,i],
 //   P[r,i] = q_i U[i,r] + q_{i+64} U[i+64,r],   Q[r,i] = q_{i+64} U[i,r] - q_i U[i+64,r]
 // which is the reference's reconstruct -> RoPE -> q.K' chain
-// (efficiency/kernel/flash_int8_latent_per_head_decoding_rope_stage1.py:149-169) with
-// the sums reordered: the rotation is moved from K onto the query side.  W is one f16 GEMM
+// (efficiency/kernel/flash_int8_latent_per_head_decoding_rope_stage1.py:149-169,
+// flash_latent_per_head_decoding_rope_stage1.py:84-165 for f16 latents) with the sums reordered: the rotation is moved
+// from K onto the query side.  W is one f16 GEMM
 //   [128 positions x 128 (cos|sin)] x [128 x 64*(heads of a pair)]
-// per tile of 128 positions and pair of heads: the A operand is a tile of a position table
-// of cos/sin values (f16, shared by every head and sequence, read from L2 by TMA), the B
-// operand [P;Q] is built once per work item and stays in shared memory, the accumulator is fp32
-// in tensor memory (three 128-column buffers).  Each epilogue thread owns one token: it
-// reads its row of W from tensor memory and dots it in fp32 with the token's int8 K row,
-// which it copied from the K ring into registers at the top of the tile (so that the ring
-// slot is refilled a whole tile before its next use).
+// per tile of 128 positions and pair of heads: the A operand is a tile of a position table of cos/sin values (f16, shared
+// by every head and sequence, read from L2 by TMA), the B operand [P;Q] is built once per work item and stays in shared
+// memory, the accumulator is fp32 in tensor memory (three 128-column buffers).  Each epilogue thread owns one token: it
+// reads its row of W from tensor memory and dots it in fp32 with the token's K row, which it copied from its slot into
+// registers at the top of the tile (so that the slot is refilled long before its next use).
 //
-// Values.  O[r] = sum_s p_s sv_s Lv[s,r] is a true contraction over the tokens and runs on
-// the tensor cores as an int8 MMA (kind::i8): the A operand is a quarter of the V tile exactly as
-// TMA wrote it (32 tokens x 64 bytes, 64-byte swizzle = the MN-major canonical layout), the
-// B operand is the tile's weights a_s = 2^(y_s - max y), y_s = z_s + log2 sv_s, written by
-// their owner threads as three unsigned 8-bit digit planes of round(a_s * (2^24 - 256));
-// the int32 accumulator (64 ranks x 8 columns per head) is read back once per tile and
-// folded into a running fp32 sum under a running reference max(y).  The weights lose nothing
-// that fp32 would keep: 24 bits relative to the largest weight of the warp's 32 tokens.  The softmax
-// denominator is accumulated by the owner threads in fp32.
+// Values.  O[r] = sum_s p_s sv_s Lv[s,r] is a true contraction over the tokens and runs on the tensor cores: the A operand
+// is a quarter of the V tile exactly as TMA wrote it (32 tokens, swizzled = the MN-major canonical layout), the B operand
+// is the tile's weights, written by their owner threads.
+//  - int8 V: kind::i8.  a_s = 2^(y_s - max y), y_s = z_s + log2 sv_s, as three unsigned 8-bit digit planes of
+//    round(a_s * (2^24 - 256)); the int32 accumulator (64 ranks x 8 columns per (head, warp)) is read back once per tile and
+//    folded into a running fp32 sum under a running reference max(y).  The weights lose nothing that fp32 would keep: 24
+//    bits relative to the largest weight of the warp's 32 tokens.
+//  - f16 V: kind::f16, the weights as three f16 terms of 11 bits each; the fp32 accumulators add up over tiles until a
+//    weight outgrows the warp's reference (HeadSums).
+// The softmax denominator is accumulated by the owner threads in fp32.
 //
-// Work.  A work item is a run of consecutive tiles of one (sequence, group of 4 heads); it ends
-// in one partial result (normalised latent-space row + log-sum-exp per head) for the merge kernel.
+// Work.  A work item is a run of consecutive tiles of one (sequence, group of heads: four for int8 latents, two for f16,
+// whose rows take twice the shared memory); it ends in one partial result (normalised latent-space row + log-sum-exp per
+// head) for the merge.
 //  - Balanced mode: all tiles of the batch, ordered by (sequence, head group, tile), are cut
 //    into equal shares, one per persistent CTA (one CTA per SM).  A share covers a few items: the
 //    tail of one (sequence, head group), whole ones, the head of another.  No SM idles in a
 //    partial last wave whatever the sequence lengths, the [P;Q] build is paid once per item, and
 //    tensor memory is allocated once.  Every CTA computes its share itself from the sequence
-//    lengths (a block-wide prefix sum at the start of the kernel).  The partial of item (sequence
-//    b, head group hg) of CTA c goes to slot (b * n_hg + hg + c), which is unique because along
-//    the tile order every new item advances the (sequence, head group) index or the CTA index.
+//    lengths.  The partial of item (sequence b, head group hg) of CTA c goes to slot (b * n_hg + hg + c),
+//    which is unique because along the tile order every new item advances the (sequence, head group)
+//    index or the CTA index.
 //    With arrival counters (one per (sequence, head), zeroed before the launch) the kernel is the
 //    whole op: the CTA that completes a head's last partial merges the partials, multiplies by
 //    the head's slice of U_v and writes the output row; an item that one CTA covers alone skips
 //    the partials altogether.  With a peer set on top, the row goes to every rank's gathered
 //    buffer (16-byte peer stores) and the CTA that exits last runs the group's barrier.  Without
 //    counters the partials and the prefix sums are left for the merge kernel.
-//  - Split mode (no plan): CTA blockIdx.x handles split blockIdx.x % n_splits of a fixed-length
+//  - Split mode (int8, whole 16-byte rows): CTA blockIdx.x handles split blockIdx.x % n_splits of a fixed-length
 //    split plan, partials in the [B, Hq, n_splits] layout of the reference's stage 1.
-// 20 warps:
-//   warps 0-15   epilogue, 4 per head: warp w owns tensor-memory lanes 32*(w%4)..+31, i.e.
-//                tokens 32*(w%4).. of every tile of head w/4
-//   warp 16      one thread issues the score MMAs
-//   warp 17      requests the table tiles and the K and V rows
-//   warps 18-19  one pair of heads each (lane 0 and lane 1 one head each): issue the value MMAs
-// The 16 epilogue warps and the 4 control warps are two register groups: after the launch the
-// control warpgroup gives registers back and the epilogue warpgroups take them (setmaxnreg).
-// Latent rows travel in units of one tile (128 tokens) of ALL the group's heads: one TMA tensor
-// copy of 32 KB (64 bytes x 128 token slots x 4 heads) when the tile's token slots are consecutive
-// and the cache is head-major, else one copy per head, else a gather of rows with 16-byte
-// cp.async through the page table.  In the busy SM a control thread needs 20-40 cycles per
-// instruction, so waiting for a slot and issuing one copy costs 600-800 cycles whatever the size
-// of the copy: with five copies per tile (half-tile units) the requesting warp, not HBM, set the
-// pace of the whole kernel.  Hence few and large copies: 3 per tile and CTA (table, K, V).
+// Warps (int8: 20, f16: 11):
+//   epilogue     4 per head: warp w owns tensor-memory lanes 32*(w%4)..+31, i.e. tokens 32*(w%4).. of every tile of
+//                head w/4
+//   score MMAs   one warp
+//   copies       one warp: table tiles, K and V rows
+//   values       one warp per pair of heads: value MMAs
+// Every role walks the CTA's items for itself and none waits for the others at an item's end: the phases of the barriers
+// run on, the next item's copies start while the last tiles of this one are worked on, and a head's merge and projection
+// run while the next item's first score MMAs do.  With int8 latents the epilogue warps and the control warps are two
+// register groups: after the launch the control warpgroup gives registers back and the epilogue warpgroups take them
+// (setmaxnreg).
+// In the busy SM a control thread needs 20-40 cycles per instruction, so waiting for a slot and issuing one copy costs
+// 600-800 cycles whatever the size of the copy: hence few and large copies, one tile of all heads at a time where the
+// token slots allow it (copy_role).
+// What bounds it (13B shape, 16 x 8192 tokens, rank 64): int8 159 us against 107 us for reading the cache at the measured
+// HBM rate; neither issue alone (without the dot of the scores 153 us) nor the copies alone: the round trip of the one K slot
+// (16 warps copy their rows out, request, arrival) and a tile's work are about as long.  f16 latents 232 us against 208 us.
 // Every wait inside the tile loop is an mbarrier wait with a time limit; on a time-out the
 // kernel records a status code and every role falls through to the common exit, which frees
 // the tensor memory.
