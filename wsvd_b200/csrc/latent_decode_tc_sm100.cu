@@ -663,24 +663,30 @@ __device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, ui
   const uint32_t v_lo = (uint32_t)vdesc0, v_hi = (uint32_t)(vdesc0 >> 32), p_lo = (uint32_t)pdesc0, p_hi = (uint32_t)(pdesc0 >> 32);
   const bool issuer = elect_one();
   Walk w;
-  bool ok = true;
+  bool ok = true, skipped = false;   // skipped: the pair was not there in the item before
   uint32_t T = 0, mine[2] = {0, 0};  // tiles so far, and those that each head took part in
   for (bool more = w.start(ta, sh, n_hg); more && ok; more = w.next(p, n_hg)) {
     const int h0 = w.hg * C::kG, G = min(C::kG, p.n_q_heads - h0);
     if (2 * pair >= G) {
       T += w.ntiles;
+      skipped = true;
       continue;
     }
     for (int t = 0; t < w.ntiles && ok; ++t, ++T) {
       const uint32_t vslot = T % C::kVSlots;
-      // the V rows arrive long before the planes are ready: wait for them first, off the
-      // critical path from "planes ready" to "D full"
-      if constexpr (!C::kAny) ok = warp_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
+      // The V rows arrive long before the planes are ready: wait for them first, off the
+      // critical path from "planes ready" to "D full".  Not so with the first tile after tiles that passed this warp by:
+      // the parity of V full says nothing while the barrier is phases behind, and the planes (whose phases are
+      // this warp's own) are ready only when all tiles of the item before are done with.
+      const bool late = skipped;
+      skipped = false;
+      if (!C::kAny && !late) ok = warp_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int g = 2 * pair + j;
         if (g >= G || !ok) break;
         ok = warp_wait(bar(C::kBarPlanes + g), mine[j] & 1);
+        if (!C::kAny && late && j == 0 && ok) ok = warp_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
         if (!ok) break;
         ++mine[j];
         tc_fence_after();
@@ -1482,6 +1488,7 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
   auto state = [&](uint32_t i) { return item_state<C>(sm, g, i); };
   bool ok = true;  // after a wait that timed out: tiles are skipped, results are NaN
   bool pending = false;  // the item before is still to be finished
+  bool idle = false;     // this warp's head was not there in the item before
   unsigned int seen = 0;
   {
     Walk w;
@@ -1502,8 +1509,11 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(C::kBarPq));
-    // a warp whose head is not there must not arrive for the next item before this one's phase is over
-    if (!active && ok) ok = warp_wait(bar(C::kBarPq), item & 1);
+    // A warp whose head is not there must not arrive for the next item before this one's phase is over.  Where its head
+    // is there again, it must not start on the tiles before every other warp is through with the item that it sat out:
+    // the parities of K full and W full, which it would wait for, say nothing while those barriers are phases behind.
+    if ((!active || idle) && ok) ok = warp_wait(bar(C::kBarPq), item & 1);
+    idle = !active;
     if (pending) finish_head<C>(ta, sm, g, state(item + 1), seen);  // the item before, while the first score MMAs of this one run
     pending = false;
 
