@@ -70,7 +70,8 @@ stage2_kernel(const float* __restrict__ mid_o, const float* __restrict__ lse, co
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       if (i0 + i >= ns) continue;
-      const float w = __expf(ls[i] - m_new);
+      // (a partial of weight zero stays one where nothing has had any weight yet: -inf minus -inf is no zero)
+      const float w = ls[i] == -INFINITY ? 0.f : __expf(ls[i] - m_new);
       wsum += w;
       o = fmaf(w, mo[i], o);
     }

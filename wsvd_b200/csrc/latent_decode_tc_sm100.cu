@@ -1000,7 +1000,8 @@ __device__ __forceinline__ void finish_head(const TcArgs& ta, uint8_t* sm, int g
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         if (i0 + i >= f.n_parts) continue;
-        const float w = __expf(ls[i] - m_new);  // (a NaN stays one)
+        // (a NaN stays one; a partial of weight zero stays one where nothing has had any weight yet)
+        const float w = ls[i] == -INFINITY ? 0.f : __expf(ls[i] - m_new);
         wsum += w;
         osum = fmaf(w, mo[i], osum);
       }
