@@ -451,7 +451,13 @@ def latent_quant_append(x_k, x_v, infer_state, cache_latent_k, cache_latent_k_sc
         check(_lib.lib().wsvd_latent_quant_append_i8(ctypes.byref(p), _stream(stream)), "wsvd_latent_quant_append_i8")
 
 
-# ---- element-wise pieces of the decode step (one kernel each)
+# ---- element-wise pieces of the decode step (one kernel each), launched on the device of their tensors
+
+def _one_device(x, **others):
+    for name, t in others.items():
+        if t.device != x.device:
+            raise ValueError(f"{name} is on {t.device}, expected {x.device}")
+
 
 def rms_norm(x: torch.Tensor, eps: float = 1e-5, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
     """x [rows, cols] f16 -> x * rsqrt(mean(x^2) + eps), f16 (no weight vector)."""
@@ -459,8 +465,10 @@ def rms_norm(x: torch.Tensor, eps: float = 1e-5, out: Optional[torch.Tensor] = N
     _need(x.is_contiguous(), "x must be contiguous")
     if out is None:
         out = torch.empty_like(x)
-    check(_lib.lib().wsvd_rms_norm_f16(_ptr(x), _ptr(out), x.shape[0], x.shape[1], float(eps), _stream(stream)),
-          "wsvd_rms_norm_f16")
+    _one_device(x, out=out)
+    with _on_device(x.device):
+        check(_lib.lib().wsvd_rms_norm_f16(_ptr(x), _ptr(out), x.shape[0], x.shape[1], float(eps), _stream(stream)),
+              "wsvd_rms_norm_f16")
     return out
 
 
@@ -470,9 +478,11 @@ def add_rms_norm(x: torch.Tensor, delta: torch.Tensor, eps: float = 1e-5, stream
     _cuda_tensor("x", x, (torch.float16,), 2)
     _cuda_tensor("delta", delta, (torch.float16,), 2)
     _need(x.is_contiguous() and delta.is_contiguous() and x.shape == delta.shape, "x and delta: same contiguous shape")
+    _one_device(x, delta=delta)
     x_out, y = torch.empty_like(x), torch.empty_like(x)
-    check(_lib.lib().wsvd_add_rms_norm_f16(_ptr(x), _ptr(delta), _ptr(x_out), _ptr(y), x.shape[0], x.shape[1],
-                                           float(eps), _stream(stream)), "wsvd_add_rms_norm_f16")
+    with _on_device(x.device):
+        check(_lib.lib().wsvd_add_rms_norm_f16(_ptr(x), _ptr(delta), _ptr(x_out), _ptr(y), x.shape[0], x.shape[1],
+                                               float(eps), _stream(stream)), "wsvd_add_rms_norm_f16")
     return x_out, y
 
 
@@ -485,8 +495,10 @@ def rope_half_(q: torch.Tensor, pos: torch.Tensor, inv_freq: torch.Tensor, strea
     _cuda_tensor("inv_freq", inv_freq, (torch.float32,), 1)
     _need(q.stride(1) == q.shape[2] and pos.numel() == q.shape[0] and inv_freq.numel() * 2 == q.shape[2],
           "q must be [B, H, D] with contiguous heads, B positions and D/2 frequencies")
-    check(_lib.lib().wsvd_rope_half_f16(_ptr(q), q.stride(0), _ptr(pos), _ptr(inv_freq), q.shape[0], q.shape[1],
-                                        q.shape[2], _stream(stream)), "wsvd_rope_half_f16")
+    _one_device(q, pos=pos, inv_freq=inv_freq)
+    with _on_device(q.device):
+        check(_lib.lib().wsvd_rope_half_f16(_ptr(q), q.stride(0), _ptr(pos), _ptr(inv_freq), q.shape[0], q.shape[1],
+                                            q.shape[2], _stream(stream)), "wsvd_rope_half_f16")
     return q
 
 
@@ -498,6 +510,8 @@ def silu_mul(up: torch.Tensor, gate: torch.Tensor, out: Optional[torch.Tensor] =
     if out is None:
         out = torch.empty(up.shape, dtype=up.dtype, device=up.device)
     _need(out.is_contiguous() and out.shape == up.shape, "out must be contiguous and shaped like up")
-    check(_lib.lib().wsvd_silu_mul_f16(_ptr(up), up.stride(0), _ptr(gate), gate.stride(0), _ptr(out), up.shape[0],
-                                       up.shape[1], _stream(stream)), "wsvd_silu_mul_f16")
+    _one_device(up, gate=gate, out=out)
+    with _on_device(up.device):
+        check(_lib.lib().wsvd_silu_mul_f16(_ptr(up), up.stride(0), _ptr(gate), gate.stride(0), _ptr(out), up.shape[0],
+                                           up.shape[1], _stream(stream)), "wsvd_silu_mul_f16")
     return out
