@@ -124,8 +124,8 @@ int wsvd_kernel_status_reset(void);
  * Fixed-length split plan: tokens per split and number of split slots per (b, h).  Replaces the
  * BLOCK_SEQ constant that the reference hard-codes on the host (flash_decoding.py:18,31-36)
  * while its kernel autotunes it.  It is what runs when p->split_len > 0 and on the generic
- * kernel.  With p->split_len == 0 and a problem the tensor-core kernel accepts (head_dim 128,
- * ranks up to 64; f16 latents: even ranks and at least 148 tiles), wsvd_latent_decode does
+ * kernel.  With p->split_len == 0 and a problem the tensor-core kernel accepts (head_dim 128, even
+ * ranks up to 64, even strides; f16 latents: at least 148 tiles), wsvd_latent_decode does
  * not use fixed-length splits at all: one kernel, one persistent CTA per SM, cuts the batch's
  * tiles of 128 positions into equal shares from the sequence lengths on the device (ragged
  * batches load every SM alike), and the CTA that completes a head's last partial merges the
@@ -337,7 +337,8 @@ int wsvd_peer_release(void* ptr);
  *  - Same arguments, result and status codes as wsvd_latent_decode, minus the workspace.
  *  - Returns WSVD_ERR_TOO_LARGE when wsvd_latent_decode_workspace_bytes(p) exceeds
  *    WSVD_STATIC_SCRATCH_BYTES (pass a prebuilt rope_table to leave more room for
- *    partials, or use wsvd_latent_decode).
+ *    partials, or use wsvd_latent_decode).  What WSVD_KERNEL_AUTO would run with balanced shares that
+ *    exceed it runs on the warp-MMA kernel where that one's fixed-length splits fit.
  *  - The first call on each device looks up the array's device address (one
  *    cudaGetSymbolAddress, with the calling thread's current device); make that first call
  *    before starting any stream capture.  No call allocates or frees memory.

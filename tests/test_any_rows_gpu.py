@@ -1,4 +1,5 @@
-"""Ranks and row addresses that the tensor copies cannot take, on the tcgen05 kernel by AUTO, against the oracle."""
+"""Ranks and row addresses that the tensor copies cannot take, by AUTO, against the oracle: even ones on the tcgen05
+kernel, odd ones on the generic kernel."""
 import pytest
 import torch
 
@@ -45,7 +46,7 @@ def test_ranks(dtype, rk, rv, heads):
 @pytest.mark.parametrize("pitch", [0, 1, 6])
 def test_row_addresses(dtype, shift, pitch):
     """Caches that start `shift` elements into their allocation, with token rows `pitch` elements longer than the heads
-    need: every alignment of a row within 16 bytes, token-major and scattered over the slots."""
+    need: rows at even alignments within 16 bytes (the others go to the generic kernel), token-major and scattered over the slots."""
     base = inputs.make_case(6, 6, 128, 64, 48, LENS, max(LENS), seed=shift, latent_dtype=dtype)
     case = inputs.token_major_copy(base, shuffle_seed=3)
     c = case.to("cuda")

@@ -1,4 +1,4 @@
-"""What WSVD_KERNEL_AUTO alone sends to the tcgen05 kernel (f16 latents, ranks and rows that the tensor copies cannot
+"""What WSVD_KERNEL_AUTO alone sends to the tcgen05 kernel (f16 latents, even ranks and rows that the tensor copies cannot
 take), as far as the C ABI shows it without a GPU: what was refused stays refused, plans stay, workspaces never shrink."""
 import ctypes
 

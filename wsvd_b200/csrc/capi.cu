@@ -60,33 +60,6 @@ bool tc_eligible(const WsvdLatentDecodeParams* p) {
   return true;
 }
 
-// What WSVD_KERNEL_AUTO alone gives to the tcgen05 kernel, in its balanced mode: f16 latents, and caches whose ranks or
-// rows do not fit the tensor copies (rank 62, token rows that do not start on 16-byte boundaries), which the kernel's
-// threads then fetch row by row.  0: none, else a Stage1Rows value.
-int tc_auto_rows(const WsvdLatentDecodeParams* p) {
-  if (p->kernel != WSVD_KERNEL_AUTO || p->split_len != 0 || tc_eligible(p)) return 0;
-  if (p->head_dim != 128 || p->rank_k > 64 || p->rank_v > 64) return 0;
-  if (p->pos_offset != nullptr && p->rope_table == nullptr) return 0;
-  if (!aligned16(p->q) || p->q_stride_b % 8 || p->q_stride_h % 8) return 0;  // 16-byte loads of q
-  if (p->rope_table && (!aligned16(p->rope_table) || p->rope_table_rows < ((p->max_len + 127) / 128) * 128)) return 0;
-  const bool f16 = p->latent_dtype == WSVD_F16;
-  const int64_t unit = f16 ? 8 : 16;  // elements of 16 bytes
-  const bool rows16 = p->rank_k % unit == 0 && p->rank_v % unit == 0 && aligned16(p->latent_k) && aligned16(p->latent_v) &&
-                      p->k_stride_t % unit == 0 && p->k_stride_h % unit == 0 && p->v_stride_t % unit == 0 &&
-                      p->v_stride_h % unit == 0;
-  if (f16) {
-    // Odd ranks stay with the generic kernel.  So do batches below one tile of 128 tokens and two heads per SM with the
-    // warp-MMA kernel: there both are bound by latency (2 sequences of 2048 tokens, 8 heads: 17 us here, 36 us there; 32
-    // heads of 512 tokens: 14 and 34 us; 8 sequences, 8 heads: 25 and 38 us; 40 heads, 16 x 8192 tokens: 250 and 713 us),
-    // and callers may rely on AUTO giving the bits that WSVD_KERNEL_MMA gives.
-    if (p->rank_k % 2 || p->rank_v % 2) return 0;
-    if ((reinterpret_cast<uintptr_t>(p->latent_k) | reinterpret_cast<uintptr_t>(p->latent_v)) & 1) return 0;
-    const int64_t groups = (p->n_q_heads + wsvd::kBalancedGroupF16 - 1) / wsvd::kBalancedGroupF16;
-    if (p->batch * groups * ((p->max_len + 127) / 128) < 148) return 0;
-  }
-  return rows16 ? wsvd::kRows16 : wsvd::kRowsAny;
-}
-
 // the caller's position table serves the warp-MMA kernel too ([2][rows][64] f16 is its layout for head_dim 128)
 bool mma_caller_table(const WsvdLatentDecodeParams* p) {
   return p->rope_table && p->head_dim == 128 && aligned16(p->rope_table) &&
@@ -106,6 +79,33 @@ bool mma_eligible(const WsvdLatentDecodeParams* p) {
   // with position offsets the table must reach max(pos_offset) + max_len, which only the caller knows
   if (p->pos_offset != nullptr && !mma_caller_table(p)) return false;
   return true;
+}
+
+// What WSVD_KERNEL_AUTO alone gives to the tcgen05 kernel, in its balanced mode, of what the warp-MMA kernel would run
+// otherwise: f16 latents, and caches whose ranks or rows do not fit the tensor copies (rank 62, token rows that do not
+// start on 16-byte boundaries), which the kernel's threads then fetch row by row.  0: none, else a Stage1Rows value.
+// Nothing that the generic kernel runs comes here (odd ranks, odd strides): it computes in fp32 what both tensor-core
+// kernels round to f16, the position table and the products of q and U_k (2-norm error against 64 bits at rank 63, 8192
+// tokens: 2.1e-4, of which 2.0e-4 is the rounding of the f16 result, against 2.8e-4).
+int tc_auto_rows(const WsvdLatentDecodeParams* p) {
+  if (p->kernel != WSVD_KERNEL_AUTO || p->split_len != 0 || tc_eligible(p) || !mma_eligible(p)) return 0;
+  if (p->head_dim != 128 || p->rank_k > 64 || p->rank_v > 64) return 0;
+  if (!aligned16(p->q) || p->q_stride_b % 8 || p->q_stride_h % 8) return 0;  // 16-byte loads of q
+  if (p->rope_table && !mma_caller_table(p)) return 0;  // (with position offsets there is one: mma_eligible)
+  const bool f16 = p->latent_dtype == WSVD_F16;
+  const int64_t unit = f16 ? 8 : 16;  // elements of 16 bytes
+  const bool rows16 = p->rank_k % unit == 0 && p->rank_v % unit == 0 && aligned16(p->latent_k) && aligned16(p->latent_v) &&
+                      p->k_stride_t % unit == 0 && p->k_stride_h % unit == 0 && p->v_stride_t % unit == 0 &&
+                      p->v_stride_h % unit == 0;
+  if (f16) {
+    // Batches below one tile of 128 tokens and two heads per SM stay with the warp-MMA kernel: there both are bound by
+    // latency (2 sequences of 2048 tokens, 8 heads: 17 us here, 36 us there; 32 heads of 512 tokens: 14 and 34 us; 8
+    // sequences, 8 heads: 25 and 38 us; 40 heads, 16 x 8192 tokens: 250 and 713 us),
+    // and callers may rely on AUTO giving the bits that WSVD_KERNEL_MMA gives.
+    const int64_t groups = (p->n_q_heads + wsvd::kBalancedGroupF16 - 1) / wsvd::kBalancedGroupF16;
+    if (p->batch * groups * ((p->max_len + 127) / 128) < 148) return 0;
+  }
+  return rows16 ? wsvd::kRows16 : wsvd::kRowsAny;
 }
 
 int table_rows_for(int max_len) {
