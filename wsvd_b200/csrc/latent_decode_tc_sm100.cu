@@ -1291,8 +1291,10 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
         if (!ok) break;
         fetch_v(sbase + C::kOffV + (Tt % C::kVSlots) * C::kUnitBytes + g * C::kHeadBytes, slot_t);
         // K of the next tile, if that is known to be gathered too and the slot's last tile was (with one slot that
-        // is this tile): then this head's rows of the slot are its own, and this warp has read them
-        k_ahead = (C::kKSlots == 1 || gathered) && lo + (t + 1) * kTile < hi && mode[(Tt + 1) & 3] == (int)(2 * (Tt + 1)) + 1;
+        // is this tile): then this head's rows of the slot are its own, and this warp has read them.  The copying warp may
+        // be publishing the word at this moment: one read decides for all lanes, which fetch together or not at all.
+        const int next_mode = __shfl_sync(0xffffffffu, lane == 0 ? mode[(Tt + 1) & 3] : 0, 0);
+        k_ahead = (C::kKSlots == 1 || gathered) && lo + (t + 1) * kTile < hi && next_mode == (int)(2 * (Tt + 1)) + 1;
         if (k_ahead) fetch_k(sbase + C::kOffK + (Tt + 1) % C::kKSlots * C::kUnitBytes + g * C::kHeadBytes, slot_c);
       } else {
         k_ahead = false;
