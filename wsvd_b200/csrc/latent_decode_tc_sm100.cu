@@ -1242,9 +1242,11 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     // ---- the next tile's scales and the page entry of the tile after it: requested a whole
     //      tile before they are used
     unsigned short sk_n = 0, sv_n = 0;
-    if (slot_n >= 0) {
-      sk_n = reinterpret_cast<const unsigned short*>(ksc)[(int64_t)slot_n * p.ks_stride_t];
-      sv_n = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_n * p.vs_stride_t];
+    if constexpr (!C::kF16) {  // (f16 latents have no scales: null pointers)
+      if (slot_n >= 0) {
+        sk_n = reinterpret_cast<const unsigned short*>(ksc)[(int64_t)slot_n * p.ks_stride_t];
+        sv_n = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_n * p.vs_stride_t];
+      }
     }
     const int slot_t = slot_c;
     slot_c = slot_n;
