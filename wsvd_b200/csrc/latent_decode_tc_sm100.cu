@@ -672,21 +672,20 @@ __device__ __forceinline__ void value_role(const TcArgs& ta, const Share& sh, ui
       skipped = true;
       continue;
     }
+    // After tiles that passed this warp by the parity of V full says nothing, for the barrier may be phases behind.  The
+    // planes, whose phases are this warp's own, are ready only when all tiles of the item before are done with.
+    if (skipped) ok = warp_wait(bar(C::kBarPlanes + 2 * pair), mine[0] & 1);
+    skipped = false;
     for (int t = 0; t < w.ntiles && ok; ++t, ++T) {
       const uint32_t vslot = T % C::kVSlots;
-      // The V rows arrive long before the planes are ready: wait for them first, off the
-      // critical path from "planes ready" to "D full".  Not so with the first tile after tiles that passed this warp by:
-      // the parity of V full says nothing while the barrier is phases behind, and the planes (whose phases are
-      // this warp's own) are ready only when all tiles of the item before are done with.
-      const bool late = skipped;
-      skipped = false;
-      if (!C::kAny && !late) ok = warp_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
+      // the V rows arrive long before the planes are ready: wait for them first, off the
+      // critical path from "planes ready" to "D full"
+      if constexpr (!C::kAny) ok = warp_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int g = 2 * pair + j;
         if (g >= G || !ok) break;
         ok = warp_wait(bar(C::kBarPlanes + g), mine[j] & 1);
-        if (!C::kAny && late && j == 0 && ok) ok = warp_wait(bar(C::kBarVFull + vslot), (T / C::kVSlots) & 1);
         if (!ok) break;
         ++mine[j];
         tc_fence_after();
