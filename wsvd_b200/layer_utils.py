@@ -14,6 +14,7 @@ from __future__ import annotations
 import math
 
 import torch
+from torch.autograd import forward_ad
 
 from . import ops
 from .infer_state import InferState
@@ -37,10 +38,17 @@ def post_attention_layernorm(x, weight, eps: float = 1e-5):
     return _rms_norm(x, weight, eps)
 
 
+def _differentiated(*tensors):
+    """Whether autograd has to see what is done with these tensors: backward, or forward with a tangent on one of them."""
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return True
+    return any(forward_ad.unpack_dual(t).tangent is not None for t in tensors)
+
+
 def _fused_rows(x, *tensors):
     """Whether the layer's element-wise chains can run as this package's kernels: f16 on a GPU, and nothing
     that autograd would have to see."""
-    if torch.is_grad_enabled() and any(t.requires_grad for t in (x, *tensors)):
+    if _differentiated(x, *tensors):
         return False
     return x.is_cuda and x.dtype == torch.float16 and all(t.dtype == torch.float16 for t in tensors)
 
