@@ -45,7 +45,8 @@ typedef enum WsvdRopeLayout { WSVD_ROPE_HALF = 0, WSVD_ROPE_INTERLEAVED = 1 } Ws
 
 /* Which stage-1 kernel to run.  AUTO picks the tcgen05 kernel when the shape allows. */
 typedef enum WsvdKernel {
-  WSVD_KERNEL_AUTO = 0,     /* tcgen05 kernel if the problem fits it, else warp-MMA, else generic */
+  WSVD_KERNEL_AUTO = 0,     /* tcgen05 kernel if the problem fits it, else warp-MMA, else generic
+                               (see wsvd_latent_decode_plan for what fits) */
   WSVD_KERNEL_GENERIC = 1,  /* CUDA-core kernel, any shape */
   WSVD_KERNEL_TC = 2,       /* tcgen05 + TMA kernel or WSVD_ERR_UNSUPPORTED */
   WSVD_KERNEL_MMA = 3       /* warp-MMA kernel (f16 or int8 latents, head_dim 16..128, even ranks) or WSVD_ERR_UNSUPPORTED */
@@ -56,6 +57,13 @@ typedef enum WsvdKernel {
  * token_decode_attention_flash_int8_latent_per_head_decoding_rope and its f16 sibling
  * pass to their kernels (efficiency/kernel/flash_decoding.py:3-55, :57-95;
  * flash_int8_latent_per_head_decoding_rope_stage1.py:33-56,250-280).
+ *
+ * What is read around the latents: rows that are not whole 16-byte pieces at 16-byte boundaries (rank 62, say)
+ * may be read in the aligned 16-byte pieces that hold them, so up to 15 bytes in front of the first row and
+ * behind the last one of latent_k and latent_v are read.  They are never used, and a piece never lies across
+ * a page.
+ * Signs of the scales: the quantiser's are positive.  The tcgen05 kernel leaves out the value of a token whose v_scale is
+ * negative or NaN where rows are whole 16-byte pieces; elsewhere, and on the other kernels, any scale counts as it is.
  */
 typedef struct WsvdLatentDecodeParams {
   const void* q;            int64_t q_stride_b, q_stride_h;

@@ -45,7 +45,7 @@ def test_f16_latents_split_lengths(split_len):
     assert_close(_run(case, split_len=split_len), oracle_for(case), f"split_len={split_len}")
 
 
-def test_auto_takes_f16_latents_to_the_mma_kernel_and_agrees_with_the_generic_one():
+def test_auto_takes_a_small_f16_batch_to_the_mma_kernel_which_agrees_with_the_generic_one():
     case = inputs.make_case(2, 8, 128, 64, 64, [2048, 900], 2048, seed=9, latent_dtype=torch.float16)
     auto, mma, gen = _run(case, "auto"), _run(case, "mma"), _run(case, "generic")
     assert torch.equal(auto, mma)

@@ -98,10 +98,9 @@ int tc_auto_rows(const WsvdLatentDecodeParams* p) {
                       p->k_stride_t % unit == 0 && p->k_stride_h % unit == 0 && p->v_stride_t % unit == 0 &&
                       p->v_stride_h % unit == 0;
   if (f16) {
-    // Batches below one tile of 128 tokens and two heads per SM stay with the warp-MMA kernel: there both are bound by
-    // latency (2 sequences of 2048 tokens, 8 heads: 17 us here, 36 us there; 32 heads of 512 tokens: 14 and 34 us; 8
-    // sequences, 8 heads: 25 and 38 us; 40 heads, 16 x 8192 tokens: 250 and 713 us),
-    // and callers may rely on AUTO giving the bits that WSVD_KERNEL_MMA gives.
+    // Batches below one tile of 128 tokens and two heads per SM (148) stay with the warp-MMA kernel, as they always
+    // were.  It is not the faster one there: 2 sequences of 2048 tokens, 8 heads: 17 us here, 36 us there; 32 heads of 512
+    // tokens: 14 and 34 us; 8 sequences, 8 heads: 25 and 38 us (40 heads, 16 x 8192 tokens: 250 and 713 us).
     const int64_t groups = (p->n_q_heads + wsvd::kBalancedGroupF16 - 1) / wsvd::kBalancedGroupF16;
     if (p->batch * groups * ((p->max_len + 127) / 128) < 148) return 0;
   }
