@@ -138,7 +138,8 @@ struct Cfg {
   static constexpr uint32_t kOffVRaw = kOffK + kTile * kG * kRawPitch;  // ANY
   static constexpr uint32_t kOffRef = kOffPlanes + 2 * kG * kPlaneBytes;  // [head][tile parity][warp] int8: reference of the tile's planes; f16: reference that a warp left with this tile
   static constexpr uint32_t kOffSum = kOffRef + kG * 2 * 4 * 4;           // [head][warp] (max z, denominator) at the end
-  static constexpr uint32_t kOffMode = kOffSum + kG * 4 * 8;              // [4] how the K and V rows of a tile arrive (ring)
+  static constexpr uint32_t kOffNeg = kOffSum + kG * 4 * 8;               // int8 ANY: [head] four sums, four references, see odd_scales
+  static constexpr uint32_t kOffMode = kOffNeg + (!F16 && ANY ? kG * 4 * 8 : 0);  // [4] how the K and V rows of a tile arrive (ring)
   static constexpr uint32_t kOffItem = kOffMode + 16;                     // [head][item parity] ItemState
   static constexpr uint32_t kOffBar = kOffItem + kG * 2 * 64;
   // barriers: V and K full/empty per ring slot, table full/empty, W full/empty, per head: D full,
@@ -308,6 +309,12 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 __device__ __forceinline__ float warp_max_redux(float v) {
   float r;
   asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+// the same, NaN if any lane's value is
+__device__ __forceinline__ float warp_max_redux_nan(float v) {
+  float r;
+  asm volatile("redux.sync.max.NaN.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return r;
 }
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -1165,6 +1172,25 @@ __device__ __forceinline__ void fold_left(HeadSums& hs, uint32_t d_addr, const f
   }
 }
 
+// int8 ANY, rarely: a token of the warp has a negative or NaN scale.  The weight of a negative scale takes its magnitude
+// (returned: y with it), and the V row goes in as -v - 1, which an int8 holds for every v: what each rank then lacks is the
+// sum of those weights, which is kept for the head's end as (reference, sum), together with any NaN, which the planes of
+// the weights cannot hold.
+// Eight sequences of up to 4096 tokens, 32 heads, rank 62: 64.1 us without any of this, 64.4 with it, 65.5 with the weights summed
+// for every token instead of here.
+__device__ __forceinline__ float odd_scales(float z, float sv, float y, float* kept) {
+  const bool neg = sv < 0.f;
+  if (neg) y = z + fast_log2(-sv);
+  const float ref = warp_max_redux(neg ? y : -INFINITY);
+  const float sum = warp_sum(y != y ? y : neg && y > -INFINITY ? fast_exp2(y - ref) : 0.f);
+  if ((threadIdx.x & 31) == 0) {
+    const float was = kept[4], m = fmaxf(was, ref);
+    kept[0] = fmaf(kept[0], fast_exp2(was - m), sum * fast_exp2(ref - m));
+    kept[4] = m;
+  }
+  return y;
+}
+
 // The tiles of an item, for one warp of a head that is there.
 template <class C>
 __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_t item, HeadSums& hs) {
@@ -1224,7 +1250,8 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                    : "=r"(w[4 * c]), "=r"(w[4 * c + 1]), "=r"(w[4 * c + 2]), "=r"(w[4 * c + 3])
                    : "r"(raw + row * C::kRawPitch + 16 * c));
-    shift_row<kWords>(w, slot >= 0 ? (int)((reinterpret_cast<uintptr_t>(base) + (int64_t)slot * stride) & 15) : 0);
+    // (2^31 slots are a multiple of 16 bytes: a sign bit that marks the slot changes nothing here; no slot: any shift does)
+    shift_row<kWords>(w, (int)((reinterpret_cast<uintptr_t>(base) + (int64_t)slot * stride) & 15));
   };
   bool k_ahead = false;  // the K rows of the tile that comes are on their way (gathered tiles)
   bool gathered = false; // the tile before was
@@ -1247,7 +1274,7 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
         sv_n = reinterpret_cast<const unsigned short*>(vsc)[(int64_t)slot_n * p.vs_stride_t];
       }
     }
-    const int slot_t = slot_c;
+    int slot_t = slot_c;
     slot_c = slot_n;
     slot_n = -1;
     if (s + 2 * kTile < hi) slot_n = page[s + 2 * kTile];
@@ -1316,6 +1343,10 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     if (!ok) break;
     tc_fence_after();
 
+    // int8 ANY: a negative or NaN scale among the warp's?  (Asked behind the wait for W, by which time the scales are here;
+    // the answer has the dot to arrive.)
+    bool odd = false;
+    if constexpr (C::kAny && !C::kF16) odd = __any_sync(0xffffffffu, sv_raw > 0x7c00);
     // ---- score: dot of this token's K row with its row of W, 16 ranks at a time
     const uint32_t taddr = tmem + ((uint32_t)(q4 * 32) << 16) + wb * 128 + (g & 1) * kRkMax;
     float2 dot0 = make_float2(0.f, 0.f), dot1 = make_float2(0.f, 0.f);
@@ -1360,7 +1391,8 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
     sv_raw = sv_n;
 
     // ---- softmax weights under the warp's reference, denominator (fp32, by the owner threads)
-    const float mz_w = warp_max_redux(z);
+    // (int8 ANY: a NaN among the scores shows in the maximum, so that it reaches l_lane whatever the others are)
+    const float mz_w = C::kAny && !C::kF16 ? warp_max_redux_nan(z) : warp_max_redux(z);
     float wgt, left;        // what the value MMA's operand is made of; what goes to refs
     uint32_t how = 0;       // f16: accumulator and whether to add to it
     if constexpr (C::kF16) {
@@ -1391,9 +1423,16 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       how |= own_buf;
       wgt = e * hs.scale;
     } else {
-      const float y = valid ? z + fast_log2(sv) : -INFINITY;  // log2(0) = -inf: a zero scale drops the token's value
+      // log2(0) = -inf: a zero scale drops the token's value.  (Whole rows: a negative or NaN scale does too.)
+      float y = valid ? z + fast_log2(sv) : -INFINITY;
+      if constexpr (C::kAny) {
+        if (odd) {
+          y = odd_scales(z, sv, y, reinterpret_cast<float*>(sm + C::kOffNeg) + g * 8 + q4);
+          if (sv < 0.f) slot_t |= (int)0x80000000;  // (the sign is looked at when the V row is put into place)
+        }
+      }
       left = warp_max_redux(y);
-      if (mz_w > -INFINITY) {
+      if (C::kAny ? !(mz_w == -INFINITY) : mz_w > -INFINITY) {
         const float m_new = fmaxf(hs.m_run, mz_w);
         hs.l_lane = fmaf(hs.l_lane, fast_exp2(hs.m_run - m_new), fast_exp2(z - m_new));  // 2^-inf = 0: m_run = -inf, masked tokens
         hs.m_run = m_new;
@@ -1418,10 +1457,18 @@ __device__ __forceinline__ bool run_tiles(const TcArgs& ta, uint8_t* sm, uint32_
       __syncwarp();
       uint32_t w[kWords + 4];
       read_raw(w, v_raw, v_base, p.v_stride_t * kEsize, slot_t);
+      if constexpr (C::kF16) {  // no token: zeros (0 x NaN)
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) w[i] = valid ? w[i] : 0u;
+      } else if (__any_sync(0xffffffffu, slot_t < -1)) {  // (see odd_scales; what an int8 row without a token holds meets a weight of 0)
+        const uint32_t flip = (uint32_t)(slot_t >> 31);
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) w[i] ^= flip;
+      }
 #pragma unroll
       for (int c = 0; c < kChunks; ++c)
-        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(vrow + C::row_off(row, c)),
-                     "r"(valid ? w[4 * c] : 0u), "r"(valid ? w[4 * c + 1] : 0u), "r"(valid ? w[4 * c + 2] : 0u), "r"(valid ? w[4 * c + 3] : 0u)
+        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(vrow + C::row_off(row, c)), "r"(w[4 * c]), "r"(w[4 * c + 1]),
+                     "r"(w[4 * c + 2]), "r"(w[4 * c + 3])
                      : "memory");
       __syncwarp();
       if (lo + (t + 1) * kTile < hi) fetch_v(v_raw, slot_c);
@@ -1523,6 +1570,10 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
 
     const float none = C::kF16 ? kNone : -INFINITY;
     HeadSums hs = {none, 0.f, none, 0.f, kNone, 0.f, 0u};
+    if constexpr (C::kAny && !C::kF16) {
+      float* kept = reinterpret_cast<float*>(sm + C::kOffNeg) + g * 8 + q4;
+      if (lane == 0) kept[0] = 0.f, kept[4] = kNone;
+    }
     if (active && ok) ok = run_tiles<C>(ta, sm, item, hs);
 
     // ---- the item's end.  What the next item needs is requested before the last value sums are waited for.
@@ -1583,10 +1634,11 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
       float m_all = none;
 #pragma unroll
       for (int w4 = 0; w4 < 4; ++w4) m_all = fmaxf(m_all, sums[w4].x);
-      float l_tot = 0.f;  // (f16: a NaN in any warp's sum stays)
+      float l_tot = 0.f;  // (f16, ANY: a NaN in any warp's sum stays)
 #pragma unroll
       for (int w4 = 0; w4 < 4; ++w4)
         if (C::kF16 || sums[w4].x > -INFINITY) l_tot = fmaf(sums[w4].y, fast_exp2(sums[w4].x - m_all), l_tot);
+        else if (C::kAny) l_tot += sums[w4].y;  // 0, or a NaN
       const int64_t slot = balanced ? ((int64_t)b * n_hg + hg + blockIdx.x) * C::kG + g
                                     : ((int64_t)b * p.n_q_heads + h) * a.n_splits + blockIdx.x % a.n_splits;
       const int r = 16 * q4 + lane;
@@ -1594,7 +1646,20 @@ __device__ __forceinline__ void epilogue_role(const TcArgs& ta, const Share& sh,
       // (after a wait that timed out the item's result is poisoned: NaN here propagates through the
       // merge into the output row, so a time-out cannot pass for a valid result)
       const float sum = hs.big_m > none ? hs.acc * fast_exp2(hs.big_m - m_all) : 0.f;
-      const float o = !ok ? __int_as_float(0x7fc00000) : C::kF16 || hs.big_m > none ? sum / l_tot : 0.f;
+      float o = C::kF16 || hs.big_m > none ? sum / l_tot : 0.f;
+      if constexpr (C::kAny && !C::kF16) {
+        const float4 kept = reinterpret_cast<const float4*>(sm + C::kOffNeg)[g * 2];
+        if ((kept.x + kept.y) + (kept.z + kept.w) != 0.f) {  // (no sum is negative)
+          const float4 ref = reinterpret_cast<const float4*>(sm + C::kOffNeg)[g * 2 + 1];
+          const float k[4] = {kept.x, kept.y, kept.z, kept.w}, kr[4] = {ref.x, ref.y, ref.z, ref.w};
+          float neg_tot = 0.f;
+#pragma unroll
+          for (int w4 = 0; w4 < 4; ++w4) neg_tot = fmaf(k[w4], m_all > -INFINITY ? fast_exp2(kr[w4] - m_all) : 1.f, neg_tot);
+          o = neg_tot != neg_tot ? neg_tot : o + neg_tot / l_tot;
+        }
+        if (l_tot != l_tot) o = l_tot;
+      }
+      if (!ok) o = __int_as_float(0x7fc00000);
       if (!fused || n_parts > 1) {
         if (lane < 16 && r < Rv) a.mid_o[slot * Rv + r] = o;
         // natural-log lse, as the merge kernel expects (stage1.py:216)
