@@ -73,3 +73,13 @@ def test_merge_inside_the_kernel(masked_tiles):
     torch.cuda.synchronize()
     assert torch.isfinite(got).all() and not torch.equal(got, whole)
     assert_close(got, low.float().cpu(), f"{masked_tiles} tiles masked", atol=1e-5, rtol=6e-4)
+
+
+def test_partials_of_the_lowest_finite_weight_count():
+    lowest = -torch.finfo(torch.float32).max
+    mid, lse = torch.arange(9.0).view(1, 1, 9, 1).expand(1, 1, 9, 8).contiguous(), torch.full((1, 1, 9), -INF)
+    lse[0, 0, [2, 8]] = lowest
+    out = torch.zeros(1, 1, 8, dtype=torch.float16, device="cuda")
+    ops.decode_stage2(mid.cuda(), lse.cuda(), torch.tensor([9 * 32], dtype=torch.int32, device="cuda"), out, 32)
+    torch.cuda.synchronize()
+    assert (out == 5).all()  # (2 + 8) / 2

@@ -52,7 +52,8 @@ stage2_kernel(const float* __restrict__ mid_o, const float* __restrict__ lse, co
   // out the weights for itself.  What bounds the kernel is latency: three loops of one load after another took 4.2 us
   // for 640 heads of 4 splits, this takes 3.3 us.
   const int r = threadIdx.x;
-  float m = -INFINITY, wsum = 0.f, o = 0.f;
+  // (The maximum starts at the lowest finite value: a partial of -inf has weight 0 also where nothing has had any yet.)
+  float m = -FLT_MAX, wsum = 0.f, o = 0.f;
   for (int i0 = 0; i0 < ns; i0 += 8) {
     float ls[8], mo[8];
 #pragma unroll
@@ -64,14 +65,13 @@ stage2_kernel(const float* __restrict__ mid_o, const float* __restrict__ lse, co
     float m_new = m;
 #pragma unroll
     for (int i = 0; i < 8; ++i) m_new = fmaxf(m_new, ls[i]);
-    const float keep = m > -INFINITY ? __expf(m - m_new) : 0.f;
+    const float keep = __expf(m - m_new);
     wsum *= keep;
     o *= keep;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       if (i0 + i >= ns) continue;
-      // (a partial of weight zero stays one where nothing has had any weight yet: -inf minus -inf is no zero)
-      const float w = ls[i] == -INFINITY ? 0.f : __expf(ls[i] - m_new);
+      const float w = __expf(ls[i] - m_new);
       wsum += w;
       o = fmaf(w, mo[i], o);
     }

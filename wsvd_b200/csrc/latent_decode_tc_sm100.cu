@@ -988,7 +988,8 @@ __device__ __forceinline__ void finish_head(const TcArgs& ta, uint8_t* sm, int g
     const int64_t slot0 = ((int64_t)f.b * n_hg + f.hg + f.c_first) * C::kG + g;
     // Eight partials at a time, their loads all in flight at once, each batch under a running maximum.  (A loop of one
     // partial after another cost a round trip to L2 each: with 16 CTAs on a head, half of the smallest call's time.)
-    float m = -INFINITY, wsum = 0.f, osum = 0.f;
+    // (The maximum starts at the lowest finite value: a partial of -inf has weight 0 also where nothing has had any yet.)
+    float m = -FLT_MAX, wsum = 0.f, osum = 0.f;
     for (int i0 = 0; i0 < f.n_parts; i0 += 8) {
       float ls[8], mo[8];
 #pragma unroll
@@ -1000,14 +1001,13 @@ __device__ __forceinline__ void finish_head(const TcArgs& ta, uint8_t* sm, int g
       float m_new = m;
 #pragma unroll
       for (int i = 0; i < 8; ++i) m_new = fmaxf(m_new, ls[i]);
-      const float keep = m > -INFINITY ? __expf(m - m_new) : 0.f;
+      const float keep = __expf(m - m_new);
       wsum *= keep;
       osum *= keep;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         if (i0 + i >= f.n_parts) continue;
-        // (a NaN stays one; a partial of weight zero stays one where nothing has had any weight yet)
-        const float w = ls[i] == -INFINITY ? 0.f : __expf(ls[i] - m_new);
+        const float w = __expf(ls[i] - m_new);  // (a NaN stays one)
         wsum += w;
         osum = fmaf(w, mo[i], osum);
       }
