@@ -133,7 +133,8 @@ int wsvd_kernel_status_reset(void);
  * BLOCK_SEQ constant that the reference hard-codes on the host (flash_decoding.py:18,31-36)
  * while its kernel autotunes it.  It is what runs when p->split_len > 0 and on the generic
  * kernel.  With p->split_len == 0 and a problem the tensor-core kernel accepts (head_dim 128, even
- * ranks up to 64, even strides; f16 latents: at least 148 tiles), wsvd_latent_decode does
+ * ranks up to 64, even strides; f16 latents: at least 148 tiles; rows that are not whole 16-byte pieces, and f16: sequences
+ * beyond the shortest, for which the warp-MMA kernel is the faster one), wsvd_latent_decode does
  * not use fixed-length splits at all: one kernel, one persistent CTA per SM, cuts the batch's
  * tiles of 128 positions into equal shares from the sequence lengths on the device (ragged
  * batches load every SM alike), and the CTA that completes a head's last partial merges the

@@ -97,6 +97,21 @@ int tc_auto_rows(const WsvdLatentDecodeParams* p) {
   const bool rows16 = p->rank_k % unit == 0 && p->rank_v % unit == 0 && aligned16(p->latent_k) && aligned16(p->latent_v) &&
                       p->k_stride_t % unit == 0 && p->k_stride_h % unit == 0 && p->v_stride_t % unit == 0 &&
                       p->v_stride_h % unit == 0;
+  // Short sequences stay with the warp-MMA kernel: a persistent CTA pays ~4 us for an item's start and end whatever its length,
+  // the other kernel's CTAs overlap theirs.  Measured (us, tcgen05 and warp-MMA kernel):
+  //   f16, whole rows, rank 64:  64 sequences x 32 heads x 64 tokens 58 and 48, x 96 tokens 58 and 55, x 128 tokens 58 and 64; a second
+  //     tile that has hardly begun, while the other kernel's CTAs are one wave: 64 x 8 x 130 tokens 35 and 26, x 160 tokens
+  //     34 and 26, x 256 tokens 34 and 34; 64 x 32 x 160 tokens 75 and 75
+  //   f16, any rows, rank 62:  64 x 32 x 64 tokens 72 and 49, x 192 tokens 104 and 89, x 256 tokens 110 and 108, x 320 tokens 126 and 147
+  //   int8, any rows, rank 62:  64 x 32 x 32 tokens 48 and 42, x 64 tokens 49 and 52, x 128 tokens 52 and 71
+  const int n = p->max_len;
+  if (!f16) {
+    if (n <= 32) return 0;
+  } else if (!rows16) {
+    if (n < 256) return 0;
+  } else if (n <= 96 || (n > 128 && n <= 160 && (int64_t)p->batch * ((p->n_q_heads + 3) / 4) <= 2 * 148)) {
+    return 0;
+  }
   if (f16) {
     // Batches below one tile of 128 tokens and two heads per SM (148) stay with the warp-MMA kernel, as they always
     // were.  It is not the faster one there: 2 sequences of 2048 tokens, 8 heads: 17 us here, 36 us there; 32 heads of 512
